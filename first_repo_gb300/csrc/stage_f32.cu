@@ -1361,13 +1361,53 @@ __global__ void k_totals(F32Form f, const unsigned long long *__restrict__ total
   if (q == 4) *emean = fstat[3 * q + 2] * inv_cells;
 }
 
-__global__ void k_to_f32(const double *__restrict__ src, int64_t n, double shift, float *__restrict__ dst) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (float)(src[i] - shift);
+// fp32 <-> fp64 conversions in integer operations, the values the hardware conversions give:
+// GB300 converts between the two at its FP64 rate (two lanes per SM and clock), which bounded
+// every kernel that hands particles or fields across (2^27 particles down: 10.9 ms, 1.1 TB/s).
+// Zeros, subnormals, infinities and NaNs (and results outside the normal fp32 range) take the
+// hardware conversion.
+__device__ __forceinline__ double widen(float v) {
+  const uint32_t u = __float_as_uint(v), a = u & 0x7fffffffu;
+  if (a - 0x00800000u >= 0x7f000000u) return (double)v;  // not a normal number
+  return __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + 0x38000000u)), (int)(u << 29));
+}
+__device__ __forceinline__ float narrow(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const uint32_t hi = (uint32_t)(b >> 32), a = hi & 0x7fffffffu;
+  // biased exponents 897 .. 1149: normal in fp32 also after rounding up
+  if (a - 0x38100000u >= 0x47e00000u - 0x38100000u) return (float)v;
+  // round to nearest even at bit 29, then rebias: exponent and fraction move as one number
+  const unsigned long long m = (b & 0x7fffffffffffffffull) + 0x0fffffffull + ((b >> 29) & 1ull);
+  return __uint_as_float((hi & 0x80000000u) | ((uint32_t)(m >> 29) - (896u << 23)));
+}
+// a cell index 0 .. 1023 as fp64
+__device__ __forceinline__ double widen_index(int i) {
+  const uint32_t u = __float_as_uint((float)i);
+  return i ? __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29)) : 0.0;
+}
+
+// up to three fields at once; every thread keeps four independent loads in flight. shift
+// must be 0 for a plain conversion (it is then not subtracted).
+struct ToF32 {
+  const double *src[3];
+  float *dst[3];
+};
+__global__ void __launch_bounds__(256) k_to_f32(ToF32 a, int64_t n, double shift) {
+  const double *__restrict__ src = a.src[blockIdx.y];
+  float *__restrict__ dst = a.dst[blockIdx.y];
+  const int64_t i0 = (int64_t)blockIdx.x * (blockDim.x * 4) + threadIdx.x;
+  double v[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = i0 + q * 256 < n ? __ldcs(src + i0 + q * 256) : 0.0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (i0 + q * 256 < n) dst[i0 + q * 256] = shift != 0.0 ? narrow(v[q] - shift) : narrow(v[q]);
 }
 
 // upload: absolute fp64 positions -> cell + fp32 offset (the reference's trunc cell)
 // particles p0 .. p0 + n - 1 from fp64 arrays holding them from index 0
+// The FP64 pipe was the bound (2^22 particles 163 us, 2.3 TB/s): a position in [0, 2^31) cells
+// takes four FP64 operations, its whole part read out of the low word of x + 2^52 (truncated).
 __global__ void k_from_f64(Geom G, F32Form f, const double *__restrict__ x, const double *__restrict__ y,
                            const double *__restrict__ z, const double *__restrict__ u, const double *__restrict__ v,
                            const double *__restrict__ w, const double *__restrict__ t, double tref, int64_t p0,
@@ -1376,15 +1416,24 @@ __global__ void k_from_f64(Geom G, F32Form f, const double *__restrict__ x, cons
   if (i >= n) return;
   const int64_t p = p0 + i;
   const double X[3] = {x[i], y[i], z[i]};
+  const double V[4] = {u[i], v[i], w[i], t[i]};
   int c[3];
   float o[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     double xi = X[d] * G.idx[d];
-    if (!isfinite(xi)) { atomicOr(err, kErrNonFinite); xi = 0.0; }
-    double fl = floor(xi);
-    int i = (int)fl;
-    float of = (float)(xi - fl);
+    int i;
+    float of;
+    if ((uint32_t)__double2hiint(xi) < 0x41e00000u) {  // 0 <= xi < 2^31
+      const double s = __dadd_rz(xi, 4503599627370496.0);
+      i = __double2loint(s);
+      of = narrow(xi - (s - 4503599627370496.0));
+    } else {
+      if (!isfinite(xi)) { atomicOr(err, kErrNonFinite); xi = 0.0; }
+      const double fl = floor(xi);
+      i = (int)fl;
+      of = (float)(xi - fl);
+    }
     if (of >= 1.0f) { of = 0.0f; i += 1; }
     c[d] = wrapi(i, G.n[d]);
     o[d] = of;
@@ -1393,15 +1442,22 @@ __global__ void k_from_f64(Geom G, F32Form f, const double *__restrict__ x, cons
   B.cell[p] = pack(c[0], c[1], c[2]);
 #pragma unroll
   for (int d = 0; d < 3; ++d) B.o[d][p] = o[d];
-  B.v[0][p] = (float)u[i];
-  B.v[1][p] = (float)v[i];
-  B.v[2][p] = (float)w[i];
-  B.v[3][p] = (float)(t[i] - tref);
+  B.v[0][p] = narrow(V[0]);
+  B.v[1][p] = narrow(V[1]);
+  B.v[2][p] = narrow(V[2]);
+  B.v[3][p] = narrow(V[3] - tref);
 }
+
+// the cell sizes l/n of the position conversions (a double division each, made on the host)
+struct Dx {
+  double d[3];
+};
+Dx cell_size(const Geom &G) { return {{G.l[0] / G.n[0], G.l[1] / G.n[1], G.l[2] / G.n[2]}}; }
+__device__ __forceinline__ double position(int i, float o, double dx) { return (widen_index(i) + widen(o)) * dx; }
 
 // download: one array of a set as fp64 (positions back to absolute coordinates)
 // particles p0 .. p0 + n - 1 into dst[0 .. n)
-__global__ void k_to_f64_arr(Geom G, Set32 S, int comp, double tref, int64_t p0, int64_t n,
+__global__ void k_to_f64_arr(Dx dx, Set32 S, int comp, double tref, int64_t p0, int64_t n,
                              double *__restrict__ dst) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
@@ -1409,11 +1465,11 @@ __global__ void k_to_f64_arr(Geom G, Set32 S, int comp, double tref, int64_t p0,
   if (comp < 3) {
     const uint32_t c = S.cell[p];
     const int i = comp == 0 ? ci_(c) : (comp == 1 ? cj_(c) : ck_(c));
-    dst[q] = ((double)i + (double)S.o[comp][p]) * (G.l[comp] / G.n[comp]);
+    dst[q] = position(i, S.o[comp][p], dx.d[comp]);
   } else if (comp < 6) {
-    dst[q] = (double)S.v[comp - 3][p];
+    dst[q] = widen(S.v[comp - 3][p]);
   } else {
-    dst[q] = (double)S.v[3][p] + tref;
+    dst[q] = widen(S.v[3][p]) + tref;
   }
 }
 
@@ -1456,12 +1512,12 @@ __global__ void __launch_bounds__(256) k_perm_batch(PermBatch<T> b, const int32_
 
 __global__ void k_f32_to_f64(const float *__restrict__ src, int64_t n, double *__restrict__ dst) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (double)src[i];
+  if (i < n) dst[i] = widen(src[i]);
 }
 
 __global__ void k_to_f32_shift(const float *__restrict__ src, int64_t n, double shift, double *__restrict__ dst) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (double)src[i] + shift;
+  if (i < n) dst[i] = widen(src[i]) + shift;
 }
 
 __global__ void k_recip32(const double *__restrict__ tau, int64_t n, float *__restrict__ out) {
@@ -1979,9 +2035,22 @@ int f32_bind_fields(pstep_ctx *h, int which) {
   }
   const double *src[4] = {h->ux, h->uy, h->uz, h->tf};
   float *dst[4] = {f.uf[0], f.uf[1], f.uf[2], f.tf};
-  for (int q = 0; q < 4; ++q) {
-    if (!src[q] || !(which & (q < 3 ? 1 : 2))) continue;
-    k_to_f32<<<nb(gs), kThreads, 0, h->stream>>>(src[q], gs, q == 3 ? f.tref : 0.0, dst[q]);
+  ToF32 a{};
+  int nf = 0;
+  for (int q = 0; q < 3; ++q)
+    if (src[q] && (which & 1)) {
+      a.src[nf] = src[q];
+      a.dst[nf++] = dst[q];
+    }
+  const unsigned blocks = (unsigned)((gs + 1023) / 1024);
+  if (nf) {
+    k_to_f32<<<dim3(blocks, (unsigned)nf), 256, 0, h->stream>>>(a, gs, 0.0);
+    PSTEP_LAUNCHED(h);
+  }
+  if (src[3] && (which & 2)) {
+    a.src[0] = src[3];
+    a.dst[0] = dst[3];
+    k_to_f32<<<blocks, 256, 0, h->stream>>>(a, gs, f.tref);
     PSTEP_LAUNCHED(h);
   }
   return PSTEP_OK;
@@ -2170,7 +2239,7 @@ int f32_end_step(pstep_ctx *h) {
 }
 
 namespace {
-__global__ void k_positions32(Geom G, Set32 S, const int32_t *__restrict__ idx, int32_t n, double *__restrict__ xyz) {
+__global__ void k_positions32(Dx dx, Set32 S, const int32_t *__restrict__ idx, int32_t n, double *__restrict__ xyz) {
   const int32_t i = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= n) return;
   const int32_t p = idx[i];
@@ -2178,7 +2247,7 @@ __global__ void k_positions32(Geom G, Set32 S, const int32_t *__restrict__ idx, 
   const uint32_t c = S.cell[p];
   const int cc[3] = {ci_(c), cj_(c), ck_(c)};
 #pragma unroll
-  for (int d = 0; d < 3; ++d) xyz[3 * i + d] = ((double)cc[d] + (double)S.o[d][p]) * (G.l[d] / G.n[d]);
+  for (int d = 0; d < 3; ++d) xyz[3 * i + d] = position(cc[d], S.o[d][p], dx.d[d]);
 }
 }  // namespace
 
@@ -2187,7 +2256,7 @@ __global__ void k_positions32(Geom G, Set32 S, const int32_t *__restrict__ idx, 
 int f32_positions(pstep_ctx *h, const int32_t *idx, int32_t n, double *xyz) {
   F32Form &f = *h->f32;
   if (n <= 0) return PSTEP_OK;
-  k_positions32<<<(n + kThreads - 1) / kThreads, kThreads, 0, h->stream>>>(h->geom, f.set[SBASE], idx, n, xyz);
+  k_positions32<<<(n + kThreads - 1) / kThreads, kThreads, 0, h->stream>>>(cell_size(h->geom), f.set[SBASE], idx, n, xyz);
   PSTEP_LAUNCHED(h);
   return PSTEP_OK;
 }
@@ -2195,21 +2264,24 @@ int f32_positions(pstep_ctx *h, const int32_t *idx, int32_t n, double *xyz) {
 namespace {
 // the base state of particles p0 .. p0 + n - 1 as fp64 (absolute positions, velocities,
 // temperature) into dst[q][0 .. n): the arrays pstep_get_particle_array returns for
-// PSTEP_X .. PSTEP_T, all seven from one read of each particle
-__global__ void k_to_f64_all(Geom G, Set32 S, double tref, int64_t p0, int64_t n, double *__restrict__ x,
+// PSTEP_X .. PSTEP_T, all seven from one read of each particle. HBM-bound with the integer
+// conversions and the cell size divided on the host (seven FP64 operations a particle are left).
+__global__ void k_to_f64_all(Dx dx, Set32 S, double tref, int64_t p0, int64_t n, double *__restrict__ x,
                              double *__restrict__ y, double *__restrict__ z, double *__restrict__ u,
                              double *__restrict__ v, double *__restrict__ w, double *__restrict__ t) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const int64_t p = p0 + q;
   const uint32_t c = S.cell[p];
-  x[q] = ((double)ci_(c) + (double)S.o[0][p]) * (G.l[0] / G.n[0]);
-  y[q] = ((double)cj_(c) + (double)S.o[1][p]) * (G.l[1] / G.n[1]);
-  z[q] = ((double)ck_(c) + (double)S.o[2][p]) * (G.l[2] / G.n[2]);
-  u[q] = (double)S.v[0][p];
-  v[q] = (double)S.v[1][p];
-  w[q] = (double)S.v[2][p];
-  t[q] = (double)S.v[3][p] + tref;
+  const float o0 = S.o[0][p], o1 = S.o[1][p], o2 = S.o[2][p];
+  const float v0 = S.v[0][p], v1 = S.v[1][p], v2 = S.v[2][p], v3 = S.v[3][p];
+  __stcs(x + q, position(ci_(c), o0, dx.d[0]));
+  __stcs(y + q, position(cj_(c), o1, dx.d[1]));
+  __stcs(z + q, position(ck_(c), o2, dx.d[2]));
+  __stcs(u + q, widen(v0));
+  __stcs(v + q, widen(v1));
+  __stcs(w + q, widen(v2));
+  __stcs(t + q, widen(v3) + tref);
 }
 }  // namespace
 
@@ -2222,7 +2294,7 @@ int f32_download(pstep_ctx *h, double *const dst[7], int32_t *flag, int on_devic
   if (n == 0) return PSTEP_OK;
   const Set32 &B = f.set[SBASE];
   if (on_device) {
-    k_to_f64_all<<<nb(n), kThreads, 0, h->stream>>>(h->geom, B, f.tref, 0, n, dst[0], dst[1], dst[2], dst[3],
+    k_to_f64_all<<<nb(n), kThreads, 0, h->stream>>>(cell_size(h->geom), B, f.tref, 0, n, dst[0], dst[1], dst[2], dst[3],
                                                     dst[4], dst[5], dst[6]);
     PSTEP_LAUNCHED(h);
     PSTEP_CUDA(cudaMemcpyAsync(flag, h->s.flag, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
@@ -2235,7 +2307,7 @@ int f32_download(pstep_ctx *h, double *const dst[7], int32_t *flag, int on_devic
     const int64_t len = n - p0 < kStageChunk ? n - p0 : kStageChunk;
     double *b = f.stage[sl];
     PSTEP_CUDA(cudaStreamWaitEvent(h->stream, f.ev_copied[sl], 0));  // the slot's last copy (any call) is done
-    k_to_f64_all<<<nb(len), kThreads, 0, h->stream>>>(h->geom, B, f.tref, p0, len, b, b + kStageChunk,
+    k_to_f64_all<<<nb(len), kThreads, 0, h->stream>>>(cell_size(h->geom), B, f.tref, p0, len, b, b + kStageChunk,
                                                       b + 2 * kStageChunk, b + 3 * kStageChunk, b + 4 * kStageChunk,
                                                       b + 5 * kStageChunk, b + 6 * kStageChunk);
     PSTEP_LAUNCHED(h);
@@ -2271,7 +2343,7 @@ int f32_get_array(pstep_ctx *h, int id, void *dst, int on_device) {
   // particles p0 .. p0 + len - 1 as fp64 into out[0 .. len)
   auto convert = [&](int64_t p0, int64_t len, double *out) {
     if (set >= 0) {
-      k_to_f64_arr<<<nb(len), kThreads, 0, h->stream>>>(h->geom, f.set[set], comp, f.tref, p0, len, out);
+      k_to_f64_arr<<<nb(len), kThreads, 0, h->stream>>>(cell_size(h->geom), f.set[set], comp, f.tref, p0, len, out);
     } else if (id >= PSTEP_UG) {
       k_to_f32_shift<<<nb(len), kThreads, 0, h->stream>>>(f.gas[id - PSTEP_UG] + p0, len,
                                                           id == PSTEP_TG ? f.tref : 0.0, out);
