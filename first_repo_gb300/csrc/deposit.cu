@@ -147,17 +147,16 @@ __global__ void k_dep_face(Geom G, DepIn d, double *__restrict__ out) {
 
 // ---- fast path ----------------------------------------------------------------
 constexpr int kB = 8;                 // brick edge (target cells)
-constexpr int kB1 = kB + 1;           // trilinear node region edge [b, b+B]
+constexpr int kB1 = kB + 1;           // trilinear node region edge [b, b+B]; trunc cells [b-1, b+B-1]
 constexpr int kB2 = kB + 2;           // face node region edge [b-1, b+B]
+constexpr int kNodes = kB1 * kB1 * kB1, kRegion = kB2 * kB2 * kB2;
 constexpr int kBrickThreads = 256;
-constexpr size_t kBrickSmem = (size_t)kB1 * kB1 * kB1 * (8 + 6) * sizeof(double);
-// A node (or node h-class segment) with more particles than this is summed by a
-// warp: lanes stride its particles in order and a fixed shuffle tree adds the
-// lane sums. The order is fixed by the segment alone, so the result is the same
-// from run to run; one thread walking a blob-centre node (~1000 particles)
-// would hold up its whole brick.
+// Lists longer than this are summed by a warp: lanes stride the particles in order and a
+// fixed shuffle tree adds the lane sums. The order is fixed by the list alone, so the result
+// is the same from run to run; one thread walking a blob-centre node (~1000 particles) would
+// hold up its whole brick.
 constexpr int kDenseSeg = 32;
-constexpr int kDenseMax = kB2 * kB2 * kB2;
+constexpr int kBins = kDenseSeg + 2;  // list lengths 0 .. kDenseSeg, and longer
 
 __device__ __forceinline__ double warp_tree_sum(double v) {
 #pragma unroll
@@ -169,19 +168,21 @@ __device__ __forceinline__ double warp_tree_sum(double v) {
 // t = (x_l, y_l, z_l) of each particle and value v (1 for the concentration),
 // M[s] = sum v * prod_{d in s} t_d for the 8 subsets s of {x (4), y (2), z (1)}.
 // The corner with (1 - t_d) in the dimensions of bit set o and t_d in the others is
-// sum_{A subset of o} (-1)^|A| M[A | ~o], formed once per node. GB300's FP64 pipe
-// is the bound of this kernel, and per particle this takes 3 + 4 + 8 FP64
-// operations instead of 6 + 3 + 24 (+ 8). x_l = frac + 0.5 - h is formed as
+// sum_{A subset of o} (-1)^|A| M[A | ~o], formed once per node, a dimension at a time.
+// GB300's FP64 pipe (two lanes per SM and clock) is the bound of this kernel, and per particle
+// this takes 3 + 4 + 8 FP64 operations instead of 6 + 3 + 24 (+ 8). x_l = frac + 0.5 - h is formed as
 // frac + (h ? -0.5 : 0.5), the same value (frac - 1 and frac - 0.5 are exact for
 // frac >= 0.5).
-__device__ __forceinline__ void moments_add(double (&m)[8], const DepIn &d, int32_t p, int mode) {
+template <int MODE>
+__device__ __forceinline__ void moments_add(double (&m)[8], const DepIn &d, int32_t p) {
   const uint32_t key = d.key[p];
-  const double xl = d.frac[0][p] + (((key >> 2) & 1) ? -0.5 : 0.5);
-  const double yl = d.frac[1][p] + (((key >> 1) & 1) ? -0.5 : 0.5);
-  const double zl = d.frac[2][p] + ((key & 1) ? -0.5 : 0.5);
+  const double f0 = d.frac[0][p], f1 = d.frac[1][p], f2 = d.frac[2][p];
+  const double v = MODE ? d.val[0][p] : 0.0;
+  const double xl = f0 + ((key & 4u) ? -0.5 : 0.5);
+  const double yl = f1 + ((key & 2u) ? -0.5 : 0.5);
+  const double zl = f2 + ((key & 1u) ? -0.5 : 0.5);
   const double xy = xl * yl, xz = xl * zl, yz = yl * zl, xyz = xy * zl;
-  if (mode) {
-    const double v = d.val[0][p];
+  if (MODE) {
     m[0] += v;
     m[4] = fma(xl, v, m[4]);
     m[2] = fma(yl, v, m[2]);
@@ -190,8 +191,7 @@ __device__ __forceinline__ void moments_add(double (&m)[8], const DepIn &d, int3
     m[5] = fma(xz, v, m[5]);
     m[3] = fma(yz, v, m[3]);
     m[7] = fma(xyz, v, m[7]);
-  } else {
-    m[0] += 1.0;
+  } else {  // m[0], the particle count, is set by the caller
     m[4] += xl;
     m[2] += yl;
     m[1] += zl;
@@ -202,17 +202,17 @@ __device__ __forceinline__ void moments_add(double (&m)[8], const DepIn &d, int3
   }
 }
 
-// corner partial o (bit 2: x takes 1 - x_l, bit 1: y, bit 0: z) from the moments
-__device__ __forceinline__ double corner_of(const double (&m)[8], int o) {
-  const int rest = ~o & 7;
-  double c = 0.0;
+// moments -> corner partials in place (index bit 2: x takes 1 - x_l, bit 1: y, bit 0: z)
+__device__ __forceinline__ void corners_of(double (&m)[8]) {
 #pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    if ((a & o) != a) continue;  // subsets of o only
-    const double t = m[a | rest];
-    c = (__popc(a) & 1) ? c - t : c + t;
-  }
-  return c;
+  for (int bit = 1; bit < 8; bit <<= 1)
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (!(s & bit)) {
+        const double without = m[s], with = m[s | bit];
+        m[s] = with;
+        m[s | bit] = without - with;
+      }
 }
 
 // face sums of one particle: (sum r, sum t r) per dimension, r = RHS_u component
@@ -234,35 +234,124 @@ __device__ inline int32_t seg_lower_h(const DepIn &d, int32_t a, int32_t b, uint
   return a;
 }
 
-// mode 0: concentration (weights) + face momentum partials at x_int; mode 1: weights * RHS_T
+// Shared memory of a brick's CTA: the partials (trilinear first, then the faces in the same
+// place), slot-major so that neighbouring slots fall on neighbouring banks.
+constexpr int kTabulated = 255;
+template <int MODE> struct BrickSmem {
+  static constexpr int kTable = MODE ? 1 : kRegion;  // the faces' tables are the int deposit's
+  union {
+    double tri[8][kNodes];    // corner partials of node b + l
+    double face[6][kNodes];   // face partials of trunc cell b - 1 + l
+  };
+  uint8_t cls_end[kTable][8];  // node b - 1 + l: ends of the h classes 0..7 (at most kTabulated particles)
+  int32_t start[kRegion];      // node b - 1 + l: first sorted position
+  int32_t count[kRegion];      // its particles
+  uint16_t length[kNodes];     // list length of an item (clamped); faces: | non-empty h classes << 8
+  uint16_t order[kNodes];      // items by list length
+  int32_t bin[kBins];
+  int32_t n_dense, n_empty, next;
+};
+
+// Items 0 .. kNodes - 1 by their list length (sm.length's low byte), ascending, into sm.order; the
+// order inside a length is left to the atomics, since every item is summed by itself. A thread
+// walks one item's list and the FP64 pipe is charged per warp instruction: lists of like
+// length side by side let a warp's lanes end together (in storage order a warp ran the longest
+// of 32 lists with about a quarter of its lanes live).
+template <int MODE>
+__device__ __forceinline__ void order_by_length(BrickSmem<MODE> &sm) {
+  const int lane = (int)(threadIdx.x & 31u);
+  for (int q = threadIdx.x; q < kBins; q += blockDim.x) sm.bin[q] = 0;
+  __syncthreads();
+  // a few lengths hold most items: one add per distinct length of a warp
+  for (int s0 = threadIdx.x - lane; s0 < kNodes; s0 += blockDim.x) {
+    const int s = s0 + lane;
+    const int b = s < kNodes ? sm.length[s] & 255 : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, b);
+    if (b >= 0 && lane == __ffs(peers) - 1) atomicAdd(&sm.bin[b], __popc(peers));
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {  // exclusive scan of the bins
+    int carry = 0;
+    for (int b0 = 0; b0 < kBins; b0 += 32) {
+      const int b = b0 + lane;
+      const int v = b < kBins ? sm.bin[b] : 0;
+      int x = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (b < kBins) sm.bin[b] = carry + x - v;
+      if (b == 0) sm.n_empty = v;
+      if (b == kBins - 1) sm.n_dense = v;
+      carry += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (lane == 0) sm.next = 0;
+  }
+  __syncthreads();
+  for (int s0 = threadIdx.x - lane; s0 < kNodes; s0 += blockDim.x) {
+    const int s = s0 + lane;
+    const int b = s < kNodes ? sm.length[s] & 255 : -1;
+    const unsigned peers = __match_any_sync(0xffffffffu, b);
+    const int leader = __ffs(peers) - 1;
+    int at = 0;
+    if (b >= 0 && lane == leader) at = atomicAdd(&sm.bin[b], __popc(peers));
+    at = __shfl_sync(0xffffffffu, at, leader);
+    if (b >= 0) sm.order[at + __popc(peers & ((1u << lane) - 1u))] = (uint16_t)s;
+  }
+  __syncthreads();
+}
+
+// The ordered items in units: one dense item for a whole warp, or up to 32 others, a lane each;
+// warps take the longest lists first. dense(s) is called by all lanes, light(s) by single ones
+// (every item but the empty ones).
+template <int MODE, typename Dense, typename Light>
+__device__ __forceinline__ void take_items(BrickSmem<MODE> &sm, Dense dense, Light light) {
+  const int lane = (int)(threadIdx.x & 31u);
+  const int nd = sm.n_dense, nl = kNodes - nd - sm.n_empty, units = nd + (nl + 31) / 32;
+  while (true) {
+    int u = 0;
+    if (lane == 0) u = atomicAdd(&sm.next, 1);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    if (u >= units) break;
+    if (u < nd) {
+      dense((int)sm.order[kNodes - 1 - u]);
+    } else {
+      const int w = kNodes - nd - 1 - ((u - nd) * 32 + lane);
+      if (w >= sm.n_empty) light((int)sm.order[w]);
+    }
+    __syncwarp();
+  }
+}
+
+// mode 0: concentration (weights) + face momentum partials at x_int; mode 1: weights * RHS_T.
 //
-// A pre-pass tabulates, for every node of the brick's region [b-1, b+B], where its
-// segment starts and where each h class ends inside it (segments are sorted by h):
-// short segments by reading their keys (independent loads), longer ones by binary
-// search, each once per brick rather than once per phase. Nodes whose segment is
-// too long for 16-bit class ends (none at the particle densities of the workloads)
-// fall back to the searches in every phase.
-__global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, int mode, int twc,
+// Trilinear: one item per node of [b, b+B], its moments summed over the node's segment. Faces:
+// one item per trunc cell of [b-1, b+B-1]; its particles are, for each h class, that class's
+// run in node c + h's segment (the runs in class order, the empty ones skipped by a mask), so
+// all of a cell's particles are summed by one thread. Bound: the FP64 pipe; per particle 14 (15
+// in mode 1) operations for the trilinear sums and 6 for the faces, 12 + 7 a node and target,
+// 3 + 3 a cell and target. The pipe answers through a queue (short scoreboard), so a brick's
+// phases stay latency-bound between barriers: three CTAs per SM keep it 40% (mode 0) and 57%
+// (mode 1) busy. 256^3 cells x 2^24 particles in 64 blobs: 5.06 and 2.64 ms (a thread per node in
+// storage order, the faces in eight h-class phases over all nodes: 15 and 5 ms).
+template <int MODE>
+__global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, int twc,
                                                              double *__restrict__ out_tri,
                                                              double *__restrict__ out_x,
                                                              double *__restrict__ out_y,
                                                              double *__restrict__ out_z) {
-  extern __shared__ double sm[];
-  double *P = sm;                              // [kB1^3][8] trilinear partials of node b + l
-  double *F = sm + kB1 * kB1 * kB1 * 8;        // [kB1^3][6] face partials of trunc cell b - 1 + l
-  __shared__ int32_t seg_a[kDenseMax];         // node b - 1 + l: first sorted position
-  __shared__ uint16_t cls_end[kDenseMax][8];   // end of h classes 0..hc, relative to seg_a
-  __shared__ int32_t dense_s[kDenseMax];
-  __shared__ int32_t n_dense;
-  constexpr uint16_t kUntabulated = 0xffffu;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  BrickSmem<MODE> &sm = *reinterpret_cast<BrickSmem<MODE> *>(smem_raw);
   const int nbx = (G.g[0] + kB - 1) / kB, nby = (G.g[1] + kB - 1) / kB;
   const int bx = (int)(blockIdx.x % nbx) * kB;
   const int by = (int)((blockIdx.x / nbx) % nby) * kB;
   const int bz = (int)(blockIdx.x / ((long long)nbx * nby)) * kB;
-  const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5), nwarps = kBrickThreads / 32;
+  const int lane = (int)(threadIdx.x & 31u);
+  const bool faces = MODE == 0 && twc;
 
-  // pre-pass: segment table of the region's nodes
-  for (int s = threadIdx.x; s < kB2 * kB2 * kB2; s += blockDim.x) {
+  // segment table of the region's nodes [b-1, b+B]
+  for (int s = threadIdx.x; s < kRegion; s += blockDim.x) {
     const int lx = s % kB2, ly = (s / kB2) % kB2, lz = s / (kB2 * kB2);
     const int ni = bx - 1 + lx, nj = by - 1 + ly, nk = bz - 1 + lz;
     int32_t a0 = 0, cnt = 0;
@@ -271,140 +360,93 @@ __global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, in
       a0 = d.cell_start[n];
       cnt = d.cell_start[n + 1] - a0;
     }
-    seg_a[s] = a0;
-    if (cnt <= 16) {
-      uint64_t c = 0;  // 8 one-byte class counts (at most 16 each)
-      for (int32_t q = 0; q < cnt; ++q) c += 1ull << (8u * (d.key[pidx(d, a0 + q)] & 7u));
-      int run = 0;
+    if (faces) {
+      uint64_t ends = 0;
+      if (cnt <= 16) {
+        uint64_t c = 0;  // 8 one-byte class counts, then their running sums (at most 16)
+        for (int32_t q = 0; q < cnt; ++q) c += 1ull << (8u * (d.key[pidx(d, a0 + q)] & 7u));
+        ends = c * 0x0101010101010101ull;
+      } else if (cnt <= kTabulated) {
+#pragma unroll 1
+        for (int hc = 0; hc < 7; ++hc)
+          ends |= (uint64_t)(seg_lower_h(d, a0, a0 + cnt, hc + 1) - a0) << (8 * hc);
+        ends |= (uint64_t)cnt << 56;
+      }
+      *reinterpret_cast<uint64_t *>(sm.cls_end[MODE ? 0 : s]) = ends;
+    }
+    sm.start[s] = a0;
+    sm.count[s] = cnt;
+    // the trilinear item of a node in [b, b+B]
+    if (lx && ly && lz)
+      sm.length[((lz - 1) * kB1 + (ly - 1)) * kB1 + (lx - 1)] = (uint16_t)min(cnt, kDenseSeg + 1);
+  }
+  for (int s = threadIdx.x; s < 8 * kNodes; s += blockDim.x) sm.tri[0][s] = 0.0;
+  __syncthreads();
+
+  // ---- trilinear: node items (slot l in [0, B]^3, region slot l + 1)
+  order_by_length(sm);
+  auto region_of = [](int s) {
+    const int lx = s % kB1, ly = (s / kB1) % kB1, lz = s / (kB1 * kB1);
+    return ((lz + 1) * kB2 + (ly + 1)) * kB2 + (lx + 1);
+  };
+  take_items(
+      sm,
+      [&](int s) {
+        const int rs = region_of(s);
+        const int32_t a = sm.start[rs], cnt = sm.count[rs];
+        double m[8];
+#pragma unroll
+        for (int o = 0; o < 8; ++o) m[o] = 0.0;
+        for (int32_t q = a + lane; q < a + cnt; q += 32) moments_add<MODE>(m, d, pidx(d, q));
+#pragma unroll
+        for (int o = MODE ? 0 : 1; o < 8; ++o) m[o] = warp_tree_sum(m[o]);
+        if (lane == 0) {
+          if (!MODE) m[0] = (double)cnt;
+          corners_of(m);
+#pragma unroll
+          for (int o = 0; o < 8; ++o) sm.tri[o][s] = m[o];
+        }
+      },
+      [&](int s) {
+        const int rs = region_of(s);
+        const int32_t a = sm.start[rs], cnt = sm.count[rs];
+        double m[8];
+#pragma unroll
+        for (int o = 0; o < 8; ++o) m[o] = 0.0;
+        for (int32_t q = a; q < a + cnt; ++q) moments_add<MODE>(m, d, pidx(d, q));
+        if (!MODE) m[0] = (double)cnt;
+        corners_of(m);
+#pragma unroll
+        for (int o = 0; o < 8; ++o) sm.tri[o][s] = m[o];
+      });
+  __syncthreads();
+  // h classes and length of every cell item (slot l in [0, B]^3: cell b - 1 + l; its class-h run
+  // is in the segment of region slot l + h)
+  auto node_of = [](int base, int hc) { return base + ((hc & 1) * kB2 + ((hc >> 1) & 1)) * kB2 + ((hc >> 2) & 1); };
+  auto run = [&](int rs, int hc, int32_t &a, int32_t &e) {
+    const int32_t a0 = sm.start[rs], cnt = sm.count[rs];
+    if (cnt <= kTabulated) {
+      a = a0 + (hc ? sm.cls_end[MODE ? 0 : rs][hc - 1] : 0);
+      e = a0 + sm.cls_end[MODE ? 0 : rs][hc];
+    } else {  // a segment longer than the table holds
+      a = hc ? seg_lower_h(d, a0, a0 + cnt, hc) : a0;
+      e = hc < 7 ? seg_lower_h(d, a, a0 + cnt, hc + 1) : a0 + cnt;
+    }
+  };
+  if (faces) {
+    for (int s = threadIdx.x; s < kNodes; s += blockDim.x) {
+      const int base = ((s / (kB1 * kB1)) * kB2 + (s / kB1) % kB1) * kB2 + s % kB1;
+      int n = 0, classes = 0;
 #pragma unroll
       for (int hc = 0; hc < 8; ++hc) {
-        run += (int)((c >> (8 * hc)) & 0xffu);
-        cls_end[s][hc] = (uint16_t)run;
-      }
-    } else if (cnt < (int32_t)kUntabulated) {
-#pragma unroll 1
-      for (int hc = 0; hc < 7; ++hc) cls_end[s][hc] = (uint16_t)(seg_lower_h(d, a0, a0 + cnt, hc + 1) - a0);
-      cls_end[s][7] = (uint16_t)cnt;
-    } else {
-      cls_end[s][7] = kUntabulated;
-    }
-  }
-  if (threadIdx.x == 0) n_dense = 0;
-  __syncthreads();
-  // [a, e) of node slot s (region index) and h class hc
-  auto seg = [&](int s, int hc, int32_t &a, int32_t &e) {
-    const int32_t a0 = seg_a[s];
-    if (cls_end[s][7] != kUntabulated) {
-      a = a0 + (hc ? cls_end[s][hc - 1] : 0);
-      e = a0 + cls_end[s][hc];
-    } else {  // a segment longer than the table holds
-      const int lx = s % kB2, ly = (s / kB2) % kB2, lz = s / (kB2 * kB2);
-      const long long n = glin(G, bx - 1 + lx, by - 1 + ly, bz - 1 + lz);
-      const int32_t e0 = d.cell_start[n + 1];
-      a = hc ? seg_lower_h(d, a0, e0, hc) : a0;
-      e = hc < 7 ? seg_lower_h(d, a, e0, hc + 1) : e0;
-    }
-  };
-  // whole segment of node slot s
-  auto whole = [&](int s, int32_t &a, int32_t &e) {
-    int32_t a1, e1;
-    seg(s, 0, a, e1);
-    seg(s, 7, a1, e);
-  };
-
-  // trilinear: per-node partials for nodes [b, b+B] (region slot = l + 1); dense nodes listed for the warps
-  for (int s = threadIdx.x; s < kB1 * kB1 * kB1; s += blockDim.x) {
-    const int lx = s % kB1, ly = (s / kB1) % kB1, lz = s / (kB1 * kB1);
-    const int rs = ((lz + 1) * kB2 + (ly + 1)) * kB2 + (lx + 1);
-    double m[8];
-#pragma unroll
-    for (int o = 0; o < 8; ++o) m[o] = 0.0;
-    int32_t a, e;
-    whole(rs, a, e);
-    if (e - a > kDenseSeg) {
-      dense_s[atomicAdd(&n_dense, 1)] = s;
-      continue;
-    }
-    // one path for every node (empty ones included): the FP64 pipe is charged per warp
-    // instruction, so lanes on different paths would cost the warp both
-    for (int32_t q = a; q < e; ++q) moments_add(m, d, pidx(d, q), mode);
-#pragma unroll
-    for (int o = 0; o < 8; ++o) P[s * 8 + o] = corner_of(m, o);
-  }
-  __syncthreads();
-  for (int k = warp; k < n_dense; k += nwarps) {
-    const int s = dense_s[k];
-    const int lx = s % kB1, ly = (s / kB1) % kB1, lz = s / (kB1 * kB1);
-    int32_t a, e;
-    whole(((lz + 1) * kB2 + (ly + 1)) * kB2 + (lx + 1), a, e);
-    double m[8];
-#pragma unroll
-    for (int o = 0; o < 8; ++o) m[o] = 0.0;
-    for (int32_t q = a + lane; q < e; q += 32) moments_add(m, d, pidx(d, q), mode);
-#pragma unroll
-    for (int o = 0; o < 8; ++o) m[o] = warp_tree_sum(m[o]);
-    if (lane == 0) {
-#pragma unroll
-      for (int o = 0; o < 8; ++o) P[s * 8 + o] = corner_of(m, o);
-    }
-  }
-  const bool faces = (mode == 0) && twc;
-  if (faces) {
-    for (int s = threadIdx.x; s < kB1 * kB1 * kB1 * 6; s += blockDim.x) F[s] = 0.0;
-  }
-  __syncthreads();
-  // face partials: trunc cell c = node - h, one h class per phase (distinct nodes -> distinct cells);
-  // dense segments listed for the warps as above
-  if (faces) {
-    for (int hc = 0; hc < 8; ++hc) {
-      const int hx = (hc >> 2) & 1, hy = (hc >> 1) & 1, hz = hc & 1;
-      if (threadIdx.x == 0) n_dense = 0;
-      __syncthreads();
-      for (int s = threadIdx.x; s < kB2 * kB2 * kB2; s += blockDim.x) {
-        const int lx = s % kB2, ly = (s / kB2) % kB2, lz = s / (kB2 * kB2);
-        const int cx = lx - hx, cy = ly - hy, cz = lz - hz;  // cell slot: cell = b - 1 + c
-        if (cx < 0 || cy < 0 || cz < 0 || cx >= kB1 || cy >= kB1 || cz >= kB1) continue;
         int32_t a, e;
-        seg(s, hc, a, e);
-        if (a == e) continue;
-        if (e - a > kDenseSeg) {
-          dense_s[atomicAdd(&n_dense, 1)] = s;
-          continue;
-        }
-        double fs[6] = {0, 0, 0, 0, 0, 0};
-        for (int32_t q = a; q < e; ++q) face_add(fs, d, pidx(d, q));
-        // (1 - x_l) r summed as sum r - sum x_l r; x_l r as is
-        double *f = F + ((cz * kB1 + cy) * kB1 + cx) * 6;
-#pragma unroll
-        for (int D = 0; D < 3; ++D) {
-          f[2 * D] += fs[2 * D] - fs[2 * D + 1];
-          f[2 * D + 1] += fs[2 * D + 1];
-        }
+        run(node_of(base, hc), hc, a, e);
+        n += e - a;
+        classes |= e > a ? 1 << hc : 0;
       }
-      __syncthreads();
-      for (int k = warp; k < n_dense; k += nwarps) {
-        const int s = dense_s[k];
-        const int lx = s % kB2, ly = (s / kB2) % kB2, lz = s / (kB2 * kB2);
-        const int cx = lx - hx, cy = ly - hy, cz = lz - hz;
-        int32_t a, e;
-        seg(s, hc, a, e);
-        double fs[6] = {0, 0, 0, 0, 0, 0};
-        for (int32_t q = a + lane; q < e; q += 32) face_add(fs, d, pidx(d, q));
-#pragma unroll
-        for (int j = 0; j < 6; ++j) fs[j] = warp_tree_sum(fs[j]);
-        if (lane == 0) {
-          double *f = F + ((cz * kB1 + cy) * kB1 + cx) * 6;
-#pragma unroll
-          for (int D = 0; D < 3; ++D) {
-            f[2 * D] += fs[2 * D] - fs[2 * D + 1];
-            f[2 * D + 1] += fs[2 * D + 1];
-          }
-        }
-      }
-      __syncthreads();
+      sm.length[s] = (uint16_t)(min(n, kDenseSeg + 1) | classes << 8);
     }
   }
-  // targets of the brick
   for (int s = threadIdx.x; s < kB * kB * kB; s += blockDim.x) {
     const int lx = s % kB, ly = (s / kB) % kB, lz = s / (kB * kB);
     const int ti = bx + lx, tj = by + ly, tk = bz + lz;
@@ -413,20 +455,62 @@ __global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, in
 #pragma unroll
     for (int o = 0; o < 8; ++o) {
       const int ox = (o >> 2) & 1, oy = (o >> 1) & 1, oz = o & 1;
-      acc += P[(((lz + oz) * kB1 + (ly + oy)) * kB1 + (lx + ox)) * 8 + o];
+      const double v = sm.tri[o][((lz + oz) * kB1 + (ly + oy)) * kB1 + (lx + ox)];
+      acc = o ? acc + v : v;
     }
+    out_tri[glin(G, ti, tj, tk)] = acc;
+  }
+  if (!faces) return;
+  __syncthreads();
+
+  // ---- faces
+  for (int s = threadIdx.x; s < 6 * kNodes; s += blockDim.x) sm.face[0][s] = 0.0;
+  order_by_length(sm);
+  auto put = [&](int s, const double (&fs)[6]) {
+    // (1 - x_l) r summed as sum r - sum x_l r; x_l r as is
+#pragma unroll
+    for (int D = 0; D < 3; ++D) {
+      sm.face[2 * D][s] = fs[2 * D] - fs[2 * D + 1];
+      sm.face[2 * D + 1][s] = fs[2 * D + 1];
+    }
+  };
+  take_items(
+      sm,
+      [&](int s) {
+        const int base = ((s / (kB1 * kB1)) * kB2 + (s / kB1) % kB1) * kB2 + s % kB1;
+        double fs[6] = {0, 0, 0, 0, 0, 0};
+        for (int classes = sm.length[s] >> 8; classes; classes &= classes - 1) {
+          const int hc = __ffs(classes) - 1;
+          int32_t a, e;
+          run(node_of(base, hc), hc, a, e);
+          for (int32_t q = a + lane; q < e; q += 32) face_add(fs, d, pidx(d, q));
+        }
+#pragma unroll
+        for (int j = 0; j < 6; ++j) fs[j] = warp_tree_sum(fs[j]);
+        if (lane == 0) put(s, fs);
+      },
+      [&](int s) {
+        const int base = ((s / (kB1 * kB1)) * kB2 + (s / kB1) % kB1) * kB2 + s % kB1;
+        double fs[6] = {0, 0, 0, 0, 0, 0};
+        for (int classes = sm.length[s] >> 8; classes; classes &= classes - 1) {
+          const int hc = __ffs(classes) - 1;
+          int32_t a, e;
+          run(node_of(base, hc), hc, a, e);
+          for (int32_t q = a; q < e; ++q) face_add(fs, d, pidx(d, q));
+        }
+        put(s, fs);
+      });
+  __syncthreads();
+  for (int s = threadIdx.x; s < kB * kB * kB; s += blockDim.x) {
+    const int lx = s % kB, ly = (s / kB) % kB, lz = s / (kB * kB);
+    const int ti = bx + lx, tj = by + ly, tk = bz + lz;
+    if (ti >= G.g[0] || tj >= G.g[1] || tk >= G.g[2]) continue;
     const long long t = glin(G, ti, tj, tk);
-    out_tri[t] = acc;
-    if (faces) {
-      // cell slot of target cell t is l + 1; its lower neighbour in dimension D is l
-      const double *ft = F + (((lz + 1) * kB1 + (ly + 1)) * kB1 + (lx + 1)) * 6;
-      const double *fxm = F + (((lz + 1) * kB1 + (ly + 1)) * kB1 + lx) * 6;
-      const double *fym = F + (((lz + 1) * kB1 + ly) * kB1 + (lx + 1)) * 6;
-      const double *fzm = F + ((lz * kB1 + (ly + 1)) * kB1 + (lx + 1)) * 6;
-      out_x[t] = fxm[1] + ft[0];
-      out_y[t] = fym[3] + ft[2];
-      out_z[t] = fzm[5] + ft[4];
-    }
+    // cell slot of target cell t is l + 1; its lower neighbour in dimension D is l
+    const int c = ((lz + 1) * kB1 + (ly + 1)) * kB1 + (lx + 1);
+    out_x[t] = sm.face[1][c - 1] + sm.face[0][c];
+    out_y[t] = sm.face[3][c - kB1] + sm.face[2][c];
+    out_z[t] = sm.face[5][c - kB1 * kB1] + sm.face[4][c];
   }
 }
 
@@ -636,11 +720,13 @@ bool reference_sums(const pstep_ctx *h) {
 
 int brick_launch(pstep_ctx *h, const DepIn &d, int mode, double *tri, double *ox, double *oy, double *oz) {
   const Geom &G = h->geom;
+  auto kern = mode ? k_dep_brick<1> : k_dep_brick<0>;
+  const size_t smem = mode ? sizeof(BrickSmem<1>) : sizeof(BrickSmem<0>);
   // the opt-in applies to the current device, which is the one this launch uses;
   // setting it at every launch keeps it right for handles on several devices
-  PSTEP_CUDA(cudaFuncSetAttribute(k_dep_brick, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBrickSmem));
+  PSTEP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long long nb = (long long)((G.g[0] + kB - 1) / kB) * ((G.g[1] + kB - 1) / kB) * ((G.g[2] + kB - 1) / kB);
-  k_dep_brick<<<(unsigned)nb, kBrickThreads, kBrickSmem, h->stream>>>(G, d, mode, h->cfg.twc, tri, ox, oy, oz);
+  kern<<<(unsigned)nb, kBrickThreads, smem, h->stream>>>(G, d, h->cfg.twc, tri, ox, oy, oz);
   PSTEP_LAUNCHED(h);
   return PSTEP_OK;
 }
