@@ -341,6 +341,8 @@ int pstep_upload_particles(pstep_handle h, int64_t n, const double *x, const dou
   h->primed = 0;
   h->phase = 0;
   h->pmax64_state = 0;
+  h->t_rebound = 0;
+  h->t_pending = 0;
   if (is_f32(h)) {
     TRY(f32_upload(h, x, y, z, u, v, w, t, on_device));
   } else {
@@ -484,6 +486,11 @@ int pstep_stage_interp_advance_deposit(pstep_handle h, int k, double pre, double
     return PSTEP_OK;
   }
   h->fields_t_at_advance = h->fields_t;
+  // A caller that binds the temperature between Send_Recv and gas2part_Temp_new (as the
+  // reference does, grid.cpp:676) did so in the last stage too: the advance then leaves the
+  // temperature gather to pstep_stage_temp instead of gathering a field that is replaced
+  // (2^24 particles on 256^3 cells, advance + gather a stage: 4.15 + 1.37 ms before, 2.26 + 1.12 ms).
+  h->t_pending = h->t_rebound;
   if (k == 3) {  // the last stage gathers the step result's max u and max ug
     PSTEP_CUDA(cudaMemsetAsync(h->pmax64, 0, sizeof(unsigned long long) * 2 * 1024, h->stream));
     h->pmax64_state = 1;
@@ -517,7 +524,9 @@ int pstep_stage_temp(pstep_handle h) {
     // the fused advance kernel interpolated T with the field bound at that time; a
     // temperature bound since then (the reference forms it after Send_Recv,
     // grid.cpp:676) is interpolated here
-    if (h->fields_t != h->fields_t_at_advance) TRY(f64_temp_gather(h));
+    h->t_rebound = h->fields_t != h->fields_t_at_advance ? 1 : 0;
+    if (h->t_rebound || h->t_pending) TRY(f64_temp_gather(h));
+    h->t_pending = 0;
     prof_begin(h, PSTEP_PHASE_SORT);
     TRY(sort_by_node(h, h->s.key_new, h->csr_new));
     prof_end(h, PSTEP_PHASE_SORT);
@@ -696,6 +705,8 @@ int pstep_get_particle_array(pstep_handle h, int id, void *dst, int on_device) {
       int q = id - PSTEP_X_NP1;
       src = h->np1_is_base ? h->s.base[q] : h->s.np1[q];
     } else {
+      // asked for before pstep_stage_temp: with the temperature bound now
+      if (h->t_pending) TRY(f64_temp_gather(h));
       src = h->s.rhs_t;
     }
     double *tmp = (double *)h->perm_tmp;

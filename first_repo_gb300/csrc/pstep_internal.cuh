@@ -128,6 +128,8 @@ struct pstep_ctx {
   // state machine
   int fields_u, fields_t, primed;
   int fields_t_at_advance;  // temperature binding seen by the fused advance kernel
+  int t_rebound;            // FP64 form: the last stage's temperature was bound after its advance
+  int t_pending;            // FP64 form: this stage's advance left the temperature gather to stage_temp
   int64_t stages_done;
   int timed;
   int phase;  // 0: idle, 1: after interp_advance_deposit, 2: after wrap, 3: after stage_temp
