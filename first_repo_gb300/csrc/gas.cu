@@ -2,19 +2,17 @@
 // handle: the two-way-coupled gas response that turns the particle step's
 // deposits into the gas disturbance (the learned correction's training runs).
 //
-// Every operation is its own kernel over the reference's loop range (ghost
-// layers included where tensor0.cpp/tensor1.cpp include them), each element
-// computed with the reference's operand order and no FMA contraction (this
-// file is compiled with -fmad=false). Stencil results get their periodic ghost
-// layers from one refresh kernel (each ghost cell copies its periodic image,
-// which is what communicator.cpp:177-278's x, y, z passes leave). The Poisson
-// solve is the reference's fixed-point iteration on constant-coefficient FFT
-// solves (poisson.cpp:391-462); the FFT is an iterative radix-2 transform, one
-// CTA per line in shared memory, with host-computed twiddles and
-// modified-wavenumber tables. Interior sums (mean) and maxima are two-pass
-// reductions in a fixed order of their own, so they round differently from
-// the reference's sequential i-outer loop: that is the only source of
-// difference from the CPU restatement.
+// Compiled with -fmad=false; every element is computed with the reference's operand order
+// except where a comment says otherwise. A kernel computes the interior cells and writes every
+// value to its periodic ghost images too (what communicator.cpp:177-278's x, y, z passes leave),
+// so stencils read the ghost layers and no refresh pass runs. GB300's FP64 rate (two lanes per
+// SM and clock) bounds the step once the passes are fused: an operation a cell at 128^3 costs
+// 3.3 us. The Poisson solve is the reference's fixed-point iteration on constant-coefficient FFT
+// solves (poisson.cpp:391-462), five kernels an iteration: residual + x transform, y, z with the
+// division by the wavenumbers and the way back, y, x + the update of P and its largest change.
+// Interior sums (mean) and maxima are two-pass reductions in a fixed order of their own, so they
+// round differently from the reference's sequential i-outer loop; together with the transform
+// that is the source of difference from the CPU restatement.
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -28,12 +26,13 @@ constexpr double kPost[4] = {1. / 6., 1. / 3., 1. / 3., 1. / 6.};
 constexpr int kT = 256;
 
 enum {
-  F_RU = 0, F_RU_INT = 3, F_RU_NEW = 6, F_RU_NP1 = 9, F_RHS_RU = 12, F_U = 15, F_RHO_FACE = 18, F_DUMMY = 21,
-  F_DUMMY2 = 24, F_PDUMMY = 27, F_P = 30, F_RHS_POIS, F_C, F_RHO, F_RHO_INT, F_RHO_NEW, F_RHO_NP1, F_RHS_RHO, F_T,
-  F_DIV, F_RHS_PT, F_CENTER, F_RHS_NEW, F_NF
+  F_RU = 0, F_RU_INT = 3, F_RU_NEW = 6, F_RU_NP1 = 9, F_RHS_RU = 12, F_U = 15, F_IRF = 18 /* 1 / Rho_face */,
+  F_P = 21, F_RHS_POIS, F_C, F_RHO, F_RHO_INT, F_RHO_NEW, F_RHO_NP1, F_IRHO /* 1 / Rho_new */, F_T, F_DIV, F_RHS_PT,
+  F_CENTER, F_NF
 };
-// device scalars: P0 and its stage copies, dP0/dt, mean of RHS_Part_Temp, scratch mean, solve error
-enum { S_P0, S_P0_INT, S_P0_NEW, S_P0_NP1, S_DP0, S_MEAN_E, S_MEAN, S_ERR, S_N };
+// device scalars: P0 and its stage copies, mean of RHS_Part_Temp, scratch means (3), solve
+// error (as bits), P0_new / R, -R / (Cp P0_new Vcell)
+enum { S_P0, S_P0_INT, S_P0_NEW, S_P0_NP1, S_MEAN_E, S_MEAN, S_MEAN_Y, S_MEAN_Z, S_ERR, S_T, S_SRC, S_N };
 
 struct Dim {
   int n, G;
@@ -46,236 +45,445 @@ __device__ __forceinline__ size_t ix(const Dim &d, int i, int j, int k) {
 
 __device__ __forceinline__ int64_t gtid() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 
-// element e of the box [lo, lo+ext)
-__device__ __forceinline__ bool in_box(int64_t e, int l0, int l1, int l2, int e0, int e1, int e2, int &i, int &j,
-                                       int &k) {
-  if (e >= (int64_t)e0 * e1 * e2) return false;
-  i = l0 + (int)(e % e0);
-  j = l1 + (int)((e / e0) % e1);
-  k = l2 + (int)(e / ((int64_t)e0 * e1));
-  return true;
+// interior cell of a thread of a (32, 8) block on a (n/32, n/8, n) grid
+__device__ __forceinline__ bool cell_of(const Dim &d, int &i, int &j, int &k) {
+  i = blockIdx.x * 32 + threadIdx.x + 1;
+  j = blockIdx.y * 8 + threadIdx.y + 1;
+  k = blockIdx.z + 1;
+  return i <= d.n && j <= d.n;
 }
 
-// tensor0::Equal_Div_F2C (tensor0.cpp:303-310), i, j, k in [0, n]
-__global__ void k_div_f2c(Dim d, double *out, const double *tx, const double *ty, const double *tz) {
-  int i, j, k;
-  if (!in_box(gtid(), 0, 0, 0, d.n + 1, d.n + 1, d.n + 1, i, j, k)) return;
-  out[ix(d, i, j, k)] = (tx[ix(d, i + 1, j, k)] - tx[ix(d, i, j, k)]) * d.idx +
-                        (ty[ix(d, i, j + 1, k)] - ty[ix(d, i, j, k)]) * d.idx +
-                        (tz[ix(d, i, j, k + 1)] - tz[ix(d, i, j, k)]) * d.idx;
+// v at interior cell (i, j, k) and its periodic images in the ghost layers
+struct Images {
+  int i2, j2, k2;
+  __device__ __forceinline__ Images(const Dim &d, int i, int j, int k)
+      : i2(i == 1 ? d.n + 1 : (i == d.n ? 0 : -1)), j2(j == 1 ? d.n + 1 : (j == d.n ? 0 : -1)),
+        k2(k == 1 ? d.n + 1 : (k == d.n ? 0 : -1)) {}
+  __device__ __forceinline__ void put(const Dim &d, double *f, int i, int j, int k, double v) const {
+    f[ix(d, i, j, k)] = v;
+    if (i2 < 0 && j2 < 0 && k2 < 0) return;
+    for (int c = 0; c < 2; ++c) {
+      const int kk = c ? k2 : k;
+      if (kk < 0) continue;
+      for (int b = 0; b < 2; ++b) {
+        const int jj = b ? j2 : j;
+        if (jj < 0) continue;
+        for (int a = 0; a < 2; ++a) {
+          const int ii = a ? i2 : i;
+          if (ii >= 0 && (a | b | c)) f[ix(d, ii, jj, kk)] = v;
+        }
+      }
+    }
+  }
+};
+
+struct V3 {
+  double *p[3];
+};
+struct CV3 {
+  const double *p[3];
+};
+
+// x / y with r = 1 / y at hand: one Newton step on the quotient (Markstein), which gives the
+// correctly rounded quotient for normal operands at 3 operations instead of a division's ten
+__device__ __forceinline__ double quotient(double x, double y, double r) {
+  const double q = x * r;
+  return fma(fma(-q, y, x), r, q);
 }
 
-// tensor0::Equal_Del2 (tensor0.cpp:312-320), interior
-__global__ void k_del2(Dim d, double *out, const double *t) {
+// Update_Rho (grid.cpp:327-333): RHS_Rho = div(RU_int), Rho_np1, Rho_new; 1 / Rho_new beside it
+__global__ void k_update_rho(Dim d, CV3 ru, const double *rho, double *np1, double *rnew, double *irho, double a_post,
+                             double a_pre, int last) {
   int i, j, k;
-  if (!in_box(gtid(), 1, 1, 1, d.n, d.n, d.n, i, j, k)) return;
+  if (!cell_of(d, i, j, k)) return;
+  const Images im(d, i, j, k);
+  const size_t c = ix(d, i, j, k), off[3] = {1, (size_t)d.G, (size_t)d.G * d.G};
+  const double rate = (ru.p[0][c + off[0]] - ru.p[0][c]) * d.idx + (ru.p[1][c + off[1]] - ru.p[1][c]) * d.idx +
+                      (ru.p[2][c + off[2]] - ru.p[2][c]) * d.idx;
+  const double a = np1[c] + a_post * rate;
+  const double v = last ? a : rho[c] + a_pre * rate;
+  im.put(d, np1, i, j, k, a);
+  im.put(d, rnew, i, j, k, v);
+  im.put(d, irho, i, j, k, 1. / v);
+}
+
+// U = RU_int / Rho_face(rho) (grid.cpp:662), T = (P0_new / R) / Rho_new (grid.cpp:676) and
+// div(U) (the viscous term's, grid.cpp:389)
+__global__ void k_velocity(Dim d, CV3 ru, CV3 irf, const double *rho, const double *rnew, const double *irho,
+                           const double *sc, V3 u, double *T, double *div) {
+  int i, j, k;
+  if (!cell_of(d, i, j, k)) return;
+  const Images im(d, i, j, k);
+  const size_t c = ix(d, i, j, k), off[3] = {1, (size_t)d.G, (size_t)d.G * d.G};
+  double s = 0.0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const size_t o = off[a];
+    const double lo = quotient(ru.p[a][c], (rho[c] + rho[c - o]) * 0.5, irf.p[a][c]);
+    const double hi = quotient(ru.p[a][c + o], (rho[c + o] + rho[c]) * 0.5, irf.p[a][c + o]);
+    im.put(d, u.p[a], i, j, k, lo);
+    s = a ? s + (hi - lo) * d.idx : (hi - lo) * d.idx;
+  }
+  im.put(d, div, i, j, k, s);
+  im.put(d, T, i, j, k, quotient(sc[S_T], rnew[c], irho[c]));
+}
+
+// 1 / Rho_face(rho) of the start (grid::Initialize), and U, T there
+__global__ void k_init_fields(Dim d, CV3 ru, const double *rho, const double *sc, V3 irf, V3 u, double *T) {
+  int i, j, k;
+  if (!cell_of(d, i, j, k)) return;
+  const Images im(d, i, j, k);
+  const size_t c = ix(d, i, j, k), off[3] = {1, (size_t)d.G, (size_t)d.G * d.G};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const double f = (rho[c] + rho[c - off[a]]) * 0.5;
+    im.put(d, irf.p[a], i, j, k, 1. / f);
+    im.put(d, u.p[a], i, j, k, ru.p[a][c] / f);
+  }
+  im.put(d, T, i, j, k, sc[S_T] / rho[c]);
+}
+
+struct RuConst {
+  double part, mu3, mu, a_force, a_const, rho0, g[3], post, pre;
+  int force, gravity, last;
+};
+
+// Update_RU_WOP (grid.cpp:387-425): RHS_RU = particle source + mu/3 grad(div U) + mu del2(U)
+// - div(U RU) + forcing + buoyancy, RU_np1 and RU_new; 1 / Rho_face(Rho_new) beside it. The
+// convective fluxes' two halves are one factor 1/4 (a power of two: the same rounding).
+__global__ void __launch_bounds__(256) k_update_ru(Dim d, RuConst q, CV3 u, CV3 rui, CV3 ru, const double *div,
+                                                   const double *rho, const double *rnew, V3 rhs, V3 np1, V3 runew,
+                                                   V3 irf) {
+  int i, j, k;
+  if (!cell_of(d, i, j, k)) return;
+  const Images im(d, i, j, k);
+  const size_t c = ix(d, i, j, k), off[3] = {1, (size_t)d.G, (size_t)d.G * d.G};
+  const double quarter = 0.25 * d.idx;
+  const double dc = div[c];
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    const double *ue = u.p[e];
+    const double uc = ue[c], two = 2 * uc;
+    double lap = 0.0, conv = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const size_t o = off[a];
+      const double up = ue[c + o], um = ue[c - o];
+      const double l = (up - two + um) * d.idx2;
+      lap = a ? lap + l : l;
+      // face(U_e, a) face(RU_a, e) at c + a and at c, each without its factor 1/4
+      const double hi = (up + uc) * (rui.p[a][c + o] + rui.p[a][c + o - off[e]]);
+      const double lo = (uc + um) * (rui.p[a][c] + rui.p[a][c - off[e]]);
+      conv = a ? conv + (hi - lo) * quarter : (hi - lo) * quarter;
+    }
+    const double gd = (dc - div[c - off[e]]) * d.idx;
+    double r = q.part * rhs.p[e][c] + q.mu3 * gd + q.mu * lap;
+    r -= conv;
+    if (q.force) {
+      r += q.a_force * rui.p[e][c];
+      if (e == 0) r += q.a_const;
+    }
+    if (q.gravity) r += ((rho[c] + rho[c - off[e]]) * 0.5 - q.rho0) * q.g[e];
+    const double a = np1.p[e][c] + q.post * r;
+    im.put(d, rhs.p[e], i, j, k, r);
+    im.put(d, np1.p[e], i, j, k, a);
+    im.put(d, runew.p[e], i, j, k, q.last ? a : ru.p[e][c] + q.pre * r);
+    im.put(d, irf.p[e], i, j, k, 1. / ((rnew[c] + rnew[c - off[e]]) * 0.5));
+  }
+}
+
+// Compute_Div_U_new (grid.cpp:556-563) and Compute_RHS_Pois (:629-637) without its mean:
+// divergence = k/Cp del2(1/Rho_new) - R/(Cp P0_new Vcell) RHS_Part_Temp, U = RU_new / Rho_face,
+// RHS = (div(U) - divergence) / (dt pre); and the solve's centre coefficient
+// -1 / I_F2C(1 / Rho_face) (poisson.cpp:391-400)
+__global__ void __launch_bounds__(256) k_rhs_pois(Dim d, CV3 runew, CV3 irf, const double *rnew, const double *irho,
+                                                  const double *pt, const double *sc, double kcp, double inv_dt,
+                                                  int cooling, V3 u, double *div, double *rhs, double *centre) {
+  int i, j, k;
+  if (!cell_of(d, i, j, k)) return;
+  const Images im(d, i, j, k);
+  const size_t c = ix(d, i, j, k), off[3] = {1, (size_t)d.G, (size_t)d.G * d.G};
+  const double two = 2 * irho[c];
+  double lap = 0.0, s = 0.0, m = 0.0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const size_t o = off[a];
+    const double l = (irho[c + o] - two + irho[c - o]) * d.idx2;
+    lap = a ? lap + l : l;
+    const double fl = irf.p[a][c], fh = irf.p[a][c + o];
+    const double lo = quotient(runew.p[a][c], (rnew[c] + rnew[c - o]) * 0.5, fl);
+    const double hi = quotient(runew.p[a][c + o], (rnew[c + o] + rnew[c]) * 0.5, fh);
+    im.put(d, u.p[a], i, j, k, lo);
+    s = a ? s + (hi - lo) * d.idx : (hi - lo) * d.idx;
+    m = a ? m + (fl + fh) * 0.5 : (fl + fh) * 0.5;
+  }
+  const double src = cooling ? pt[c] - sc[S_MEAN] : pt[c];
+  const double dv = kcp * lap + sc[S_SRC] * src;
+  im.put(d, div, i, j, k, dv);
+  rhs[c] = (s - dv) * inv_dt;
+  centre[c] = -1. / ((1. / 3.) * m);
+}
+
+// Update_RU_WP (grid.cpp:651-657) and TimeAdvance_RK4 (:705-712)
+__global__ void k_pressure_step(Dim d, const double *P, CV3 runew, V3 np1, V3 rui, const double *rnew, double *rhoi,
+                                double a_post, double a_pre, int last) {
+  int i, j, k;
+  if (!cell_of(d, i, j, k)) return;
+  const Images im(d, i, j, k);
+  const size_t c = ix(d, i, j, k), off[3] = {1, (size_t)d.G, (size_t)d.G * d.G};
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    const double g = (P[c] - P[c - off[e]]) * d.idx;
+    const double a = np1.p[e][c] + a_post * g;
+    im.put(d, np1.p[e], i, j, k, a);
+    im.put(d, rui.p[e], i, j, k, last ? a : runew.p[e][c] + a_pre * g);
+  }
+  im.put(d, rhoi, i, j, k, rnew[c]);
+}
+
+// Correct_mean_RU (grid.cpp:566-572) and TimeAdvance (:315-325)
+__global__ void k_end_step(Dim d, V3 np1, V3 ru, const double *rho_np1, double *rho, const double *sc, double mean_x) {
+  int i, j, k;
+  if (!cell_of(d, i, j, k)) return;
+  const Images im(d, i, j, k);
   const size_t c = ix(d, i, j, k);
-  out[c] = (t[ix(d, i + 1, j, k)] - 2 * t[c] + t[ix(d, i - 1, j, k)]) * d.idx2 +
-           (t[ix(d, i, j + 1, k)] - 2 * t[c] + t[ix(d, i, j - 1, k)]) * d.idx2 +
-           (t[ix(d, i, j, k + 1)] - 2 * t[c] + t[ix(d, i, j, k - 1)]) * d.idx2;
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    double v = np1.p[e][c] - sc[S_MEAN + e];
+    if (e == 0) v += mean_x;
+    im.put(d, np1.p[e], i, j, k, v);
+    im.put(d, ru.p[e], i, j, k, v);
+  }
+  im.put(d, rho, i, j, k, rho_np1[c]);
 }
 
-// tensor0::Equal_I{x,y,z}_C2F (tensor0.cpp:353-378): (t(c) + t(c - e_axis)) * 0.5
-// with the axis index in [1, n+1] and the others over the ghosted range;
-// with grad != 0, tensor1::Equal_Grad_C2F's component (t(c) - t(c - e_axis)) * idx
-__global__ void k_c2f(Dim d, double *out, const double *t, int axis, int grad) {
-  int i, j, k;
-  const int a0 = axis == 0, a1 = axis == 1, a2 = axis == 2;
-  if (!in_box(gtid(), a0, a1, a2, d.G - a0, d.G - a1, d.G - a2, i, j, k)) return;
-  const size_t c = ix(d, i, j, k), m = ix(d, i - a0, j - a1, k - a2);
-  out[c] = grad ? (t[c] - t[m]) * d.idx : (t[c] + t[m]) * 0.5;
-}
-
-// tensor0::Equal_I_F2C(tensor1) (tensor0.cpp:408-416), [0, n]^3
-__global__ void k_i_f2c_vec(Dim d, double *out, const double *tx, const double *ty, const double *tz) {
-  int i, j, k;
-  if (!in_box(gtid(), 0, 0, 0, d.n + 1, d.n + 1, d.n + 1, i, j, k)) return;
-  const double third = 1. / 3.;
-  const size_t c = ix(d, i, j, k);
-  out[c] = third * ((tx[c] + tx[ix(d, i + 1, j, k)]) * 0.5 + (ty[c] + ty[ix(d, i, j + 1, k)]) * 0.5 +
-                    (tz[c] + tz[ix(d, i, j, k + 1)]) * 0.5);
-}
-
-// periodic ghost layers: every ghost cell takes its periodic image
-__global__ void k_refresh(Dim d, double *f) {
-  int i, j, k;
-  if (!in_box(gtid(), 0, 0, 0, d.G, d.G, d.G, i, j, k)) return;
-  const int n = d.n;
-  const int si = i == 0 ? n : (i == n + 1 ? 1 : i);
-  const int sj = j == 0 ? n : (j == n + 1 ? 1 : j);
-  const int sk = k == 0 ? n : (k == n + 1 ? 1 : k);
-  if (si != i || sj != j || sk != k) f[ix(d, i, j, k)] = f[ix(d, si, sj, sk)];
-}
-
-// ------------------------------------------------------------ elementwise
-__global__ void k_lin2(double *out, double a, const double *x, double b, const double *y, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) out[q] = a * x[q] + b * y[q];
-}
-__global__ void k_lin3(double *out, double a, const double *x, double b, const double *y, double c, const double *z,
-                       int64_t n) {
-  int64_t q = gtid();
-  if (q < n) out[q] = a * x[q] + b * y[q] + c * z[q];
-}
-__global__ void k_axpy(double *y, double a, const double *x, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) y[q] += a * x[q];
-}
-__global__ void k_div(double *out, const double *x, const double *y, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) out[q] = x[q] / y[q];
-}
-__global__ void k_sdiv(double *out, double a, const double *y, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) out[q] = a / y[q];
-}
-__global__ void k_mul(double *x, const double *y, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) x[q] *= y[q];
-}
-__global__ void k_sub(double *x, const double *y, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) x[q] -= y[q];
-}
-__global__ void k_add(double *x, const double *y, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) x[q] += y[q];
-}
-__global__ void k_adds(double *x, double s, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) x[q] += s;
-}
-__global__ void k_subs_dev(double *x, const double *s, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) x[q] -= *s;
-}
-__global__ void k_muls(double *x, double s, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) x[q] *= s;
-}
-__global__ void k_mul_to(double *out, const double *x, double s, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) out[q] = x[q] * s;
-}
 __global__ void k_fill(double *x, double s, int64_t n) {
   int64_t q = gtid();
   if (q < n) x[q] = s;
 }
-// T = (P0_x / R) / rho (grid.cpp:221, :676)
-__global__ void k_t_from_rho(double *T, const double *rho, const double *sc, int which, double R, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) {
-    const double a = sc[which] / R;
-    T[q] = a / rho[q];
-  }
-}
-// divergence = k/Cp * del2(1/rho_new) - R/(Cp*P0_new*Vcell) * RHS_Part_Temp (grid.cpp:562)
-__global__ void k_div_u(double *div, const double *dy, const double *dz, const double *sc, double a, double R, double cp,
-                        double vcell, int64_t n) {
-  int64_t q = gtid();
-  if (q < n) {
-    const double b = -R / (cp * sc[S_P0_NEW] * vcell);
-    div[q] = a * dy[q] + b * dz[q];
-  }
-}
-// Update_P0 (grid.cpp:539-554); the mean is already in sc[S_MEAN_E]
-__global__ void k_update_p0(double *sc, int k3, double dt_post, double dt_pre, double R, double cv, int cooling) {
-  const double dp0 = cooling ? 0.0 : -R / cv * sc[S_MEAN_E];
-  sc[S_DP0] = dp0;
-  sc[S_P0_NP1] += dt_post * dp0;
-  sc[S_P0_NEW] = k3 ? sc[S_P0_NP1] : sc[S_P0] + dt_pre * dp0;
-}
-__global__ void k_scalar_copy(double *sc, int dst, int src) { sc[dst] = sc[src]; }
 
 // ----------------------------------------------------------- reductions
-// one warp per (j, k) interior row
-__global__ void k_rows(Dim d, const double *f, int mode, double *rows) {
+// one warp per (j, k) interior row; blockIdx.y picks the field
+__global__ void k_rows(Dim d, CV3 f, double *rows) {
   const int64_t w = gtid() >> 5;
   const int lane = threadIdx.x & 31;
   const int64_t nr = (int64_t)d.n * d.n;
   if (w >= nr) return;
   const int j = (int)(w % d.n) + 1, k = (int)(w / d.n) + 1;
-  const double *r = f + ix(d, 0, j, k);
+  const double *r = f.p[blockIdx.y] + ix(d, 0, j, k);
   double s = 0.0;
-  for (int i = lane + 1; i <= d.n; i += 32) s = mode ? fmax(s, fabs(r[i])) : s + r[i];
+  for (int i = lane + 1; i <= d.n; i += 32) s += r[i];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double v = __shfl_down_sync(0xffffffffu, s, o);
-    s = mode ? fmax(s, v) : s + v;
-  }
-  if (lane == 0) rows[w] = s;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) rows[blockIdx.y * nr + w] = s;
 }
-// one block: sum (mode 0, times inv) or maximum (mode 1) of the row values
-__global__ void k_rows_total(const double *rows, int64_t nr, int mode, double inv, double *out) {
-  __shared__ double sm[256];
+
+// Update_P0 (grid.cpp:539-554) from the mean of RHS_Part_Temp
+struct P0Const {
+  int on, k3, cooling;
+  double post, pre, r, cv, cp, vcell;
+};
+__device__ __forceinline__ void update_p0(double *sc, const P0Const &q) {
+  const double dp0 = q.cooling ? 0.0 : -q.r / q.cv * sc[S_MEAN_E];
+  sc[S_P0_NP1] += q.post * dp0;
+  sc[S_P0_NEW] = q.k3 ? sc[S_P0_NP1] : sc[S_P0] + q.pre * dp0;
+  sc[S_T] = sc[S_P0_NEW] / q.r;
+  sc[S_SRC] = -q.r / (q.cp * sc[S_P0_NEW] * q.vcell);
+}
+
+// one block per field: sum of its row sums times inv into sc[slot + field]; then Update_P0
+__global__ void __launch_bounds__(1024) k_rows_total(const double *rows, int64_t nr, double inv, double *sc, int slot,
+                                                     P0Const q) {
+  __shared__ double sm[32];
+  const double *r0 = rows + blockIdx.x * nr;
   double s = 0.0;
-  for (int64_t r = threadIdx.x; r < nr; r += blockDim.x) s = mode ? fmax(s, rows[r]) : s + rows[r];
-  sm[threadIdx.x] = s;
+  for (int64_t r = threadIdx.x; r < nr; r += 1024) s += r0[r];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sm[threadIdx.x] = mode ? fmax(sm[threadIdx.x], sm[threadIdx.x + o]) : sm[threadIdx.x] + sm[threadIdx.x + o];
-    __syncthreads();
+  if (threadIdx.x < 32) {
+    s = sm[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) {
+      sc[slot + blockIdx.x] = s * inv;
+      if (q.on) update_p0(sc, q);
+    }
   }
-  if (threadIdx.x == 0) *out = mode ? sm[0] : sm[0] * inv;
 }
+__global__ void k_scalar_copy(double *sc, int dst, int src) { sc[dst] = sc[src]; }
 
 // ------------------------------------------------------------------ FFT
-__global__ void k_pack(Dim d, double2 *z, const double *rhs) {
-  int i, j, k;
-  if (!in_box(gtid(), 0, 0, 0, d.n, d.n, d.n, i, j, k)) return;
-  z[((size_t)k * d.n + j) * d.n + i] = make_double2(rhs[ix(d, i + 1, j + 1, k + 1)], 0.0);
-}
-
-// one CTA per line along `axis`; radix-2 decimation in time after a bit-reversal load
-__global__ void k_fft_line(double2 *z, int n, int logn, int axis, const double2 *__restrict__ tw) {
-  extern __shared__ double2 s[];
-  const int64_t l = blockIdx.x;
-  const int64_t nn = (int64_t)n * n;
-  int64_t base, stride;
-  if (axis == 0) { base = l * n; stride = 1; }
-  else if (axis == 1) { base = (l / n) * nn + (l % n); stride = n; }
-  else { base = l; stride = nn; }
-  for (int e = threadIdx.x; e < n; e += blockDim.x) s[__brev((unsigned)e) >> (32 - logn)] = z[base + e * stride];
+// The right-hand side is real: two rows go through one complex transform along x and half the
+// spectrum (n/2 + 1 bins) through y and z, 1/2 the FP64 work of a complex transform. Lines are
+// transformed in shared memory, W of them side by side (element e of line w at e W + w), so that
+// y and z move W neighbouring bins per row. Radix 2 in time with a +- w b as six fused
+// operations (a + w b in four, the other sum as 2 a - that), the first two levels free of
+// products: 38 operations a pair of points at n = 128 instead of 70.
+__device__ __forceinline__ void fft_lines(double2 *s, int n, int logn, int W, const double2 *__restrict__ tw, int inv) {
+  const double sg = inv ? -1.0 : 1.0;
+  for (int t = threadIdx.x; t < W * (n >> 2); t += blockDim.x) {
+    const int w = t % W, e = (t / W) << 2;
+    double2 *p = s + e * W + w;
+    const double2 a0 = p[0], a1 = p[W], a2 = p[2 * W], a3 = p[3 * W];
+    const double2 b0 = make_double2(a0.x + a1.x, a0.y + a1.y), b1 = make_double2(a0.x - a1.x, a0.y - a1.y);
+    const double2 b2 = make_double2(a2.x + a3.x, a2.y + a3.y), b3 = make_double2(a2.x - a3.x, a2.y - a3.y);
+    // w = -i forward, +i backward
+    const double2 m = inv ? make_double2(-b3.y, b3.x) : make_double2(b3.y, -b3.x);
+    p[0] = make_double2(b0.x + b2.x, b0.y + b2.y);
+    p[W] = make_double2(b1.x + m.x, b1.y + m.y);
+    p[2 * W] = make_double2(b0.x - b2.x, b0.y - b2.y);
+    p[3 * W] = make_double2(b1.x - m.x, b1.y - m.y);
+  }
   __syncthreads();
-  for (int len = 2; len <= n; len <<= 1) {
-    const int half = len >> 1, step = n / len;
-    for (int q = threadIdx.x; q < n / 2; q += blockDim.x) {
-      const int kk = q % half, ia = (q / half) * len + kk, ib = ia + half;
-      const double2 w = tw[kk * step];
-      const double2 a = s[ia], b = s[ib];
-      const double tr = b.x * w.x - b.y * w.y;
-      const double ti = b.x * w.y + b.y * w.x;
-      s[ib] = make_double2(a.x - tr, a.y - ti);
-      s[ia] = make_double2(a.x + tr, a.y + ti);
+  for (int lh = 2; lh < logn; ++lh) {
+    const int half = 1 << lh, step = n >> (lh + 1);
+    for (int t = threadIdx.x; t < W * (n >> 1); t += blockDim.x) {
+      const int w = t % W, q = t / W, kk = q & (half - 1);
+      double2 *pa = s + ((((q & ~(half - 1)) << 1) | kk)) * W + w, *pb = pa + half * W;
+      const double2 f = tw[kk * step], a = *pa, b = *pb;
+      const double wy = sg * f.y;
+      const double rx = fma(-wy, b.y, fma(f.x, b.x, a.x)), ry = fma(wy, b.x, fma(f.x, b.y, a.y));
+      *pa = make_double2(rx, ry);
+      *pb = make_double2(fma(2.0, a.x, -rx), fma(2.0, a.y, -ry));
     }
     __syncthreads();
   }
-  for (int e = threadIdx.x; e < n; e += blockDim.x) z[base + e * stride] = s[e];
 }
+__device__ __forceinline__ int bitrev(int e, int logn) { return (int)(__brev((unsigned)e) >> (32 - logn)); }
 
-__global__ void k_kmod_div(int n, double2 *z, const double *kmod) {
-  const int64_t c = gtid();
-  if (c >= (int64_t)n * n * n) return;
-  const int i = (int)(c % n), j = (int)((c / n) % n), k = (int)(c / ((int64_t)n * n));
-  if (i + j + k > 0) {
-    const double den = kmod[i] + kmod[j] + kmod[k];
-    double2 v = z[c];
-    v.y /= den;
-    v.x /= den;
-    z[c] = v;
+// One iteration's right-hand side (poisson.cpp:405-420), ((div(C grad P) - (RHS - mean)) centre),
+// and its transform along x: W pairs of rows per CTA. The flux differences are summed with
+// fused operations and scaled by idx^2 once.
+__global__ void __launch_bounds__(256) k_res_fft_x(Dim d, int logn, int W, const double2 *__restrict__ tw,
+                                                   const double *P, CV3 irf, const double *rhs, const double *centre,
+                                                   double *sc, double2 *z) {
+  extern __shared__ double2 s[];
+  const int n = d.n, nh = n / 2 + 1;
+  const int64_t row0 = (int64_t)blockIdx.x * 2 * W;
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc[S_ERR] = 0.0;
+  const double mean = sc[S_MEAN], idx2 = d.idx * d.idx;
+  const size_t oy = (size_t)d.G, oz = (size_t)d.G * d.G;
+  for (int t = threadIdx.x; t < 2 * W * n; t += blockDim.x) {
+    const int i = t & (n - 1), r = t >> logn;
+    const int64_t row = row0 + r;
+    const size_t c = ix(d, i + 1, (int)(row & (n - 1)) + 1, (int)(row >> logn) + 1);
+    const double pc = P[c];
+    double a = irf.p[0][c + 1] * (P[c + 1] - pc);
+    a = fma(-irf.p[0][c], pc - P[c - 1], a);
+    a = fma(irf.p[1][c + oy], P[c + oy] - pc, a);
+    a = fma(-irf.p[1][c], pc - P[c - oy], a);
+    a = fma(irf.p[2][c + oz], P[c + oz] - pc, a);
+    a = fma(-irf.p[2][c], pc - P[c - oz], a);
+    const double v = fma(a, idx2, mean - rhs[c]) * centre[c];
+    reinterpret_cast<double *>(s)[2 * (bitrev(i, logn) * W + (r >> 1)) + (r & 1)] = v;
+  }
+  __syncthreads();
+  fft_lines(s, n, logn, W, tw, 0);
+  // the two rows' spectra, each twice (the factor 1/2 is in k_fft_x_back's scale)
+  for (int t = threadIdx.x; t < W * nh; t += blockDim.x) {
+    const int kx = t % nh, w = t / nh;
+    const double2 a = s[kx * W + w], b = s[((n - kx) & (n - 1)) * W + w];
+    double2 *o = z + (row0 + 2 * w) * nh + kx;
+    o[0] = make_double2(a.x + b.x, a.y - b.y);
+    o[nh] = make_double2(a.y + b.y, b.x - a.x);
   }
 }
 
-__global__ void k_scatter(Dim d, double *out, const double *lin) {
-  int i, j, k;
-  if (!in_box(gtid(), 0, 0, 0, d.n, d.n, d.n, i, j, k)) return;
-  out[ix(d, i + 1, j + 1, k + 1)] = lin[((size_t)k * d.n + j) * d.n + i];
+// along y, in place: CTA (tile of W bins, plane)
+__global__ void __launch_bounds__(256) k_fft_y(int n, int logn, int W, const double2 *__restrict__ tw, int inv,
+                                               double2 *z) {
+  extern __shared__ double2 s[];
+  const int nh = n / 2 + 1, x0 = blockIdx.x * W;
+  double2 *pl = z + (int64_t)blockIdx.y * n * nh;
+  for (int t = threadIdx.x; t < W * n; t += blockDim.x) {
+    const int w = t % W, e = t / W;
+    s[bitrev(e, logn) * W + w] = x0 + w < nh ? pl[(int64_t)e * nh + x0 + w] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  fft_lines(s, n, logn, W, tw, inv);
+  for (int t = threadIdx.x; t < W * n; t += blockDim.x) {
+    const int w = t % W, e = t / W;
+    if (x0 + w < nh) pl[(int64_t)e * nh + x0 + w] = s[t];
+  }
 }
 
-__global__ void k_unpack(Dim d, double *out, const double2 *z, double tot) {
+// along z, division by the modified wavenumbers (the zero mode is left alone) and back
+__global__ void __launch_bounds__(256) k_fft_z(int n, int logn, int W, const double2 *__restrict__ tw,
+                                               const double *__restrict__ kmod, double2 *z) {
+  extern __shared__ double2 s[];
+  const int nh = n / 2 + 1;
+  const int64_t plane = (int64_t)n * nh;
+  double2 *col = z + (int64_t)blockIdx.x * W;
+  for (int t = threadIdx.x; t < W * n; t += blockDim.x) {
+    const int w = t % W, e = t / W;
+    s[bitrev(e, logn) * W + w] = col[e * plane + w];
+  }
+  __syncthreads();
+  fft_lines(s, n, logn, W, tw, 0);
+  for (int t = threadIdx.x; t < W * n; t += blockDim.x) {
+    const int w = t % W, e = t / W, r = bitrev(e, logn);
+    if (r < e) continue;  // this thread takes both of a pair
+    const int c = (int)blockIdx.x * W + w;
+    const double kxy = kmod[c % nh] + kmod[c / nh];
+    const double de = kxy + kmod[e], dr = kxy + kmod[r];
+    const double fe = c + e > 0 ? 1.0 / de : 1.0, fr = r == e ? fe : 1.0 / dr;
+    const double2 a = s[e * W + w], b = s[r * W + w];
+    s[r * W + w] = make_double2(a.x * fe, a.y * fe);
+    if (r != e) s[e * W + w] = make_double2(b.x * fr, b.y * fr);
+  }
+  __syncthreads();
+  fft_lines(s, n, logn, W, tw, 1);
+  for (int t = threadIdx.x; t < W * n; t += blockDim.x) {
+    const int w = t % W, e = t / W;
+    col[e * plane + w] = s[t];
+  }
+}
+
+// back along x: P += the solution, sc[S_ERR] = its largest magnitude (non-negative doubles order
+// like their bits)
+__global__ void __launch_bounds__(256) k_fft_x_back(Dim d, int logn, int W, const double2 *__restrict__ tw,
+                                                    const double2 *z, double scale, double *P, double *sc) {
+  extern __shared__ double2 s[];
+  __shared__ double top[8];
+  const int n = d.n, nh = n / 2 + 1;
+  const int64_t row0 = (int64_t)blockIdx.x * 2 * W;
+  for (int t = threadIdx.x; t < W * nh; t += blockDim.x) {
+    const int kx = t % nh, w = t / nh;
+    const double2 *o = z + (row0 + 2 * w) * nh + kx;
+    const double2 a = o[0], b = o[nh];
+    s[bitrev(kx, logn) * W + w] = make_double2(a.x - b.y, a.y + b.x);
+    if (kx > 0 && kx < n / 2) s[bitrev(n - kx, logn) * W + w] = make_double2(a.x + b.y, b.x - a.y);
+  }
+  __syncthreads();
+  fft_lines(s, n, logn, W, tw, 1);
+  double m = 0.0;
+  for (int t = threadIdx.x; t < 2 * W * n; t += blockDim.x) {
+    const int i = t & (n - 1), r = t >> logn;
+    const int64_t row = row0 + r;
+    const int j = (int)(row & (n - 1)) + 1, k = (int)(row >> logn) + 1;
+    const double v = reinterpret_cast<const double *>(s)[2 * (i * W + (r >> 1)) + (r & 1)] * scale;
+    const Images im(d, i + 1, j, k);
+    im.put(d, P, i + 1, j, k, P[ix(d, i + 1, j, k)] + v);
+    m = fmax(m, fabs(v));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < (int)(blockDim.x >> 5); ++q) m = fmax(m, top[q]);
+    atomicMax(reinterpret_cast<unsigned long long *>(sc + S_ERR), (unsigned long long)__double_as_longlong(m));
+  }
+}
+
+// interior n^3 (i fastest) -> ghosted
+__global__ void k_scatter(Dim d, double *out, const double *lin) {
   int i, j, k;
-  if (!in_box(gtid(), 0, 0, 0, d.n, d.n, d.n, i, j, k)) return;
-  out[ix(d, i + 1, j + 1, k + 1)] = (-1) * z[((size_t)k * d.n + j) * d.n + i].x / tot;
+  if (!cell_of(d, i, j, k)) return;
+  const Images im(d, i, j, k);
+  im.put(d, out, i, j, k, lin[((size_t)(k - 1) * d.n + (j - 1)) * d.n + (i - 1)]);
 }
 
 }  // namespace pgas
@@ -288,8 +496,8 @@ struct pgas_ctx {
   double *f[pgas::F_NF];
   double *sc;      // device scalars
   double *rows;    // reduction scratch (n^2)
-  double2 *z;      // FFT buffer (n^3)
-  double2 *tw[2];  // twiddles: forward, backward
+  double2 *z;      // half spectrum, n^2 (n/2 + 1)
+  double2 *tw;     // twiddles, forward
   double *kmod;
   double r, vcell;
   int logn, last_iterations;
@@ -328,74 +536,56 @@ struct Ops {
   cudaStream_t s;
   int64_t S;
   Dim d;
-  explicit Ops(pgas_ctx *g_) : g(g_), s(g_->stream), S(g_->size), d(g_->d) {}
+  dim3 grid, block;
+  explicit Ops(pgas_ctx *g_)
+      : g(g_), s(g_->stream), S(g_->size), d(g_->d), grid((d.n + 31) / 32, (d.n + 7) / 8, d.n), block(32, 8) {}
   double *F(int q) const { return g->f[q]; }
-  void refresh(double *f) const { k_refresh<<<nblk(S), kT, 0, s>>>(d, f); }
-  void div_f2c(double *out, const double *x, const double *y, const double *z) const {
-    k_div_f2c<<<nblk((int64_t)(d.n + 1) * (d.n + 1) * (d.n + 1)), kT, 0, s>>>(d, out, x, y, z);
-    refresh(out);
-  }
-  void del2(double *out, const double *t) const {
-    k_del2<<<nblk((int64_t)d.n * d.n * d.n), kT, 0, s>>>(d, out, t);
-    refresh(out);
-  }
-  void c2f(double *out, const double *t, int axis, int grad) const {
-    k_c2f<<<nblk(S), kT, 0, s>>>(d, out, t, axis, grad);
-    refresh(out);
-  }
-  void grad(double *const *o, const double *t) const {
-    for (int a = 0; a < 3; ++a) k_c2f<<<nblk(S), kT, 0, s>>>(d, o[a], t, a, 1);
-    for (int a = 0; a < 3; ++a) refresh(o[a]);
-  }
+  V3 v3(int q) const { return {{g->f[q], g->f[q + 1], g->f[q + 2]}}; }
+  CV3 c3(int q) const { return {{g->f[q], g->f[q + 1], g->f[q + 2]}}; }
   void copy(double *dst, const double *src) const {
     cudaMemcpyAsync(dst, src, sizeof(double) * S, cudaMemcpyDeviceToDevice, s);
   }
-  // interior mean (mode 0) or max |.| (mode 1) into sc[slot]
-  void reduce(const double *f, int mode, int slot) const {
+  // interior means of nf fields into sc[slot ..], then Update_P0 where q.on
+  void means(CV3 f, int nf, int slot, P0Const q = P0Const{}) const {
     const int64_t nr = (int64_t)d.n * d.n;
-    k_rows<<<nblk(nr * 32), kT, 0, s>>>(d, f, mode, g->rows);
-    k_rows_total<<<1, 256, 0, s>>>(g->rows, nr, mode, 1.0 / ((double)d.n * d.n * d.n), g->sc + slot);
-  }
-  void mean_zero(double *f) const {
-    reduce(f, 0, S_MEAN);
-    k_subs_dev<<<nblk(S), kT, 0, s>>>(f, g->sc + S_MEAN, S);
+    k_rows<<<dim3(nblk(nr * 32), (unsigned)nf), kT, 0, s>>>(d, f, g->rows);
+    k_rows_total<<<(unsigned)nf, 1024, 0, s>>>(g->rows, nr, 1.0 / ((double)d.n * d.n * d.n), g->sc, slot, q);
   }
 };
 
-void ccp_fft(const Ops &o, const double *rhs, double *out) {
-  pgas_ctx *g = o.g;
-  const int n = g->c.n;
-  const int64_t n3 = (int64_t)n * n * n;
-  k_pack<<<nblk(n3), kT, 0, o.s>>>(o.d, g->z, rhs);
-  const int th = n / 2 < 256 ? n / 2 : 256;
-  const size_t sh = sizeof(double2) * (size_t)n;
-  for (int a = 0; a < 3; ++a) k_fft_line<<<(unsigned)((int64_t)n * n), th, sh, o.s>>>(g->z, n, g->logn, a, g->tw[0]);
-  k_kmod_div<<<nblk(n3), kT, 0, o.s>>>(n, g->z, g->kmod);
-  for (int a = 0; a < 3; ++a) k_fft_line<<<(unsigned)((int64_t)n * n), th, sh, o.s>>>(g->z, n, g->logn, a, g->tw[1]);
-  k_unpack<<<nblk(n3), kT, 0, o.s>>>(o.d, out, g->z, (double)n3);
+// lines per CTA: 32 KB of them where the line is short enough, at least 4; along y the count
+// that leaves the fewest idle bins in the last tile of the half spectrum
+int lines_per_cta(int n) { return n <= 256 ? 8 : 4; }
+int lines_along_y(int n) {
+  const int nh = n / 2 + 1, most = n <= 128 ? 16 : (n == 256 ? 8 : 4);
+  int best = most;
+  for (int w = most - 1; 2 * w > most; --w)
+    if ((nh + w - 1) / w * w < (nh + best - 1) / best * best) best = w;
+  return best;
 }
 
 int solve_poisson(pgas_ctx *g) {
   Ops o(g);
-  double *C[3] = {o.F(F_DUMMY), o.F(F_DUMMY + 1), o.F(F_DUMMY + 2)};
-  for (int a = 0; a < 3; ++a) k_sdiv<<<nblk(o.S), kT, 0, o.s>>>(C[a], 1., o.F(F_RHO_FACE + a), o.S);
-  double *cc = o.F(F_CENTER), *rn = o.F(F_RHS_NEW), *P = o.F(F_P);
-  double *pd[3] = {o.F(F_PDUMMY), o.F(F_PDUMMY + 1), o.F(F_PDUMMY + 2)};
-  k_i_f2c_vec<<<nblk((int64_t)(g->c.n + 1) * (g->c.n + 1) * (g->c.n + 1)), kT, 0, o.s>>>(o.d, cc, C[0], C[1], C[2]);
-  o.refresh(cc);
-  k_sdiv<<<nblk(o.S), kT, 0, o.s>>>(cc, -1., cc, o.S);
+  const int n = g->c.n, W = lines_per_cta(n), Wy = lines_along_y(n), nh = n / 2 + 1;
+  const size_t sx = sizeof(double2) * (size_t)W * n, sy = sizeof(double2) * (size_t)Wy * n;
+  if (sx > 48 * 1024) {  // the opt-in belongs to the current device: set per solve
+    GCUDA(g, cudaFuncSetAttribute(k_res_fft_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx));
+    GCUDA(g, cudaFuncSetAttribute(k_fft_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx));
+    GCUDA(g, cudaFuncSetAttribute(k_fft_x_back, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx));
+  }
+  if (sy > 48 * 1024) GCUDA(g, cudaFuncSetAttribute(k_fft_y, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sy));
+  const unsigned bx = (unsigned)((int64_t)n * n / (2 * W)), bz = (unsigned)((int64_t)n * nh / W);
+  const dim3 by((nh + Wy - 1) / Wy, n);
+  const double scale = -0.5 / ((double)n * n * n);  // a power of two
   int it = 0;
   double error = 100;
   while (it < g->c.iterations && error > g->c.epsilon) {
-    o.grad(pd, P);
-    for (int a = 0; a < 3; ++a) k_mul<<<nblk(o.S), kT, 0, o.s>>>(pd[a], C[a], o.S);
-    o.div_f2c(rn, pd[0], pd[1], pd[2]);
-    k_sub<<<nblk(o.S), kT, 0, o.s>>>(rn, o.F(F_RHS_POIS), o.S);
-    k_mul<<<nblk(o.S), kT, 0, o.s>>>(rn, cc, o.S);
-    ccp_fft(o, rn, pd[0]);
-    k_add<<<nblk(o.S), kT, 0, o.s>>>(P, pd[0], o.S);
-    o.refresh(P);
-    o.reduce(pd[0], 1, S_ERR);
+    k_res_fft_x<<<bx, kT, sx, o.s>>>(o.d, g->logn, W, g->tw, o.F(F_P), o.c3(F_IRF), o.F(F_RHS_POIS), o.F(F_CENTER),
+                                     g->sc, g->z);
+    k_fft_y<<<by, kT, sy, o.s>>>(n, g->logn, Wy, g->tw, 0, g->z);
+    k_fft_z<<<bz, kT, sx, o.s>>>(n, g->logn, W, g->tw, g->kmod, g->z);
+    k_fft_y<<<by, kT, sy, o.s>>>(n, g->logn, Wy, g->tw, 1, g->z);
+    k_fft_x_back<<<bx, kT, sx, o.s>>>(o.d, g->logn, W, g->tw, g->z, scale, o.F(F_P), g->sc);
     GCUDA(g, cudaMemcpyAsync(&error, g->sc + S_ERR, sizeof(double), cudaMemcpyDeviceToHost, o.s));
     GCUDA(g, cudaStreamSynchronize(o.s));
     it++;
@@ -406,8 +596,8 @@ int solve_poisson(pgas_ctx *g) {
 
 int update_particle(pgas_ctx *g, pstep_handle h, int k) {
   Ops o(g);
-  for (int a = 0; a < 3; ++a) k_div<<<nblk(o.S), kT, 0, o.s>>>(o.F(F_U + a), o.F(F_RU_INT + a), o.F(F_RHO_FACE + a), o.S);
-  k_t_from_rho<<<nblk(o.S), kT, 0, o.s>>>(o.F(F_T), o.F(F_RHO_NEW), g->sc, S_P0_NEW, g->r, o.S);
+  k_velocity<<<o.grid, o.block, 0, o.s>>>(o.d, o.c3(F_RU_INT), o.c3(F_IRF), o.F(F_RHO_INT), o.F(F_RHO_NEW),
+                                          o.F(F_IRHO), g->sc, o.v3(F_U), o.F(F_T), o.F(F_DIV));
   if (!h) {
     k_fill<<<nblk(o.S), kT, 0, o.s>>>(o.F(F_C), 0.0, o.S);
     for (int a = 0; a < 3; ++a) k_fill<<<nblk(o.S), kT, 0, o.s>>>(o.F(F_RHS_RU + a), 0.0, o.S);
@@ -431,83 +621,42 @@ int stage(pgas_ctx *g, pstep_handle h, int k) {
   Ops o(g);
   const pgas_config &c = g->c;
   const double dt = c.dt;
-  const int64_t S = o.S;
-  // Update_Rho (grid.cpp:327-333)
-  o.div_f2c(o.F(F_RHS_RHO), o.F(F_RU_INT), o.F(F_RU_INT + 1), o.F(F_RU_INT + 2));
-  k_axpy<<<nblk(S), kT, 0, o.s>>>(o.F(F_RHO_NP1), -(dt * kPost[k]), o.F(F_RHS_RHO), S);
-  if (k != 3) k_lin2<<<nblk(S), kT, 0, o.s>>>(o.F(F_RHO_NEW), 1, o.F(F_RHO), -dt * kPre[k], o.F(F_RHS_RHO), S);
-  else o.copy(o.F(F_RHO_NEW), o.F(F_RHO_NP1));
-  // Update_P0 (grid.cpp:539-554)
-  o.reduce(o.F(F_RHS_PT), 0, S_MEAN_E);
-  k_update_p0<<<1, 1, 0, o.s>>>(g->sc, k == 3, dt * kPost[k], dt * kPre[k], g->r, c.cv, c.cooling);
-  // Update_Particle (grid.cpp:659-680)
+  const int last = k == 3;
+  const CV3 pt = {{o.F(F_RHS_PT), o.F(F_RHS_PT), o.F(F_RHS_PT)}};
+  // Update_Rho (grid.cpp:327-333), Update_P0 (:539-554), Update_Particle (:659-680)
+  k_update_rho<<<o.grid, o.block, 0, o.s>>>(o.d, o.c3(F_RU_INT), o.F(F_RHO), o.F(F_RHO_NP1), o.F(F_RHO_NEW),
+                                            o.F(F_IRHO), -(dt * kPost[k]), -dt * kPre[k], last);
+  o.means(pt, 1, S_MEAN_E, P0Const{1, last, c.cooling, dt * kPost[k], dt * kPre[k], g->r, c.cv, c.cp, g->vcell});
   GTRY(update_particle(g, h, k));
   // Update_RU_WOP (grid.cpp:387-425)
-  {
-    double *U[3] = {o.F(F_U), o.F(F_U + 1), o.F(F_U + 2)};
-    double *D[3] = {o.F(F_DUMMY), o.F(F_DUMMY + 1), o.F(F_DUMMY + 2)};
-    double *D2[3] = {o.F(F_DUMMY2), o.F(F_DUMMY2 + 1), o.F(F_DUMMY2 + 2)};
-    double *R[3] = {o.F(F_RHS_RU), o.F(F_RHS_RU + 1), o.F(F_RHS_RU + 2)};
-    double *RUI[3] = {o.F(F_RU_INT), o.F(F_RU_INT + 1), o.F(F_RU_INT + 2)};
-    o.div_f2c(o.F(F_DIV), U[0], U[1], U[2]);
-    o.grad(D2, o.F(F_DIV));
-    for (int a = 0; a < 3; ++a) o.del2(D[a], U[a]);
-    for (int a = 0; a < 3; ++a)
-      k_lin3<<<nblk(S), kT, 0, o.s>>>(R[a], -c.mp / g->vcell, R[a], c.mu0 / 3., D2[a], c.mu0, D[a], S);
-    for (int e = 0; e < 3; ++e) {
-      for (int a = 0; a < 3; ++a) o.c2f(D[a], U[e], a, 0);
-      for (int a = 0; a < 3; ++a) o.c2f(D2[a], RUI[a], e, 0);
-      for (int a = 0; a < 3; ++a) k_mul<<<nblk(S), kT, 0, o.s>>>(D[a], D2[a], S);
-      o.div_f2c(D2[e], D[0], D[1], D[2]);
-      k_sub<<<nblk(S), kT, 0, o.s>>>(R[e], D2[e], S);
-    }
-    for (int a = 0; a < 3; ++a) k_axpy<<<nblk(S), kT, 0, o.s>>>(R[a], c.a_force, RUI[a], S);
-    k_adds<<<nblk(S), kT, 0, o.s>>>(R[0], -(c.a_force * c.rho0 * c.u0), S);
-    const double gv[3] = {c.gx, c.gy, c.gz};
-    for (int a = 0; a < 3; ++a) {
-      k_adds<<<nblk(S), kT, 0, o.s>>>(o.F(F_RHO_FACE + a), -c.rho0, S);
-      k_mul_to<<<nblk(S), kT, 0, o.s>>>(D[a], o.F(F_RHO_FACE + a), gv[a], S);
-      k_add<<<nblk(S), kT, 0, o.s>>>(R[a], D[a], S);
-    }
-    for (int a = 0; a < 3; ++a) k_axpy<<<nblk(S), kT, 0, o.s>>>(o.F(F_RU_NP1 + a), dt * kPost[k], R[a], S);
-    if (k != 3) {
-      for (int a = 0; a < 3; ++a)
-        k_lin2<<<nblk(S), kT, 0, o.s>>>(o.F(F_RU_NEW + a), 1, o.F(F_RU + a), dt * kPre[k], R[a], S);
-    } else {
-      for (int a = 0; a < 3; ++a) o.copy(o.F(F_RU_NEW + a), o.F(F_RU_NP1 + a));
-    }
-  }
-  // Compute_Div_U_new (grid.cpp:556-563)
-  k_sdiv<<<nblk(S), kT, 0, o.s>>>(o.F(F_DUMMY), 1., o.F(F_RHO_NEW), S);
-  o.del2(o.F(F_DUMMY + 1), o.F(F_DUMMY));
-  o.copy(o.F(F_DUMMY + 2), o.F(F_RHS_PT));
-  if (c.cooling) o.mean_zero(o.F(F_DUMMY + 2));
-  k_div_u<<<nblk(S), kT, 0, o.s>>>(o.F(F_DIV), o.F(F_DUMMY + 1), o.F(F_DUMMY + 2), g->sc, c.k / c.cp, g->r, c.cp,
-                                   g->vcell, S);
-  // Compute_RHS_Pois (grid.cpp:629-637)
-  for (int a = 0; a < 3; ++a) o.c2f(o.F(F_RHO_FACE + a), o.F(F_RHO_NEW), a, 0);
-  for (int a = 0; a < 3; ++a) k_div<<<nblk(S), kT, 0, o.s>>>(o.F(F_U + a), o.F(F_RU_NEW + a), o.F(F_RHO_FACE + a), S);
-  o.div_f2c(o.F(F_RHS_POIS), o.F(F_U), o.F(F_U + 1), o.F(F_U + 2));
-  k_sub<<<nblk(S), kT, 0, o.s>>>(o.F(F_RHS_POIS), o.F(F_DIV), S);
-  k_muls<<<nblk(S), kT, 0, o.s>>>(o.F(F_RHS_POIS), 1. / (dt * kPre[k]), S);
-  o.mean_zero(o.F(F_RHS_POIS));
+  RuConst q;
+  q.part = -c.mp / g->vcell;
+  q.mu3 = c.mu0 / 3.;
+  q.mu = c.mu0;
+  q.a_force = c.a_force;
+  q.a_const = -(c.a_force * c.rho0 * c.u0);
+  q.rho0 = c.rho0;
+  q.g[0] = c.gx; q.g[1] = c.gy; q.g[2] = c.gz;
+  q.post = dt * kPost[k];
+  q.pre = dt * kPre[k];
+  q.force = c.a_force != 0.0;
+  q.gravity = c.gx != 0.0 || c.gy != 0.0 || c.gz != 0.0;
+  q.last = last;
+  k_update_ru<<<o.grid, o.block, 0, o.s>>>(o.d, q, o.c3(F_U), o.c3(F_RU_INT), o.c3(F_RU), o.F(F_DIV), o.F(F_RHO_INT),
+                                           o.F(F_RHO_NEW), o.v3(F_RHS_RU), o.v3(F_RU_NP1), o.v3(F_RU_NEW),
+                                           o.v3(F_IRF));
+  // Compute_Div_U_new (grid.cpp:556-563), Compute_RHS_Pois (:629-637)
+  if (c.cooling) o.means(pt, 1, S_MEAN);
+  k_rhs_pois<<<o.grid, o.block, 0, o.s>>>(o.d, o.c3(F_RU_NEW), o.c3(F_IRF), o.F(F_RHO_NEW), o.F(F_IRHO),
+                                          o.F(F_RHS_PT), g->sc, c.k / c.cp, 1. / (dt * kPre[k]), c.cooling, o.v3(F_U),
+                                          o.F(F_DIV), o.F(F_RHS_POIS), o.F(F_CENTER));
+  o.means(CV3{{o.F(F_RHS_POIS), nullptr, nullptr}}, 1, S_MEAN);
   GCUDA(g, cudaGetLastError());
   // Solve_Poisson (grid.cpp:639-643)
   GTRY(solve_poisson(g));
-  // Update_RU_WP (grid.cpp:651-657)
-  {
-    double *D[3] = {o.F(F_DUMMY), o.F(F_DUMMY + 1), o.F(F_DUMMY + 2)};
-    o.grad(D, o.F(F_P));
-    for (int a = 0; a < 3; ++a) k_axpy<<<nblk(S), kT, 0, o.s>>>(o.F(F_RU_NP1 + a), -(dt * kPost[k]), D[a], S);
-    if (k != 3) {
-      for (int a = 0; a < 3; ++a) k_axpy<<<nblk(S), kT, 0, o.s>>>(o.F(F_RU_NEW + a), -(dt * kPre[k]), D[a], S);
-    } else {
-      for (int a = 0; a < 3; ++a) o.copy(o.F(F_RU_NEW + a), o.F(F_RU_NP1 + a));
-    }
-  }
-  // TimeAdvance_RK4 (grid.cpp:705-712)
-  o.copy(o.F(F_RHO_INT), o.F(F_RHO_NEW));
-  for (int a = 0; a < 3; ++a) o.copy(o.F(F_RU_INT + a), o.F(F_RU_NEW + a));
+  // Update_RU_WP (grid.cpp:651-657), TimeAdvance_RK4 (grid.cpp:705-712)
+  k_pressure_step<<<o.grid, o.block, 0, o.s>>>(o.d, o.F(F_P), o.c3(F_RU_NEW), o.v3(F_RU_NP1), o.v3(F_RU_INT),
+                                               o.F(F_RHO_NEW), o.F(F_RHO_INT), -(dt * kPost[k]), -(dt * kPre[k]), last);
   k_scalar_copy<<<1, 1, 0, o.s>>>(g->sc, S_P0_INT, S_P0_NEW);
   if (h) GTRY(pstep_end_stage(h));
   GCUDA(g, cudaGetLastError());
@@ -552,23 +701,21 @@ int pgas_create(const pgas_config *cfg, pgas_handle *out) {
     ok = alloc((void **)&g->f[q], sizeof(double) * g->size);
     if (ok) cudaMemset(g->f[q], 0, sizeof(double) * g->size);
   }
-  ok = ok && alloc((void **)&g->sc, sizeof(double) * S_N) && alloc((void **)&g->rows, sizeof(double) * n * n) &&
-       alloc((void **)&g->z, sizeof(double2) * (size_t)n * n * n) && alloc((void **)&g->tw[0], sizeof(double2) * n) &&
-       alloc((void **)&g->tw[1], sizeof(double2) * n) && alloc((void **)&g->kmod, sizeof(double) * n);
+  ok = ok && alloc((void **)&g->sc, sizeof(double) * S_N) && alloc((void **)&g->rows, sizeof(double) * 3 * n * n) &&
+       alloc((void **)&g->z, sizeof(double2) * (size_t)n * n * (n / 2 + 1)) &&
+       alloc((void **)&g->tw, sizeof(double2) * n) && alloc((void **)&g->kmod, sizeof(double) * n);
   if (!ok) {
     pgas_destroy(g);
     return PSTEP_ERR_NOMEM;
   }
-  // twiddles (cos, -/+ sin of 2 pi m / n) and modified wavenumbers (poisson.cpp:428-448)
+  // twiddles (cos, -sin of 2 pi m / n) and modified wavenumbers (poisson.cpp:428-448)
   const double two_pi = 2 * 3.141592653589793;
   double2 *tw = (double2 *)malloc(sizeof(double2) * n);
-  for (int sgn = 0; sgn < 2; ++sgn) {
-    for (int m = 0; m < n / 2; ++m) {
-      const double a = two_pi * (double)m / (double)n;
-      tw[m] = make_double2(cos(a), (sgn == 0 ? -1 : 1) * sin(a));
-    }
-    cudaMemcpy(g->tw[sgn], tw, sizeof(double2) * n, cudaMemcpyHostToDevice);
+  for (int m = 0; m < n / 2; ++m) {
+    const double a = two_pi * (double)m / (double)n;
+    tw[m] = make_double2(cos(a), -sin(a));
   }
+  cudaMemcpy(g->tw, tw, sizeof(double2) * (n / 2), cudaMemcpyHostToDevice);
   free(tw);
   double *km = (double *)malloc(sizeof(double) * n);
   {
@@ -595,7 +742,7 @@ int pgas_destroy(pgas_handle g) {
   else cudaDeviceSynchronize();
   for (int q = 0; q < F_NF; ++q)
     if (g->f[q]) cudaFree(g->f[q]);
-  void *ps[6] = {g->sc, g->rows, g->z, g->tw[0], g->tw[1], g->kmod};
+  void *ps[5] = {g->sc, g->rows, g->z, g->tw, g->kmod};
   for (void *p : ps)
     if (p) cudaFree(p);
   delete g;
@@ -620,13 +767,13 @@ int pgas_init(pgas_handle g, pstep_handle h, const double *ru_x, const double *r
   for (int q = 0; q < 4; ++q) {
     GCUDA(g, cudaMemcpyAsync(g->z, src[q], sizeof(double) * n3,
                              on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, o.s));
-    k_scatter<<<nblk(n3), kT, 0, o.s>>>(o.d, o.F(dst[q]), (const double *)g->z);
-    o.refresh(o.F(dst[q]));
+    k_scatter<<<o.grid, o.block, 0, o.s>>>(o.d, o.F(dst[q]), (const double *)g->z);
     GCUDA(g, cudaStreamSynchronize(o.s));  // the buffer is reused for the next field
   }
   k_fill<<<nblk(o.S), kT, 0, o.s>>>(o.F(F_P), 0.0, o.S);
   double sc[S_N] = {0};
   sc[S_P0] = sc[S_P0_INT] = sc[S_P0_NP1] = sc[S_P0_NEW] = p0;
+  sc[S_T] = p0 / g->r;
   GCUDA(g, cudaMemcpyAsync(g->sc, sc, sizeof sc, cudaMemcpyHostToDevice, o.s));
   for (int a = 0; a < 3; ++a) {
     o.copy(o.F(F_RU_INT + a), o.F(F_RU + a));
@@ -634,9 +781,7 @@ int pgas_init(pgas_handle g, pstep_handle h, const double *ru_x, const double *r
   }
   o.copy(o.F(F_RHO_INT), o.F(F_RHO));
   o.copy(o.F(F_RHO_NP1), o.F(F_RHO));
-  for (int a = 0; a < 3; ++a) o.c2f(o.F(F_RHO_FACE + a), o.F(F_RHO), a, 0);
-  k_t_from_rho<<<nblk(o.S), kT, 0, o.s>>>(o.F(F_T), o.F(F_RHO_INT), g->sc, S_P0_INT, g->r, o.S);
-  for (int a = 0; a < 3; ++a) k_div<<<nblk(o.S), kT, 0, o.s>>>(o.F(F_U + a), o.F(F_RU + a), o.F(F_RHO_FACE + a), o.S);
+  k_init_fields<<<o.grid, o.block, 0, o.s>>>(o.d, o.c3(F_RU), o.F(F_RHO_INT), g->sc, o.v3(F_IRF), o.v3(F_U), o.F(F_T));
   if (h) {
     GTRY(pstep_set_stream(h, g->stream));
     GTRY(pstep_bind_velocity(h, o.F(F_U), o.F(F_U + 1), o.F(F_U + 2), 1));
@@ -660,12 +805,10 @@ int pgas_stage(pgas_handle g, pstep_handle h, int k) {
 int pgas_end_step(pgas_handle g, pstep_handle h) {
   if (!g) return PSTEP_ERR_ARG;
   Ops o(g);
-  // Correct_mean_RU (grid.cpp:566-572, box)
-  for (int a = 0; a < 3; ++a) o.mean_zero(o.F(F_RU_NP1 + a));
-  k_adds<<<nblk(o.S), kT, 0, o.s>>>(o.F(F_RU_NP1), g->c.rho0 * g->c.u0, o.S);
-  // TimeAdvance (grid.cpp:315-325)
-  o.copy(o.F(F_RHO), o.F(F_RHO_NP1));
-  for (int a = 0; a < 3; ++a) o.copy(o.F(F_RU + a), o.F(F_RU_NP1 + a));
+  // Correct_mean_RU (grid.cpp:566-572, box) and TimeAdvance (grid.cpp:315-325)
+  o.means(o.c3(F_RU_NP1), 3, S_MEAN);
+  k_end_step<<<o.grid, o.block, 0, o.s>>>(o.d, o.v3(F_RU_NP1), o.v3(F_RU), o.F(F_RHO_NP1), o.F(F_RHO), g->sc,
+                                          g->c.rho0 * g->c.u0);
   k_scalar_copy<<<1, 1, 0, o.s>>>(g->sc, S_P0, S_P0_NP1);
   if (h) GTRY(pstep_end_step(h));
   GCUDA(g, cudaGetLastError());
