@@ -52,10 +52,8 @@ typedef enum {
   PSTEP_ERR_RANGE = 7,      /* a particle position outside [0, L] (or at L, where the
                                reference indexes past its ghost layer) */
   PSTEP_ERR_MOVE = 8,       /* FP32 form: a particle's stage position more than one cell from
-                               its step-start cell along some axis (the deposit gathers each
-                               brick's sources from two cells around it, which holds only for
-                               moves of at most one cell per stage); the stage's deposits are
-                               then incomplete */
+                               its step-start cell along some axis (the step is meant for moves
+                               of at most one cell per stage) */
   PSTEP_ERR_NOMEM = 9,      /* device allocation failed */
   PSTEP_ERR_TIMEOUT = 10,   /* a bounded device-side wait gave up */
   PSTEP_ERR_IO = 11         /* a snapshot file could not be created, read or written */
