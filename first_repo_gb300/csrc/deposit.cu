@@ -561,49 +561,44 @@ __global__ void k_fold_x(Geom G, FieldSet fs) {
   f[glin(G, 1, j, k)] += top;
 }
 
-// communicator.cpp:177-278 on one rank: x (interior j,k), y (all i, interior k), z (all i,j)
-__global__ void k_refresh_x(Geom G, FieldSet fs) {
+// communicator.cpp:177-278 on one rank: its x, y and z passes leave in every ghost cell the value of
+// its periodic image; one launch over the ghost layers, reading interior cells only
+__global__ void k_refresh(Geom G, FieldSet fs) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long per = (long long)G.n[1] * G.n[2];
+  const long long nz = 2ll * G.g[0] * G.g[1], ny = 2ll * G.g[0] * G.n[2], nx = 2ll * G.n[1] * G.n[2];
+  const long long per = nz + ny + nx;
   if (t >= per * fs.nf) return;
-  int q = (int)(t / per);
-  long long r = t % per;
-  int j = (int)(r % G.n[1]) + 1, k = (int)(r / G.n[1]) + 1;
-  double *f = fs.f[q];
-  const int I = G.g[0];
-  f[glin(G, I - 1, j, k)] = f[glin(G, 1, j, k)];
-  f[glin(G, 0, j, k)] = f[glin(G, I - 2, j, k)];
-}
-
-__global__ void k_refresh_y(Geom G, FieldSet fs) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long per = (long long)G.g[0] * G.n[2];
-  if (t >= per * fs.nf) return;
-  int q = (int)(t / per);
-  long long r = t % per;
-  int i = (int)(r % G.g[0]), k = (int)(r / G.g[0]) + 1;
-  double *f = fs.f[q];
-  const int J = G.g[1];
-  f[glin(G, i, J - 1, k)] = f[glin(G, i, 1, k)];
-  f[glin(G, i, 0, k)] = f[glin(G, i, J - 2, k)];
-}
-
-__global__ void k_refresh_z(Geom G, FieldSet fs) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long plane = (long long)G.g[0] * G.g[1];
-  if (t >= plane * fs.nf) return;
-  int q = (int)(t / plane);
-  long long ij = t % plane;
-  double *f = fs.f[q];
-  const int K = G.g[2];
-  f[(long long)(K - 1) * plane + ij] = f[plane + ij];
-  f[ij] = f[(long long)(K - 2) * plane + ij];
+  double *f = fs.f[t / per];
+  t %= per;
+  int i, j, k;
+  if (t < nz) {
+    const unsigned u = (unsigned)t;
+    i = (int)(u % (unsigned)G.g[0]);
+    j = (int)((u / (unsigned)G.g[0]) % (unsigned)G.g[1]);
+    k = t < nz / 2 ? 0 : G.g[2] - 1;
+  } else if (t < nz + ny) {
+    const unsigned u = (unsigned)(t - nz), r = u / (unsigned)G.g[0];
+    i = (int)(u % (unsigned)G.g[0]);
+    k = (int)(r % (unsigned)G.n[2]) + 1;
+    j = (int)(r / (unsigned)G.n[2]) ? G.g[1] - 1 : 0;
+  } else {
+    const unsigned u = (unsigned)(t - nz - ny), r = u / (unsigned)G.n[1];
+    j = (int)(u % (unsigned)G.n[1]) + 1;
+    k = (int)(r % (unsigned)G.n[2]) + 1;
+    i = (int)(r / (unsigned)G.n[2]) ? G.g[0] - 1 : 0;
+  }
+  const int si = i == 0 ? G.n[0] : (i == G.g[0] - 1 ? 1 : i), sj = j == 0 ? G.n[1] : (j == G.g[1] - 1 ? 1 : j),
+            sk = k == 0 ? G.n[2] : (k == G.g[2] - 1 ? 1 : k);
+  f[glin(G, i, j, k)] = f[glin(G, si, sj, sk)];
 }
 
 // Interior sum, fixed order: per-block tree over a strided range, then one block.
 constexpr int kRedBlocks = 1024;
-__global__ void k_sum_partial(Geom G, const double *__restrict__ f, double *__restrict__ part) {
+// (blockIdx.y: the field, and its kRedBlocks partials)
+__global__ void k_sum_partial(Geom G, FieldSet fs, double *__restrict__ part) {
   __shared__ double sm[kThreads];
+  const double *__restrict__ f = fs.f[blockIdx.y];
+  part += (size_t)blockIdx.y * kRedBlocks;
   // rows (j,k) distributed over blocks, the i loop over threads: fixed order, coalesced
   const long long rows = (long long)G.n[1] * G.n[2];
   double s = 0.0;
@@ -623,6 +618,7 @@ __global__ void k_sum_partial(Geom G, const double *__restrict__ f, double *__re
 
 __global__ void k_sum_final(const double *__restrict__ part, int np, double inv_count, double *__restrict__ out) {
   __shared__ double sm[kThreads];
+  part += (size_t)blockIdx.x * kRedBlocks;
   double s = 0.0;
   for (int i = threadIdx.x; i < np; i += kThreads) s += part[i];
   sm[threadIdx.x] = s;
@@ -631,7 +627,7 @@ __global__ void k_sum_final(const double *__restrict__ part, int np, double inv_
     if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *out = sm[0] * inv_count;
+  if (threadIdx.x == 0) out[blockIdx.x] = sm[0] * inv_count;
 }
 
 inline int blocks_for(long long n) { return (int)((n + kThreads - 1) / kThreads); }
@@ -652,22 +648,13 @@ DepIn make_in(pstep_ctx *h, const Csr &csr, double *const frac[3], const uint32_
 
 }  // namespace
 
-// refresh: 0 fold only, 1 fold then refresh, 2 refresh only (interior already periodic)
+// the cumulative fold of nf fields, then the ghost refresh of the last `refresh` of them
 int fold_fields(pstep_ctx *h, double *const *f, int nf, int refresh) {
   const Geom &G = h->geom;
   FieldSet fs;
   fs.nf = nf;
   for (int q = 0; q < nf; ++q) fs.f[q] = f[q];
   long long plane = (long long)G.g[0] * G.g[1];
-  if (refresh == 2) {
-    k_refresh_x<<<blocks_for((long long)G.n[1] * G.n[2] * nf), kThreads, 0, h->stream>>>(G, fs);
-    PSTEP_LAUNCHED(h);
-    k_refresh_y<<<blocks_for((long long)G.g[0] * G.n[2] * nf), kThreads, 0, h->stream>>>(G, fs);
-    PSTEP_LAUNCHED(h);
-    k_refresh_z<<<blocks_for(plane * nf), kThreads, 0, h->stream>>>(G, fs);
-    PSTEP_LAUNCHED(h);
-    return PSTEP_OK;
-  }
   k_fold_z<<<blocks_for(plane * nf), kThreads, 0, h->stream>>>(G, fs);
   PSTEP_LAUNCHED(h);
   k_fold_y<<<blocks_for((long long)G.g[0] * G.n[2] * nf), kThreads, 0, h->stream>>>(G, fs);
@@ -675,11 +662,10 @@ int fold_fields(pstep_ctx *h, double *const *f, int nf, int refresh) {
   k_fold_x<<<blocks_for((long long)G.n[1] * G.n[2] * nf), kThreads, 0, h->stream>>>(G, fs);
   PSTEP_LAUNCHED(h);
   if (refresh) {
-    k_refresh_x<<<blocks_for((long long)G.n[1] * G.n[2] * nf), kThreads, 0, h->stream>>>(G, fs);
-    PSTEP_LAUNCHED(h);
-    k_refresh_y<<<blocks_for((long long)G.g[0] * G.n[2] * nf), kThreads, 0, h->stream>>>(G, fs);
-    PSTEP_LAUNCHED(h);
-    k_refresh_z<<<blocks_for(plane * nf), kThreads, 0, h->stream>>>(G, fs);
+    fs.nf = refresh;
+    for (int q = 0; q < refresh; ++q) fs.f[q] = f[nf - refresh + q];
+    const long long ghosts = 2 * plane + 2ll * G.g[0] * G.n[2] + 2ll * G.n[1] * G.n[2];
+    k_refresh<<<blocks_for(ghosts * refresh), kThreads, 0, h->stream>>>(G, fs);
     PSTEP_LAUNCHED(h);
   }
   return PSTEP_OK;
@@ -687,7 +673,10 @@ int fold_fields(pstep_ctx *h, double *const *f, int nf, int refresh) {
 
 int interior_mean(pstep_ctx *h, const double *f, double *out_dev) {
   const Geom &G = h->geom;
-  k_sum_partial<<<kRedBlocks, kThreads, 0, h->stream>>>(G, f, h->red_partials);
+  FieldSet fs;
+  fs.nf = 1;
+  fs.f[0] = const_cast<double *>(f);
+  k_sum_partial<<<kRedBlocks, kThreads, 0, h->stream>>>(G, fs, h->red_partials);
   PSTEP_LAUNCHED(h);
   double inv = 1.0 / (double)((long long)G.n[0] * G.n[1] * G.n[2]);
   k_sum_final<<<1, kThreads, 0, h->stream>>>(h->red_partials, kRedBlocks, inv, out_dev);
@@ -703,13 +692,14 @@ int momentum_sums(pstep_ctx *h) {
     PSTEP_CUDA(cudaMemsetAsync(h->mom_dev, 0, 3 * sizeof(double), h->stream));
     return PSTEP_OK;
   }
-  for (int d = 0; d < 3; ++d) {
-    double *part = h->red_partials + (1 + d) * kRedBlocks;
-    k_sum_partial<<<kRedBlocks, kThreads, 0, h->stream>>>(G, h->dep[PSTEP_FIELD_RU_X + d], part);
-    PSTEP_LAUNCHED(h);
-    k_sum_final<<<1, kThreads, 0, h->stream>>>(part, kRedBlocks, 1.0, h->mom_dev + d);
-    PSTEP_LAUNCHED(h);
-  }
+  FieldSet fs;
+  fs.nf = 3;
+  for (int d = 0; d < 3; ++d) fs.f[d] = h->dep[PSTEP_FIELD_RU_X + d];
+  double *part = h->red_partials + kRedBlocks;
+  k_sum_partial<<<dim3(kRedBlocks, 3), kThreads, 0, h->stream>>>(G, fs, part);
+  PSTEP_LAUNCHED(h);
+  k_sum_final<<<3, kThreads, 0, h->stream>>>(part, kRedBlocks, 1.0, h->mom_dev);
+  PSTEP_LAUNCHED(h);
   return PSTEP_OK;
 }
 
@@ -756,14 +746,12 @@ int f64_deposit_int(pstep_ctx *h) {
     int rc = brick_launch(h, d, 0, h->dep[PSTEP_FIELD_C], h->dep[PSTEP_FIELD_RU_X], h->dep[PSTEP_FIELD_RU_Y],
                           h->dep[PSTEP_FIELD_RU_Z]);
     if (rc) return rc;
-    double *c1[1] = {h->dep[PSTEP_FIELD_C]};
-    rc = fold_fields(h, c1, 1, 0);  // the reference does not refresh C's ghosts
+    // (the reference does not refresh C's ghosts)
+    double *all[4] = {h->dep[PSTEP_FIELD_C], h->dep[PSTEP_FIELD_RU_X], h->dep[PSTEP_FIELD_RU_Y],
+                      h->dep[PSTEP_FIELD_RU_Z]};
+    rc = fold_fields(h, all, h->cfg.twc ? 4 : 1, h->cfg.twc ? 3 : 0);
     if (rc) return rc;
-    if (h->cfg.twc) {
-      double *ru[3] = {h->dep[PSTEP_FIELD_RU_X], h->dep[PSTEP_FIELD_RU_Y], h->dep[PSTEP_FIELD_RU_Z]};
-      rc = fold_fields(h, ru, 3, 1);
-      if (rc) return rc;
-    } else {
+    if (!h->cfg.twc) {
       for (int q = PSTEP_FIELD_RU_X; q <= PSTEP_FIELD_RU_Z; ++q)
         PSTEP_CUDA(cudaMemsetAsync(h->dep[q], 0, sizeof(double) * G.gsize, h->stream));
     }
@@ -782,7 +770,7 @@ int f64_deposit_int(pstep_ctx *h) {
     k_dep_face<2><<<blocks_for(G.gsize), kThreads, 0, h->stream>>>(G, d, h->dep[PSTEP_FIELD_RU_Z]);
     PSTEP_LAUNCHED(h);
     double *ru[3] = {h->dep[PSTEP_FIELD_RU_X], h->dep[PSTEP_FIELD_RU_Y], h->dep[PSTEP_FIELD_RU_Z]};
-    rc = fold_fields(h, ru, 3, 1);
+    rc = fold_fields(h, ru, 3, 3);
     if (rc) return rc;
   } else {
     for (int q = PSTEP_FIELD_RU_X; q <= PSTEP_FIELD_RU_Z; ++q)

@@ -133,7 +133,7 @@ void release(pstep_ctx *h) {
   for (int d = 0; d < 3; ++d) { dfree(h->s.frac_prev[d]); dfree(h->s.frac_new[d]); dfree(h->s.rhs_u[d]); }
   dfree(h->s.key_prev); dfree(h->s.key_new);
   dfree(h->csr_prev.cell_start); dfree(h->csr_prev.sidx); dfree(h->csr_new.cell_start); dfree(h->csr_new.sidx);
-  dfree(h->counts); dfree(h->cursor); dfree(h->scan_blocks); dfree(h->big_list); dfree(h->big_count);
+  dfree(h->counts); dfree(h->cursor); dfree(h->scan_status); dfree(h->scan_ticket); dfree(h->big_list); dfree(h->big_count);
   void *pt = h->perm_tmp; if (pt) cudaFree(pt); h->perm_tmp = nullptr;
   for (int d = 0; d < 3; ++d) dfree(h->own_u[d]);
   dfree(h->own_t);
@@ -191,7 +191,10 @@ int alloc_all(pstep_ctx *h) {
   int64_t scan_n = (int64_t)gs + 1;
   if ((int64_t)cap > scan_n) scan_n = (int64_t)cap;
   h->scan_nblocks = scan_blocks_needed(scan_n) + 1;
-  TRY(dalloc(h, h->scan_blocks, (size_t)h->scan_nblocks));
+  TRY(dalloc(h, h->scan_status, (size_t)h->scan_nblocks));
+  TRY(dalloc(h, h->scan_ticket, 1));
+  PSTEP_CUDA(cudaMemsetAsync(h->scan_status, 0, sizeof(unsigned long long) * h->scan_nblocks, h->stream));
+  PSTEP_CUDA(cudaMemsetAsync(h->scan_ticket, 0, sizeof(int32_t), h->stream));
   for (int f = 0; f < PSTEP_NUM_FIELDS; ++f) {
     TRY(dalloc(h, h->dep[f], gs));
     PSTEP_CUDA(cudaMemsetAsync(h->dep[f], 0, sizeof(double) * gs, h->stream));

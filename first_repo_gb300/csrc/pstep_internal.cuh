@@ -94,7 +94,9 @@ struct pstep_ctx {
   // counting sort scratch
   int32_t *counts;      // gsize
   int32_t *cursor;      // gsize
-  int32_t *scan_blocks; // block sums
+  unsigned long long *scan_status;  // one word per tile of a scan, and the scans' ticket and epoch
+  int32_t *scan_ticket;
+  uint32_t scan_epoch;
   int32_t *big_list;    // nodes with long segments (gsize)
   int32_t *big_count;   // device counter
   int64_t scan_nblocks;

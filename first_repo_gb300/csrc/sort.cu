@@ -52,41 +52,29 @@ __device__ inline int32_t block_excl_scan(int32_t v, int32_t *smem, int32_t &tot
   return warp_off + x - v;
 }
 
-// phase 1: per-tile sums
-__global__ void k_scan_reduce(const int32_t *__restrict__ in, int64_t n, int32_t *__restrict__ block_sums) {
-  __shared__ int32_t sm[kThreads / 32];
-  int64_t base = (int64_t)blockIdx.x * kScanTile;
-  int32_t s = 0;
-#pragma unroll
-  for (int q = 0; q < kScanItems; ++q) {
-    int64_t i = base + (int64_t)q * kThreads + threadIdx.x;
-    if (i < n) s += in[i];
-  }
-  int32_t total;
-  block_excl_scan(s, sm, total);
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-// phase 2: exclusive scan of the tile sums (one block, sequential over chunks)
-__global__ void k_scan_blocks(int32_t *__restrict__ sums, int64_t nb) {
-  __shared__ int32_t sm[kThreads / 32];
-  int32_t carry = 0;
-  for (int64_t base = 0; base < nb; base += kThreads) {
-    int64_t i = base + threadIdx.x;
-    int32_t v = i < nb ? sums[i] : 0;
-    int32_t total;
-    int32_t e = block_excl_scan(v, sm, total);
-    if (i < nb) sums[i] = carry + e;
-    carry += total;
-  }
-}
-
-// phase 3: per-tile exclusive scan in blocked order; writes out[0..n] (out[n] = total)
-__global__ void k_scan_apply(const int32_t *__restrict__ in, int64_t n, const int32_t *__restrict__ block_off,
-                             int32_t *__restrict__ out, int32_t *__restrict__ out2) {
+// Exclusive scan in one pass (decoupled look-back): every block takes the next tile by a ticket,
+// publishes its tile's sum, then adds up its predecessors' published values from the nearest one
+// back until it meets an inclusive prefix. Tickets are handed out in order, so a tile's
+// predecessors are running or done; the wait is bounded all the same. A tile's word is
+// (epoch, state, value): words of an earlier scan are told by their epoch, so nothing is cleared.
+// Writes out[0..n] (out[n] = total) and out2 (optional). The three-launch form (tile sums, their
+// scan by one block, apply) took 9.3 us at 64^3 keys and 26 us at 256^3, this 4.5 and 25 us.
+constexpr uint32_t kScanSum = 1, kScanPrefix = 2;
+constexpr uint32_t kScanWait = 1u << 24;  // polls of one predecessor
+__global__ void __launch_bounds__(kThreads) k_scan(const int32_t *__restrict__ in, int64_t n, unsigned long long *status,
+                                                   int32_t *ticket, uint32_t epoch, int32_t *__restrict__ out,
+                                                   int32_t *__restrict__ out2, int32_t *__restrict__ err) {
   static_assert(kScanItems % 4 == 0, "whole 16-byte vectors per thread");
   __shared__ int32_t sm[kThreads / 32];
-  int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
+  __shared__ int32_t s_tile, s_before;
+  if (threadIdx.x == 0) {
+    const int32_t t = atomicAdd(ticket, 1);
+    if (t == (int32_t)gridDim.x - 1) *ticket = 0;  // the last ticket of this scan
+    s_tile = t;
+  }
+  __syncthreads();
+  const int32_t tile = s_tile;
+  int64_t base = (int64_t)tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
   // whole tiles move as 16-byte vectors (the arrays are 16-byte aligned and base is a
   // multiple of 4 elements); the ragged last tile element by element
   const bool whole = base + kScanItems <= n && (((uintptr_t)in | (uintptr_t)out | (uintptr_t)out2) & 15) == 0;
@@ -105,7 +93,46 @@ __global__ void k_scan_apply(const int32_t *__restrict__ in, int64_t n, const in
 #pragma unroll
   for (int q = 0; q < kScanItems; ++q) s += v[q];
   int32_t total;
-  int32_t e = block_excl_scan(s, sm, total) + block_off[blockIdx.x];
+  int32_t e = block_excl_scan(s, sm, total);
+  if (threadIdx.x < 32) {
+    const int lane = (int)threadIdx.x;
+    volatile unsigned long long *st = status;
+    auto word = [&](uint32_t state, int32_t value) {
+      return ((unsigned long long)(epoch * 4 + state) << 32) | (uint32_t)value;
+    };
+    int32_t before = 0;
+    if (tile == 0) {
+      if (lane == 0) st[0] = word(kScanPrefix, total);
+    } else {
+      if (lane == 0) st[tile] = word(kScanSum, total);
+      for (int32_t at = tile - 1; at >= 0; at -= 32) {  // 32 predecessors at a time, the nearest in lane 0
+        const int32_t q = at - lane;
+        uint32_t state = kScanPrefix;
+        int32_t value = 0;
+        if (q >= 0) {
+          unsigned long long w = st[q];
+          uint32_t polls = 0;
+          while ((uint32_t)(w >> 34) != (epoch & 0x3fffffffu) || ((uint32_t)(w >> 32) & 3u) == 0) {
+            if (++polls == kScanWait) {
+              atomicOr(err, kErrTimeout);
+              break;
+            }
+            w = st[q];
+          }
+          state = (uint32_t)(w >> 32) & 3u;
+          value = (int32_t)(uint32_t)w;
+        }
+        const unsigned prefix = __ballot_sync(0xffffffffu, state == kScanPrefix);
+        const int stop = prefix ? __ffs(prefix) - 1 : 31;
+        before += (int32_t)__reduce_add_sync(0xffffffffu, (unsigned)(lane <= stop ? value : 0));
+        if (prefix) break;
+      }
+      if (lane == 0) st[tile] = word(kScanPrefix, before + total);
+    }
+    if (lane == 0) s_before = before;
+  }
+  __syncthreads();
+  e += s_before;
   if (whole) {
 #pragma unroll
     for (int q = 0; q < kScanItems; q += 4) {
@@ -161,8 +188,9 @@ __device__ __forceinline__ unsigned long long seg_item(const int32_t *__restrict
 // k_scatter with the particles' items instead of their indices
 __global__ void k_scatter_items(const uint32_t *__restrict__ keys, int shift, int64_t n,
                                 const int32_t *__restrict__ order, int32_t *__restrict__ cursor,
-                                unsigned long long *__restrict__ items) {
+                                unsigned long long *__restrict__ items, int32_t *__restrict__ big_count) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *big_count = 0;  // k_segrank's list
   bool valid = i < n;
   uint32_t node = valid ? (keys[i] >> shift) : 0xffffffffu;
   unsigned active = __ballot_sync(0xffffffffu, valid);
@@ -274,11 +302,10 @@ int exclusive_scan(pstep_ctx *h, const int32_t *in, int64_t n, int32_t *out, int
     snprintf(h->err, sizeof h->err, "scan scratch too small");
     return PSTEP_ERR_STATE;
   }
-  k_scan_reduce<<<(int)nb, kThreads, 0, h->stream>>>(in, n, h->scan_blocks);
-  PSTEP_LAUNCHED(h);
-  k_scan_blocks<<<1, kThreads, 0, h->stream>>>(h->scan_blocks, nb);
-  PSTEP_LAUNCHED(h);
-  k_scan_apply<<<(int)nb, kThreads, 0, h->stream>>>(in, n, h->scan_blocks, out, out2);
+  h->scan_epoch = (h->scan_epoch + 1) & 0x3fffffffu;
+  if (h->scan_epoch == 0) h->scan_epoch = 1;  // the words start as epoch 0
+  k_scan<<<(int)nb, kThreads, 0, h->stream>>>(in, n, h->scan_status, h->scan_ticket, h->scan_epoch, out, out2,
+                                              h->err_word);
   PSTEP_LAUNCHED(h);
   return PSTEP_OK;
 }
@@ -301,9 +328,9 @@ int csr_sort(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, const
     PSTEP_LAUNCHED(h);
   } else if (h->np > 0) {
     unsigned long long *items = (unsigned long long *)h->perm_tmp;  // capacity x 8 bytes, free between calls
-    k_scatter_items<<<blocks_for(h->np), kThreads, 0, h->stream>>>(keys, shift, h->np, order, h->cursor, items);
+    k_scatter_items<<<blocks_for(h->np), kThreads, 0, h->stream>>>(keys, shift, h->np, order, h->cursor, items,
+                                                                    h->big_count);
     PSTEP_LAUNCHED(h);
-    PSTEP_CUDA(cudaMemsetAsync(h->big_count, 0, sizeof(int32_t), h->stream));
     k_segrank<<<blocks_for(h->np, 256), 256, 0, h->stream>>>(items, keys, shift, h->np, cell_start, sidx, h->big_list,
                                                              h->big_count, h->err_word);
     PSTEP_LAUNCHED(h);
