@@ -150,18 +150,40 @@ constexpr int kB = 8;                 // brick edge (target cells)
 constexpr int kB1 = kB + 1;           // trilinear node region edge [b, b+B]; trunc cells [b-1, b+B-1]
 constexpr int kB2 = kB + 2;           // face node region edge [b-1, b+B]
 constexpr int kNodes = kB1 * kB1 * kB1, kRegion = kB2 * kB2 * kB2;
-constexpr int kBrickThreads = 256;
+constexpr int kBrickThreads = 384;
 // Lists longer than this are summed by a warp: lanes stride the particles in order and a
 // fixed shuffle tree adds the lane sums. The order is fixed by the list alone, so the result
 // is the same from run to run; one thread walking a blob-centre node (~1000 particles) would
 // hold up its whole brick.
-constexpr int kDenseSeg = 32;
-constexpr int kBins = kDenseSeg + 2;  // list lengths 0 .. kDenseSeg, and longer
+// The line: a warp pays ceil(n / 32) rounds and a reduction, 32 threads with lists alike n rounds
+// for 32 lists; beside each other at 2^24 particles in 64 blobs: node lists up to 24, 32, 64, 128
+// by threads 2.06, 2.05, 1.86, 1.83 ms (temperature deposit), but cell lists, which gather from
+// eight runs, 4.28, 4.13, 4.50, 4.77 ms (with the trilinear part).
+constexpr int kDenseNode = 64, kDenseCell = 32;
+constexpr int kBins = kDenseNode + 2;  // list lengths 0 .. 64, and longer
 
-__device__ __forceinline__ double warp_tree_sum(double v) {
+// The warp's sums of m[0..7] in a fixed order; each round a lane hands over the half of its values
+// that its partner goes on with: 9 FP64 additions instead of 40. Lane l ends with the sum of
+// m[(l >> 2) & 7 as bits 4, 3, 2], the same in the four lanes of a value.
+__device__ __forceinline__ double warp_sums8(const double (&m)[8], int lane) {
+  double a[4];
+  bool up = lane & 16;
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-  return v;  // lane 0 holds the sum
+  for (int i = 0; i < 4; ++i) {
+    const double got = __shfl_xor_sync(0xffffffffu, up ? m[i] : m[i + 4], 16);
+    a[i] = (up ? m[i + 4] : m[i]) + got;
+  }
+  up = lane & 8;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const double got = __shfl_xor_sync(0xffffffffu, up ? a[i] : a[i + 2], 8);
+    a[i] = (up ? a[i + 2] : a[i]) + got;
+  }
+  up = lane & 4;
+  const double got = __shfl_xor_sync(0xffffffffu, up ? a[0] : a[1], 4);
+  double v = (up ? a[1] : a[0]) + got;
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  return v + __shfl_xor_sync(0xffffffffu, v, 1);
 }
 
 // The fast deposit sums moments per node instead of the 8 corner weights: with
@@ -173,14 +195,26 @@ __device__ __forceinline__ double warp_tree_sum(double v) {
 // this takes 3 + 4 + 8 FP64 operations instead of 6 + 3 + 24 (+ 8). x_l = frac + 0.5 - h is formed as
 // frac + (h ? -0.5 : 0.5), the same value (frac - 1 and frac - 0.5 are exact for
 // frac >= 0.5).
+template <int MODE> struct TriRec {
+  uint32_t key;
+  double f[3], v;
+};
 template <int MODE>
-__device__ __forceinline__ void moments_add(double (&m)[8], const DepIn &d, int32_t p) {
-  const uint32_t key = d.key[p];
-  const double f0 = d.frac[0][p], f1 = d.frac[1][p], f2 = d.frac[2][p];
-  const double v = MODE ? d.val[0][p] : 0.0;
-  const double xl = f0 + ((key & 4u) ? -0.5 : 0.5);
-  const double yl = f1 + ((key & 2u) ? -0.5 : 0.5);
-  const double zl = f2 + ((key & 1u) ? -0.5 : 0.5);
+__device__ __forceinline__ TriRec<MODE> tri_load(const DepIn &d, int32_t p) {
+  TriRec<MODE> r;
+  r.key = d.key[p];
+#pragma unroll
+  for (int D = 0; D < 3; ++D) r.f[D] = d.frac[D][p];
+  r.v = MODE ? d.val[0][p] : 0.0;
+  return r;
+}
+template <int MODE>
+__device__ __forceinline__ void moments_add(double (&m)[8], const TriRec<MODE> &r) {
+  const uint32_t key = r.key;
+  const double v = r.v;
+  const double xl = r.f[0] + ((key & 4u) ? -0.5 : 0.5);
+  const double yl = r.f[1] + ((key & 2u) ? -0.5 : 0.5);
+  const double zl = r.f[2] + ((key & 1u) ? -0.5 : 0.5);
   const double xy = xl * yl, xz = xl * zl, yz = yl * zl, xyz = xy * zl;
   if (MODE) {
     m[0] += v;
@@ -216,12 +250,23 @@ __device__ __forceinline__ void corners_of(double (&m)[8]) {
 }
 
 // face sums of one particle: (sum r, sum t r) per dimension, r = RHS_u component
-__device__ __forceinline__ void face_add(double (&f)[6], const DepIn &d, int32_t p) {
+struct FaceRec {
+  double f[3], r[3];
+};
+__device__ __forceinline__ FaceRec face_load(const DepIn &d, int32_t p) {
+  FaceRec q;
 #pragma unroll
   for (int D = 0; D < 3; ++D) {
-    const double r = d.val[D][p];
-    f[2 * D] += r;
-    f[2 * D + 1] = fma(d.frac[D][p], r, f[2 * D + 1]);
+    q.f[D] = d.frac[D][p];
+    q.r[D] = d.val[D][p];
+  }
+  return q;
+}
+__device__ __forceinline__ void face_add(double (&f)[6], const FaceRec &q) {
+#pragma unroll
+  for (int D = 0; D < 3; ++D) {
+    f[2 * D] += q.r[D];
+    f[2 * D + 1] = fma(q.f[D], q.r[D], f[2 * D + 1]);
   }
 }
 
@@ -257,7 +302,7 @@ template <int MODE> struct BrickSmem {
 // walks one item's list and the FP64 pipe is charged per warp instruction: lists of like
 // length side by side let a warp's lanes end together (in storage order a warp ran the longest
 // of 32 lists with about a quarter of its lanes live).
-template <int MODE>
+template <int DENSE, int MODE>
 __device__ __forceinline__ void order_by_length(BrickSmem<MODE> &sm) {
   const int lane = (int)(threadIdx.x & 31u);
   for (int q = threadIdx.x; q < kBins; q += blockDim.x) sm.bin[q] = 0;
@@ -283,7 +328,7 @@ __device__ __forceinline__ void order_by_length(BrickSmem<MODE> &sm) {
       }
       if (b < kBins) sm.bin[b] = carry + x - v;
       if (b == 0) sm.n_empty = v;
-      if (b == kBins - 1) sm.n_dense = v;
+      if (b == DENSE + 1) sm.n_dense = v;
       carry += __shfl_sync(0xffffffffu, x, 31);
     }
     if (lane == 0) sm.next = 0;
@@ -332,11 +377,12 @@ __device__ __forceinline__ void take_items(BrickSmem<MODE> &sm, Dense dense, Lig
 // all of a cell's particles are summed by one thread. Bound: the FP64 pipe; per particle 14 (15
 // in mode 1) operations for the trilinear sums and 6 for the faces, 12 + 7 a node and target,
 // 3 + 3 a cell and target. The pipe answers through a queue (short scoreboard), so a brick's
-// phases stay latency-bound between barriers: three CTAs per SM keep it 40% (mode 0) and 57%
-// (mode 1) busy. 256^3 cells x 2^24 particles in 64 blobs: 5.06 and 2.64 ms (a thread per node in
-// storage order, the faces in eight h-class phases over all nodes: 15 and 5 ms).
+// phases stay latency-bound between barriers (three CTAs per SM). 256^3 cells x 2^24 particles in
+// 64 blobs: 4.4 and 1.7 ms, of the first 1.9 the trilinear part, 0.8 the class table and order
+// of the cells, 1.7 the face sums (a thread per node in storage order, the faces in eight
+// h-class phases over all nodes: 15 and 5 ms).
 template <int MODE>
-__global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, int twc,
+__global__ void __launch_bounds__(kBrickThreads, 3) k_dep_brick(Geom G, DepIn d, int twc,
                                                              double *__restrict__ out_tri,
                                                              double *__restrict__ out_x,
                                                              double *__restrict__ out_y,
@@ -378,13 +424,13 @@ __global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, in
     sm.count[s] = cnt;
     // the trilinear item of a node in [b, b+B]
     if (lx && ly && lz)
-      sm.length[((lz - 1) * kB1 + (ly - 1)) * kB1 + (lx - 1)] = (uint16_t)min(cnt, kDenseSeg + 1);
+      sm.length[((lz - 1) * kB1 + (ly - 1)) * kB1 + (lx - 1)] = (uint16_t)min(cnt, kDenseNode + 1);
   }
   for (int s = threadIdx.x; s < 8 * kNodes; s += blockDim.x) sm.tri[0][s] = 0.0;
   __syncthreads();
 
   // ---- trilinear: node items (slot l in [0, B]^3, region slot l + 1)
-  order_by_length(sm);
+  order_by_length<kDenseNode>(sm);
   auto region_of = [](int s) {
     const int lx = s % kB1, ly = (s / kB1) % kB1, lz = s / (kB1 * kB1);
     return ((lz + 1) * kB2 + (ly + 1)) * kB2 + (lx + 1);
@@ -397,15 +443,10 @@ __global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, in
         double m[8];
 #pragma unroll
         for (int o = 0; o < 8; ++o) m[o] = 0.0;
-        for (int32_t q = a + lane; q < a + cnt; q += 32) moments_add<MODE>(m, d, pidx(d, q));
-#pragma unroll
-        for (int o = MODE ? 0 : 1; o < 8; ++o) m[o] = warp_tree_sum(m[o]);
-        if (lane == 0) {
-          if (!MODE) m[0] = (double)cnt;
-          corners_of(m);
-#pragma unroll
-          for (int o = 0; o < 8; ++o) sm.tri[o][s] = m[o];
-        }
+        for (int32_t q = a + lane; q < a + cnt; q += 32) moments_add<MODE>(m, tri_load<MODE>(d, pidx(d, q)));
+        // the moments as they are; their corners below, a lane per node
+        const double v = warp_sums8(m, lane);
+        if (!(lane & 3)) sm.tri[lane >> 2][s] = !MODE && lane == 0 ? (double)cnt : v;
       },
       [&](int s) {
         const int rs = region_of(s);
@@ -413,12 +454,31 @@ __global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, in
         double m[8];
 #pragma unroll
         for (int o = 0; o < 8; ++o) m[o] = 0.0;
-        for (int32_t q = a; q < a + cnt; ++q) moments_add<MODE>(m, d, pidx(d, q));
+        // a list's loads ahead of its sums: the index two particles ahead, the record one
+        int32_t ahead = cnt > 1 ? pidx(d, a + 1) : 0;
+        TriRec<MODE> rec = tri_load<MODE>(d, pidx(d, a));
+        for (int32_t q = a + 1; q < a + cnt; ++q) {
+          const TriRec<MODE> next = tri_load<MODE>(d, ahead);
+          if (q + 1 < a + cnt) ahead = pidx(d, q + 1);
+          moments_add<MODE>(m, rec);
+          rec = next;
+        }
+        moments_add<MODE>(m, rec);
         if (!MODE) m[0] = (double)cnt;
         corners_of(m);
 #pragma unroll
         for (int o = 0; o < 8; ++o) sm.tri[o][s] = m[o];
       });
+  __syncthreads();
+  for (int w = threadIdx.x; w < sm.n_dense; w += blockDim.x) {
+    const int s = sm.order[kNodes - 1 - w];
+    double m[8];
+#pragma unroll
+    for (int o = 0; o < 8; ++o) m[o] = sm.tri[o][s];
+    corners_of(m);
+#pragma unroll
+    for (int o = 0; o < 8; ++o) sm.tri[o][s] = m[o];
+  }
   __syncthreads();
   // h classes and length of every cell item (slot l in [0, B]^3: cell b - 1 + l; its class-h run
   // is in the segment of region slot l + h)
@@ -444,7 +504,7 @@ __global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, in
         n += e - a;
         classes |= e > a ? 1 << hc : 0;
       }
-      sm.length[s] = (uint16_t)(min(n, kDenseSeg + 1) | classes << 8);
+      sm.length[s] = (uint16_t)(min(n, kDenseCell + 1) | classes << 8);
     }
   }
   for (int s = threadIdx.x; s < kB * kB * kB; s += blockDim.x) {
@@ -465,7 +525,7 @@ __global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, in
 
   // ---- faces
   for (int s = threadIdx.x; s < 6 * kNodes; s += blockDim.x) sm.face[0][s] = 0.0;
-  order_by_length(sm);
+  order_by_length<kDenseCell>(sm);
   auto put = [&](int s, const double (&fs)[6]) {
     // (1 - x_l) r summed as sum r - sum x_l r; x_l r as is
 #pragma unroll
@@ -483,21 +543,42 @@ __global__ void __launch_bounds__(kBrickThreads) k_dep_brick(Geom G, DepIn d, in
           const int hc = __ffs(classes) - 1;
           int32_t a, e;
           run(node_of(base, hc), hc, a, e);
-          for (int32_t q = a + lane; q < e; q += 32) face_add(fs, d, pidx(d, q));
+          for (int32_t q = a + lane; q < e; q += 32) face_add(fs, face_load(d, pidx(d, q)));
         }
-#pragma unroll
-        for (int j = 0; j < 6; ++j) fs[j] = warp_tree_sum(fs[j]);
-        if (lane == 0) put(s, fs);
+        const double m[8] = {fs[0], fs[1], fs[2], fs[3], fs[4], fs[5], 0.0, 0.0};
+        const double v = warp_sums8(m, lane);  // lanes 0, 4, .. 20: fs[0..5]
+        const double w = __shfl_down_sync(0xffffffffu, v, 4);
+        // (1 - x_l) r summed as sum r - sum x_l r; x_l r as is
+        if (!(lane & 7) && lane < 24) {
+          sm.face[lane >> 2][s] = v - w;
+          sm.face[(lane >> 2) + 1][s] = w;
+        }
       },
       [&](int s) {
         const int base = ((s / (kB1 * kB1)) * kB2 + (s / kB1) % kB1) * kB2 + s % kB1;
         double fs[6] = {0, 0, 0, 0, 0, 0};
-        for (int classes = sm.length[s] >> 8; classes; classes &= classes - 1) {
-          const int hc = __ffs(classes) - 1;
-          int32_t a, e;
-          run(node_of(base, hc), hc, a, e);
-          for (int32_t q = a; q < e; ++q) face_add(fs, d, pidx(d, q));
+        // the cell's particles one after the other, run by run; the next one's loads ahead
+        int classes = sm.length[s] >> 8;
+        int32_t q = 0, e = 0;
+        auto next = [&]() -> int32_t {  // -1 at the end
+          if (q == e) {
+            if (!classes) return -1;
+            const int hc = __ffs(classes) - 1;
+            classes &= classes - 1;
+            run(node_of(base, hc), hc, q, e);
+          }
+          return pidx(d, q++);
+        };
+        int32_t ahead = next();
+        FaceRec rec = face_load(d, ahead);
+        ahead = next();
+        while (ahead >= 0) {
+          const FaceRec following = face_load(d, ahead);
+          ahead = next();
+          face_add(fs, rec);
+          rec = following;
         }
+        face_add(fs, rec);
         put(s, fs);
       });
   __syncthreads();
