@@ -133,6 +133,7 @@ void release(pstep_ctx *h) {
   for (int d = 0; d < 3; ++d) { dfree(h->s.frac_prev[d]); dfree(h->s.frac_new[d]); dfree(h->s.rhs_u[d]); }
   dfree(h->s.key_prev); dfree(h->s.key_new);
   dfree(h->csr_prev.cell_start); dfree(h->csr_prev.sidx); dfree(h->csr_new.cell_start); dfree(h->csr_new.sidx);
+  dfree(h->csr_prev.okey); dfree(h->csr_new.okey);
   dfree(h->counts); dfree(h->cursor); dfree(h->scan_status); dfree(h->scan_ticket); dfree(h->big_list); dfree(h->big_count);
   void *pt = h->perm_tmp; if (pt) cudaFree(pt); h->perm_tmp = nullptr;
   for (int d = 0; d < 3; ++d) dfree(h->own_u[d]);
@@ -171,6 +172,9 @@ int alloc_all(pstep_ctx *h) {
     if (h->cfg.flags & PSTEP_TRACK_ORDER) {
       TRY(dalloc(h, h->ref_of_phys, cap)); TRY(dalloc(h, h->phys_of_ref, cap));
       TRY(dalloc(h, h->leave_code, cap));
+      if (h->cfg.flags & PSTEP_REFERENCE_SUMS) {
+        TRY(dalloc(h, h->csr_prev.okey, cap)); TRY(dalloc(h, h->csr_new.okey, cap));
+      }
       h->ord_scratch_len = (int64_t)cap + 64;
       TRY(dalloc(h, h->ord_scratch, (size_t)order_scratch_words((int64_t)cap)));
       TRY(dalloc(h, h->ord_count, 8));

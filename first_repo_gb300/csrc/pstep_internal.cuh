@@ -65,6 +65,7 @@ struct F32Form;
 struct Csr {
   int32_t *cell_start;  // gsize + 1
   int32_t *sidx;        // sorted physical indices
+  int32_t *okey;        // REFERENCE_SUMS: the sorted particles' reference positions (order within a node)
   int identity;         // sidx[i] == i (after the per-step reorder)
 };
 
@@ -180,7 +181,7 @@ int f64_stage_temp(pstep_ctx *h);
 int f64_reorder(pstep_ctx *h);
 int sort_by_node(pstep_ctx *h, const uint32_t *keys, Csr &out);
 int csr_sort(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, const int32_t *order, int32_t *cell_start,
-             int32_t *sidx, int order_within);
+             int32_t *sidx, int32_t *okey, int order_within);
 int csr_count(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, int32_t *cell_start);
 template <typename T>
 __global__ void k_gather(const T *__restrict__ src, const int32_t *__restrict__ idx, int64_t n, T *__restrict__ dst);

@@ -219,7 +219,7 @@ constexpr int kBigSegMax = 16384;     // per-node particles sortable on chip (8 
 __global__ void __launch_bounds__(256) k_segrank(const unsigned long long *__restrict__ items,
                                                  const uint32_t *__restrict__ keys, int shift, int64_t n,
                                                  const int32_t *__restrict__ cell_start, int32_t *__restrict__ sidx,
-                                                 int32_t *__restrict__ big_list, int32_t *__restrict__ big_count,
+                                                 int32_t *__restrict__ okey, int32_t *__restrict__ big_list, int32_t *__restrict__ big_count,
                                                  int32_t *__restrict__ err) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
@@ -232,17 +232,22 @@ __global__ void __launch_bounds__(256) k_segrank(const unsigned long long *__res
       if (b - a > kBigSegMax) atomicOr(err, kErrCapacity);
       big_list[atomicAdd(big_count, 1)] = (int32_t)node;
     }
-    if (b - a > kBigSegMax) sidx[p] = v;  // left unsorted, reported
+    if (b - a > kBigSegMax) {  // left unsorted, reported
+      sidx[p] = v;
+      if (okey) okey[p] = (int32_t)(mine >> 32);
+    }
     return;
   }
   int rank = 0;
   for (int32_t q = a; q < b; ++q) rank += items[q] < mine ? 1 : 0;
   sidx[a + rank] = v;
+  if (okey) okey[a + rank] = (int32_t)(mine >> 32);
 }
 
 // one block per listed long segment of (lo, hi] items: bitonic sort in shared memory
 __global__ void k_segsort_big(const int32_t *__restrict__ cell_start, const unsigned long long *__restrict__ items,
-                              int32_t *__restrict__ sidx, const int32_t *__restrict__ big_list,
+                              int32_t *__restrict__ sidx, int32_t *__restrict__ okey,
+                              const int32_t *__restrict__ big_list,
                               const int32_t *__restrict__ big_count, int32_t lo, int32_t hi) {
   extern __shared__ unsigned long long sk[];
   const int32_t nbig = *big_count;
@@ -269,7 +274,10 @@ __global__ void k_segsort_big(const int32_t *__restrict__ cell_start, const unsi
         __syncthreads();
       }
     }
-    for (int32_t q = threadIdx.x; q < len; q += blockDim.x) sidx[a + q] = (int32_t)(uint32_t)sk[q];
+    for (int32_t q = threadIdx.x; q < len; q += blockDim.x) {
+      sidx[a + q] = (int32_t)(uint32_t)sk[q];
+      if (okey) okey[a + q] = (int32_t)(sk[q] >> 32);
+    }
     __syncthreads();
   }
 }
@@ -315,7 +323,7 @@ int64_t scan_blocks_needed(int64_t n) { return (n + kScanTile - 1) / kScanTile; 
 // Counting sort of the h->np particles by (keys[i] >> shift) into nkeys buckets:
 // cell_start[0..nkeys] and sidx, every bucket ordered by the secondary key.
 int csr_sort(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, const int32_t *order, int32_t *cell_start,
-             int32_t *sidx, int order_within) {
+             int32_t *sidx, int32_t *okey, int order_within) {
   PSTEP_CUDA(cudaMemsetAsync(h->counts, 0, sizeof(int32_t) * nkeys, h->stream));
   if (h->np > 0) {
     k_count<<<blocks_for(h->np), kThreads, 0, h->stream>>>(keys, shift, h->np, h->counts);
@@ -331,16 +339,17 @@ int csr_sort(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, const
     k_scatter_items<<<blocks_for(h->np), kThreads, 0, h->stream>>>(keys, shift, h->np, order, h->cursor, items,
                                                                     h->big_count);
     PSTEP_LAUNCHED(h);
-    k_segrank<<<blocks_for(h->np, 256), 256, 0, h->stream>>>(items, keys, shift, h->np, cell_start, sidx, h->big_list,
+    k_segrank<<<blocks_for(h->np, 256), 256, 0, h->stream>>>(items, keys, shift, h->np, cell_start, sidx, okey,
+                                                             h->big_list,
                                                              h->big_count, h->err_word);
     PSTEP_LAUNCHED(h);
     k_segsort_big<<<8 * h->num_sms, 256, kMidSeg * sizeof(unsigned long long), h->stream>>>(
-        cell_start, items, sidx, h->big_list, h->big_count, kRankSeg, kMidSeg);
+        cell_start, items, sidx, okey, h->big_list, h->big_count, kRankSeg, kMidSeg);
     PSTEP_LAUNCHED(h);
     if (h->np > kMidSeg) {
       const size_t smem = (size_t)kBigSegMax * sizeof(unsigned long long);
       PSTEP_CUDA(cudaFuncSetAttribute(k_segsort_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_segsort_big<<<h->num_sms, 1024, smem, h->stream>>>(cell_start, items, sidx, h->big_list, h->big_count,
+      k_segsort_big<<<h->num_sms, 1024, smem, h->stream>>>(cell_start, items, sidx, okey, h->big_list, h->big_count,
                                                            kMidSeg, kBigSegMax);
       PSTEP_LAUNCHED(h);
     }
@@ -362,7 +371,8 @@ int csr_count(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, int3
 int sort_by_node(pstep_ctx *h, const uint32_t *keys, Csr &out) {
   const int32_t *order =
       ((h->cfg.flags & PSTEP_TRACK_ORDER) && (h->cfg.flags & PSTEP_REFERENCE_SUMS)) ? h->ref_of_phys : nullptr;
-  int rc = csr_sort(h, keys, 3, h->geom.gsize, order, out.cell_start, out.sidx, 1);
+  int rc = csr_sort(h, keys, 3, h->geom.gsize, order, out.cell_start, out.sidx,
+                    order ? out.okey : nullptr, 1);
   out.identity = 0;
   return rc;
 }

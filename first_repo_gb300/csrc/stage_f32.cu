@@ -1624,7 +1624,7 @@ int sort_step(pstep_ctx *h, bool check_sorted = false) {
   if (in_order)
     TRY32(csr_count(h, f.key, 0, ncell, f.cell_start));
   else
-    TRY32(csr_sort(h, f.key, 0, ncell, h->s.flag, f.cell_start, f.sidx, 0));
+    TRY32(csr_sort(h, f.key, 0, ncell, h->s.flag, f.cell_start, f.sidx, nullptr, 0));
   if (n > 0 && !in_order) {
     Set32 &B = f.set[SBASE];
     // every 4-byte per-particle array that lives across steps; the addresses of their
