@@ -116,10 +116,6 @@ __global__ void k_gather_ref_i(const int32_t *__restrict__ src, const int32_t *_
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = src[phys_of_ref ? phys_of_ref[i] : i];
 }
-__global__ void k_fill_i32(int32_t *a, int64_t n, int32_t v) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) a[i] = v;
-}
 
 int blocks_for(int64_t n) { return (int)((n + kThreads - 1) / kThreads); }
 
@@ -175,13 +171,9 @@ int alloc_all(pstep_ctx *h) {
       if (h->cfg.flags & PSTEP_REFERENCE_SUMS) {
         TRY(dalloc(h, h->csr_prev.okey, cap)); TRY(dalloc(h, h->csr_new.okey, cap));
       }
-      h->ord_scratch_len = (int64_t)cap + 64;
       TRY(dalloc(h, h->ord_scratch, (size_t)order_scratch_words((int64_t)cap)));
       TRY(dalloc(h, h->ord_count, 8));
-      // anchor slots start empty (-1); the order passes restore them after use
-      int32_t *slots = h->ord_scratch + 5 * h->ord_scratch_len;
-      k_fill_i32<<<blocks_for(h->ord_scratch_len), kThreads, 0, h->stream>>>(slots, h->ord_scratch_len, -1);
-      PSTEP_LAUNCHED(h);
+      TRY(order_clear(h));
     }
   }
   {  // permutation / download scratch, both forms
@@ -198,7 +190,7 @@ int alloc_all(pstep_ctx *h) {
   TRY(dalloc(h, h->scan_status, (size_t)h->scan_nblocks));
   TRY(dalloc(h, h->scan_ticket, 1));
   PSTEP_CUDA(cudaMemsetAsync(h->scan_status, 0, sizeof(unsigned long long) * h->scan_nblocks, h->stream));
-  PSTEP_CUDA(cudaMemsetAsync(h->scan_ticket, 0, sizeof(int32_t), h->stream));
+  PSTEP_CUDA(cudaMemsetAsync(h->scan_ticket, 0, sizeof(unsigned long long), h->stream));
   for (int f = 0; f < PSTEP_NUM_FIELDS; ++f) {
     TRY(dalloc(h, h->dep[f], gs));
     PSTEP_CUDA(cudaMemsetAsync(h->dep[f], 0, sizeof(double) * gs, h->stream));

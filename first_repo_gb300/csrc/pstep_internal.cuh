@@ -95,9 +95,8 @@ struct pstep_ctx {
   // counting sort scratch
   int32_t *counts;      // gsize
   int32_t *cursor;      // gsize
-  unsigned long long *scan_status;  // one word per tile of a scan, and the scans' ticket and epoch
-  int32_t *scan_ticket;
-  uint32_t scan_epoch;
+  unsigned long long *scan_status;  // one word per tile of a scan (scan.cuh), and the scans' ticket
+  unsigned long long *scan_ticket;
   int32_t *big_list;    // nodes with long segments (gsize)
   int32_t *big_count;   // device counter
   int64_t scan_nblocks;
@@ -124,7 +123,6 @@ struct pstep_ctx {
   uint32_t *bitmap;         // n bits
   int32_t *ord_scratch;     // misc scratch for the order passes
   int32_t *ord_count;       // device counters
-  int64_t ord_scratch_len;
 
   int32_t *err_word;  // device
 
@@ -195,5 +193,6 @@ int f32_fused_max(pstep_ctx *h, int id, double *out);
 int f64_fused_max(pstep_ctx *h, int id, double *out);
 int order_passes(pstep_ctx *h);
 int order_init(pstep_ctx *h);
+int order_clear(pstep_ctx *h);
 int order_permute(pstep_ctx *h, const int32_t *sidx);
 }  // namespace pstep

@@ -1,0 +1,105 @@
+// One-pass scans over tiles (decoupled look-back), for kernels whose blocks take a tile each: every
+// block takes the next tile by a ticket, publishes its tile's sum, then adds up its predecessors'
+// published values from the nearest one back until it meets an inclusive prefix. Tickets are handed
+// out in order, so a tile's predecessors are running or done; the wait is bounded all the same. A
+// tile's word is (epoch, state, value): words of an earlier scan are told by their epoch, so nothing
+// is cleared. The epoch is counted on the device beside the ticket, so that a launch that is
+// replayed has one of its own each time.
+#pragma once
+#include "pstep_internal.cuh"
+
+namespace pstep {
+
+struct ScanState {
+  unsigned long long *status;  // a word per tile
+  unsigned long long *ticket;  // epoch << 32 | the next tile
+  int32_t *err;
+};
+
+inline ScanState scan_state(pstep_ctx *h) { return ScanState{h->scan_status, h->scan_ticket, h->err_word}; }
+
+constexpr uint32_t kScanSum = 1, kScanPrefix = 2;
+constexpr uint32_t kScanEpochs = 0x3fffffffu;
+constexpr uint32_t kScanWait = 1u << 24;  // polls of one predecessor
+
+// The block's tile of this launch (all threads call).
+__device__ inline int32_t scan_take(const ScanState &scan, uint32_t &epoch) {
+  __shared__ unsigned long long taken;
+  if (threadIdx.x == 0) {
+    const unsigned long long t = atomicAdd(scan.ticket, 1ull);
+    if ((uint32_t)t == gridDim.x - 1)  // the last one of this launch
+      *scan.ticket = (((t >> 32) + 1) & kScanEpochs) << 32;
+    taken = t;
+  }
+  __syncthreads();
+  epoch = (uint32_t)(taken >> 32);
+  return (int32_t)(uint32_t)taken;
+}
+
+// The sum of the tiles before `tile`, whose own sum is `total` (one whole warp calls).
+__device__ inline int32_t scan_before(const ScanState &scan, uint32_t epoch, int32_t tile, int32_t total) {
+  const int lane = (int)(threadIdx.x & 31);
+  volatile unsigned long long *st = scan.status;
+  auto word = [&](uint32_t state, int32_t value) {
+    return ((unsigned long long)(epoch * 4 + state) << 32) | (uint32_t)value;
+  };
+  if (tile == 0) {
+    if (lane == 0) st[0] = word(kScanPrefix, total);
+    return 0;
+  }
+  if (lane == 0) st[tile] = word(kScanSum, total);
+  int32_t before = 0;
+  for (int32_t at = tile - 1; at >= 0; at -= 32) {  // 32 predecessors at a time, the nearest in lane 0
+    const int32_t q = at - lane;
+    uint32_t state = kScanPrefix;
+    int32_t value = 0;
+    if (q >= 0) {
+      unsigned long long w = st[q];
+      uint32_t polls = 0;
+      while ((uint32_t)(w >> 34) != epoch || ((uint32_t)(w >> 32) & 3u) == 0) {
+        if (++polls == kScanWait) {
+          atomicOr(scan.err, kErrTimeout);
+          break;
+        }
+        w = st[q];
+      }
+      state = (uint32_t)(w >> 32) & 3u;
+      value = (int32_t)(uint32_t)w;
+    }
+    const unsigned prefix = __ballot_sync(0xffffffffu, state == kScanPrefix);
+    const int stop = prefix ? __ffs(prefix) - 1 : 31;
+    before += (int32_t)__reduce_add_sync(0xffffffffu, (unsigned)(lane <= stop ? value : 0));
+    if (prefix) break;
+  }
+  if (lane == 0) st[tile] = word(kScanPrefix, before + total);
+  return before;
+}
+
+// Exclusive scan over the block's kThreads threads; smem: kThreads / 32 words.
+__device__ inline int32_t block_excl_scan(int32_t v, int32_t *smem, int32_t &total) {
+  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) smem[w] = x;
+  __syncthreads();
+  if (w == 0) {
+    int32_t s = lane < (kThreads / 32) ? smem[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      int32_t y = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += y;
+    }
+    if (lane < (kThreads / 32)) smem[lane] = s;
+  }
+  __syncthreads();
+  int32_t warp_off = w > 0 ? smem[w - 1] : 0;
+  total = smem[kThreads / 32 - 1];
+  __syncthreads();
+  return warp_off + x - v;
+}
+
+}  // namespace pstep

@@ -5,7 +5,7 @@
 // Order within a node is fixed by an explicit secondary key (the particle's
 // position in the reference's vectors, or its storage index), so the CSR -- and
 // every sum taken over it -- is identical from run to run.
-#include "pstep_internal.cuh"
+#include "scan.cuh"
 
 namespace pstep {
 namespace {
@@ -25,55 +25,16 @@ __global__ void k_count(const uint32_t *__restrict__ keys, int shift, int64_t n,
   if ((int)(threadIdx.x & 31) == leader) atomicAdd(&counts[node], __popc(peers));
 }
 
-__device__ inline int32_t block_excl_scan(int32_t v, int32_t *smem, int32_t &total) {
-  // smem: kThreads/32 ints
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int32_t x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    int32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) smem[w] = x;
-  __syncthreads();
-  if (w == 0) {
-    int32_t s = lane < (kThreads / 32) ? smem[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      int32_t y = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += y;
-    }
-    if (lane < (kThreads / 32)) smem[lane] = s;
-  }
-  __syncthreads();
-  int32_t warp_off = w > 0 ? smem[w - 1] : 0;
-  total = smem[kThreads / 32 - 1];
-  __syncthreads();
-  return warp_off + x - v;
-}
-
-// Exclusive scan in one pass (decoupled look-back): every block takes the next tile by a ticket,
-// publishes its tile's sum, then adds up its predecessors' published values from the nearest one
-// back until it meets an inclusive prefix. Tickets are handed out in order, so a tile's
-// predecessors are running or done; the wait is bounded all the same. A tile's word is
-// (epoch, state, value): words of an earlier scan are told by their epoch, so nothing is cleared.
-// Writes out[0..n] (out[n] = total) and out2 (optional). The three-launch form (tile sums, their
-// scan by one block, apply) took 9.3 us at 64^3 keys and 26 us at 256^3, this 4.5 and 25 us.
-constexpr uint32_t kScanSum = 1, kScanPrefix = 2;
-constexpr uint32_t kScanWait = 1u << 24;  // polls of one predecessor
-__global__ void __launch_bounds__(kThreads) k_scan(const int32_t *__restrict__ in, int64_t n, unsigned long long *status,
-                                                   int32_t *ticket, uint32_t epoch, int32_t *__restrict__ out,
-                                                   int32_t *__restrict__ out2, int32_t *__restrict__ err) {
+// Exclusive scan in one pass (scan_take, scan_before). Writes out[0..n] (out[n] = total) and out2
+// (optional). The three-launch form (tile sums, their scan by one block, apply) took 9.3 us at 64^3
+// keys and 26 us at 256^3, this 4.5 and 25 us.
+__global__ void __launch_bounds__(kThreads) k_scan(const int32_t *__restrict__ in, int64_t n, ScanState scan,
+                                                   int32_t *__restrict__ out, int32_t *__restrict__ out2) {
   static_assert(kScanItems % 4 == 0, "whole 16-byte vectors per thread");
   __shared__ int32_t sm[kThreads / 32];
-  __shared__ int32_t s_tile, s_before;
-  if (threadIdx.x == 0) {
-    const int32_t t = atomicAdd(ticket, 1);
-    if (t == (int32_t)gridDim.x - 1) *ticket = 0;  // the last ticket of this scan
-    s_tile = t;
-  }
-  __syncthreads();
-  const int32_t tile = s_tile;
+  __shared__ int32_t s_before;
+  uint32_t epoch;
+  const int32_t tile = scan_take(scan, epoch);
   int64_t base = (int64_t)tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
   // whole tiles move as 16-byte vectors (the arrays are 16-byte aligned and base is a
   // multiple of 4 elements); the ragged last tile element by element
@@ -95,41 +56,8 @@ __global__ void __launch_bounds__(kThreads) k_scan(const int32_t *__restrict__ i
   int32_t total;
   int32_t e = block_excl_scan(s, sm, total);
   if (threadIdx.x < 32) {
-    const int lane = (int)threadIdx.x;
-    volatile unsigned long long *st = status;
-    auto word = [&](uint32_t state, int32_t value) {
-      return ((unsigned long long)(epoch * 4 + state) << 32) | (uint32_t)value;
-    };
-    int32_t before = 0;
-    if (tile == 0) {
-      if (lane == 0) st[0] = word(kScanPrefix, total);
-    } else {
-      if (lane == 0) st[tile] = word(kScanSum, total);
-      for (int32_t at = tile - 1; at >= 0; at -= 32) {  // 32 predecessors at a time, the nearest in lane 0
-        const int32_t q = at - lane;
-        uint32_t state = kScanPrefix;
-        int32_t value = 0;
-        if (q >= 0) {
-          unsigned long long w = st[q];
-          uint32_t polls = 0;
-          while ((uint32_t)(w >> 34) != (epoch & 0x3fffffffu) || ((uint32_t)(w >> 32) & 3u) == 0) {
-            if (++polls == kScanWait) {
-              atomicOr(err, kErrTimeout);
-              break;
-            }
-            w = st[q];
-          }
-          state = (uint32_t)(w >> 32) & 3u;
-          value = (int32_t)(uint32_t)w;
-        }
-        const unsigned prefix = __ballot_sync(0xffffffffu, state == kScanPrefix);
-        const int stop = prefix ? __ffs(prefix) - 1 : 31;
-        before += (int32_t)__reduce_add_sync(0xffffffffu, (unsigned)(lane <= stop ? value : 0));
-        if (prefix) break;
-      }
-      if (lane == 0) st[tile] = word(kScanPrefix, before + total);
-    }
-    if (lane == 0) s_before = before;
+    const int32_t before = scan_before(scan, epoch, tile, total);
+    if (threadIdx.x == 0) s_before = before;
   }
   __syncthreads();
   e += s_before;
@@ -310,10 +238,7 @@ int exclusive_scan(pstep_ctx *h, const int32_t *in, int64_t n, int32_t *out, int
     snprintf(h->err, sizeof h->err, "scan scratch too small");
     return PSTEP_ERR_STATE;
   }
-  h->scan_epoch = (h->scan_epoch + 1) & 0x3fffffffu;
-  if (h->scan_epoch == 0) h->scan_epoch = 1;  // the words start as epoch 0
-  k_scan<<<(int)nb, kThreads, 0, h->stream>>>(in, n, h->scan_status, h->scan_ticket, h->scan_epoch, out, out2,
-                                              h->err_word);
+  k_scan<<<(int)nb, kThreads, 0, h->stream>>>(in, n, scan_state(h), out, out2);
   PSTEP_LAUNCHED(h);
   return PSTEP_OK;
 }
