@@ -632,120 +632,133 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_dep_brick(Geom G, DepIn d,
   }
 }
 
-// communicator.cpp:422-511 on one rank, one phase per launch; nf fields at once
+// The cumulative ghost fold (communicator.cpp:422-511 on one rank: z, then y, then x, every layer
+// added to its image), the ghost refresh (communicator.cpp:177-278) and the interior sum of up to
+// four fields in one launch. A boundary cell's up to seven ghost images belong to no other cell, so
+// its thread reads them all, adds them in the order of the three passes and leaves in them what
+// the passes leave: fields before `first` keep the partly folded ghosts, the others take the
+// refreshed value and are summed over their interior, in an order fixed by the grid alone: a warp a
+// row (j, k), the rows over the warps, a tree over the block; the launch's last block adds the blocks.
+// Passes, refresh and sums as launches of their own, each a few microseconds of work and a gap, took
+// 91 us for the temperature and 205 for C and the momentum at 256^3 cells (and 5 launches each); this
+// 73 and 179 us.
 struct FieldSet {
-  double *f[5];
-  int nf;
+  double *f[4];
+  int first;
 };
-
-__global__ void k_fold_z(Geom G, FieldSet fs) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long plane = (long long)G.g[0] * G.g[1];
-  if (t >= plane * fs.nf) return;
-  int q = (int)(t / plane);
-  long long ij = t % plane;
-  double *f = fs.f[q];
-  const int K = G.g[2];
-  double top = f[(long long)(K - 1) * plane + ij], bot = f[ij];
-  f[(long long)(K - 2) * plane + ij] += bot;
-  f[plane + ij] += top;
-}
-
-__global__ void k_fold_y(Geom G, FieldSet fs) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long per = (long long)G.g[0] * G.n[2];
-  if (t >= per * fs.nf) return;
-  int q = (int)(t / per);
-  long long r = t % per;
-  int i = (int)(r % G.g[0]), k = (int)(r / G.g[0]) + 1;
-  double *f = fs.f[q];
-  const int J = G.g[1];
-  double top = f[glin(G, i, J - 1, k)], bot = f[glin(G, i, 0, k)];
-  f[glin(G, i, J - 2, k)] += bot;
-  f[glin(G, i, 1, k)] += top;
-}
-
-__global__ void k_fold_x(Geom G, FieldSet fs) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long per = (long long)G.n[1] * G.n[2];
-  if (t >= per * fs.nf) return;
-  int q = (int)(t / per);
-  long long r = t % per;
-  int j = (int)(r % G.n[1]) + 1, k = (int)(r / G.n[1]) + 1;
-  double *f = fs.f[q];
-  const int I = G.g[0];
-  double top = f[glin(G, I - 1, j, k)], bot = f[glin(G, 0, j, k)];
-  f[glin(G, I - 2, j, k)] += bot;
-  f[glin(G, 1, j, k)] += top;
-}
-
-// communicator.cpp:177-278 on one rank: its x, y and z passes leave in every ghost cell the value of
-// its periodic image; one launch over the ghost layers, reading interior cells only
-__global__ void k_refresh(Geom G, FieldSet fs) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long nz = 2ll * G.g[0] * G.g[1], ny = 2ll * G.g[0] * G.n[2], nx = 2ll * G.n[1] * G.n[2];
-  const long long per = nz + ny + nx;
-  if (t >= per * fs.nf) return;
-  double *f = fs.f[t / per];
-  t %= per;
-  int i, j, k;
-  if (t < nz) {
-    const unsigned u = (unsigned)t;
-    i = (int)(u % (unsigned)G.g[0]);
-    j = (int)((u / (unsigned)G.g[0]) % (unsigned)G.g[1]);
-    k = t < nz / 2 ? 0 : G.g[2] - 1;
-  } else if (t < nz + ny) {
-    const unsigned u = (unsigned)(t - nz), r = u / (unsigned)G.g[0];
-    i = (int)(u % (unsigned)G.g[0]);
-    k = (int)(r % (unsigned)G.n[2]) + 1;
-    j = (int)(r / (unsigned)G.n[2]) ? G.g[1] - 1 : 0;
-  } else {
-    const unsigned u = (unsigned)(t - nz - ny), r = u / (unsigned)G.n[1];
-    j = (int)(u % (unsigned)G.n[1]) + 1;
-    k = (int)(r % (unsigned)G.n[2]) + 1;
-    i = (int)(r / (unsigned)G.n[2]) ? G.g[0] - 1 : 0;
-  }
-  const int si = i == 0 ? G.n[0] : (i == G.g[0] - 1 ? 1 : i), sj = j == 0 ? G.n[1] : (j == G.g[1] - 1 ? 1 : j),
-            sk = k == 0 ? G.n[2] : (k == G.g[2] - 1 ? 1 : k);
-  f[glin(G, i, j, k)] = f[glin(G, si, sj, sk)];
-}
-
-// Interior sum, fixed order: per-block tree over a strided range, then one block.
 constexpr int kRedBlocks = 1024;
-// (blockIdx.y: the field, and its kRedBlocks partials)
-__global__ void k_sum_partial(Geom G, FieldSet fs, double *__restrict__ part) {
-  __shared__ double sm[kThreads];
-  const double *__restrict__ f = fs.f[blockIdx.y];
-  part += (size_t)blockIdx.y * kRedBlocks;
-  // rows (j,k) distributed over blocks, the i loop over threads: fixed order, coalesced
-  const long long rows = (long long)G.n[1] * G.n[2];
-  double s = 0.0;
-  for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-    const int j = (int)(r % G.n[1]) + 1, k = (int)(r / G.n[1]) + 1;
-    const double *row = f + glin(G, 0, j, k);
-    for (int i = threadIdx.x + 1; i <= G.n[0]; i += blockDim.x) s += row[i];
+
+__device__ inline double fold_cell(const Geom &G, double *f, int i, int j, int k, bool whole) {
+  const bool bx = i == 1 || i == G.n[0], by = j == 1 || j == G.n[1], bz = k == 1 || k == G.n[2];
+  const int x[2] = {i, i == 1 ? G.n[0] + 1 : 0}, y[2] = {j, j == 1 ? G.n[1] + 1 : 0}, z[2] = {k, k == 1 ? G.n[2] + 1 : 0};
+  double v[8];
+#pragma unroll
+  for (int o = 0; o < 8; ++o) {
+    const bool in = (!(o & 4) || bx) && (!(o & 2) || by) && (!(o & 1) || bz);
+    v[o] = in ? f[glin(G, x[o >> 2], y[(o >> 1) & 1], z[o & 1])] : 0.0;
   }
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = kThreads / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
-    __syncthreads();
+#pragma unroll
+  for (int o = 0; o < 8; o += 2)
+    if (bz) v[o] += v[o + 1];
+  const double z1 = v[2], z3 = v[6];
+  if (by) {
+    v[0] += v[2];
+    v[4] += v[6];
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
+  const double y1 = v[4];
+  if (bx) v[0] += v[4];
+  const double all = v[0];
+  f[glin(G, i, j, k)] = all;
+  if (whole) {
+#pragma unroll
+    for (int o = 1; o < 8; ++o)
+      if ((!(o & 4) || bx) && (!(o & 2) || by) && (!(o & 1) || bz))
+        f[glin(G, x[o >> 2], y[(o >> 1) & 1], z[o & 1])] = all;
+  } else {
+    if (by) f[glin(G, i, y[1], k)] = z1;
+    if (bx) f[glin(G, x[1], j, k)] = y1;
+    if (bx && by) f[glin(G, x[1], y[1], k)] = z3;
+  }
+  return all;
 }
 
-__global__ void k_sum_final(const double *__restrict__ part, int np, double inv_count, double *__restrict__ out) {
-  __shared__ double sm[kThreads];
-  part += (size_t)blockIdx.x * kRedBlocks;
+__global__ void __launch_bounds__(kThreads, 6) k_fold(Geom G, FieldSet fs, double scale, double *__restrict__ parts,
+                                                   unsigned *__restrict__ tickets, double *__restrict__ out) {
+  __shared__ double sm[kThreads / 32];
+  __shared__ bool last;
+  const bool whole = (int)blockIdx.y >= fs.first;
+  double *f = blockIdx.y < 2 ? (blockIdx.y ? fs.f[1] : fs.f[0]) : (blockIdx.y == 2 ? fs.f[2] : fs.f[3]);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, n0 = G.n[0];
+  const int rows = G.n[1] * G.n[2];
   double s = 0.0;
-  for (int i = threadIdx.x; i < np; i += kThreads) s += part[i];
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = kThreads / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sm[threadIdx.x] += sm[threadIdx.x + o];
-    __syncthreads();
+  // boundary rows take several times longer: the rows turn over the warps, or a warp would have one at
+  // every step where the number of warps is a multiple of n1
+  const int warps = (int)gridDim.x * (kThreads / 32);
+  int turn = (int)blockIdx.x * (kThreads / 32) + wid;
+  for (int first = 0; first < rows; first += warps, turn = turn + 37 < warps ? turn + 37 : (turn + 37) % warps) {
+    const int r = first + turn;
+    if (r >= rows) continue;
+    const int k = r / G.n[1] + 1, j = r - (k - 1) * G.n[1] + 1;
+    if (j == 1 || j == G.n[1] || k == 1 || k == G.n[2]) {
+      for (int i = lane + 1; i <= n0; i += 32) s += fold_cell(G, f, i, j, k, whole);
+      continue;
+    }
+    double *row = f + glin(G, 0, j, k);
+    // folded along x alone: lanes 0 and 1 the two ends
+    const int end = lane ? n0 : 1, ghost = lane ? 0 : n0 + 1;
+    double e = 0.0, g = 0.0;
+    if (lane < 2) {
+      e = row[end];
+      g = row[ghost];
+    }
+    if (whole) {
+      // four pieces of 32 cells at a time, their loads before the sums
+      for (int i0 = lane + 1; i0 - lane <= n0; i0 += 128) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + 32 * u;
+          v[u] = i > 1 && i < n0 ? row[i] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (i0 - lane + 32 * u <= n0) s += v[u];
+      }
+    }
+    if (lane < 2) {
+      e += g;
+      row[end] = e;
+      if (whole) {
+        row[ghost] = e;
+        s += e;
+      }
+    }
   }
-  if (threadIdx.x == 0) out[blockIdx.x] = sm[0] * inv_count;
+  if (!whole) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) sm[wid] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < kThreads / 32; ++q) s += sm[q];
+    parts[blockIdx.y * kRedBlocks + blockIdx.x] = s;
+    __threadfence();
+    last = atomicInc(&tickets[blockIdx.y], gridDim.x - 1) == gridDim.x - 1;  // back to 0 with the last
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const double *p = parts + blockIdx.y * kRedBlocks;
+  s = 0.0;
+  for (int q = threadIdx.x; q < (int)gridDim.x; q += kThreads) s += __ldcg(p + q);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) sm[wid] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < kThreads / 32; ++q) s += sm[q];
+    out[(int)blockIdx.y - fs.first] = s * scale;
+  }
 }
 
 inline int blocks_for(long long n) { return (int)((n + kThreads - 1) / kThreads); }
@@ -766,58 +779,28 @@ DepIn make_in(pstep_ctx *h, const Csr &csr, double *const frac[3], const uint32_
 
 }  // namespace
 
-// the cumulative fold of nf fields, then the ghost refresh of the last `refresh` of them
-int fold_fields(pstep_ctx *h, double *const *f, int nf, int refresh) {
+// folds f[0 .. nf); refreshes f[first .. nf) and leaves scale x their interior sums in out
+int fold_fields(pstep_ctx *h, double *const *f, int nf, int first, double scale, double *out) {
   const Geom &G = h->geom;
   FieldSet fs;
-  fs.nf = nf;
+  fs.first = first;
   for (int q = 0; q < nf; ++q) fs.f[q] = f[q];
-  long long plane = (long long)G.g[0] * G.g[1];
-  k_fold_z<<<blocks_for(plane * nf), kThreads, 0, h->stream>>>(G, fs);
-  PSTEP_LAUNCHED(h);
-  k_fold_y<<<blocks_for((long long)G.g[0] * G.n[2] * nf), kThreads, 0, h->stream>>>(G, fs);
-  PSTEP_LAUNCHED(h);
-  k_fold_x<<<blocks_for((long long)G.n[1] * G.n[2] * nf), kThreads, 0, h->stream>>>(G, fs);
-  PSTEP_LAUNCHED(h);
-  if (refresh) {
-    fs.nf = refresh;
-    for (int q = 0; q < refresh; ++q) fs.f[q] = f[nf - refresh + q];
-    const long long ghosts = 2 * plane + 2ll * G.g[0] * G.n[2] + 2ll * G.n[1] * G.n[2];
-    k_refresh<<<blocks_for(ghosts * refresh), kThreads, 0, h->stream>>>(G, fs);
-    PSTEP_LAUNCHED(h);
-  }
-  return PSTEP_OK;
-}
-
-int interior_mean(pstep_ctx *h, const double *f, double *out_dev) {
-  const Geom &G = h->geom;
-  FieldSet fs;
-  fs.nf = 1;
-  fs.f[0] = const_cast<double *>(f);
-  k_sum_partial<<<kRedBlocks, kThreads, 0, h->stream>>>(G, fs, h->red_partials);
-  PSTEP_LAUNCHED(h);
-  double inv = 1.0 / (double)((long long)G.n[0] * G.n[1] * G.n[2]);
-  k_sum_final<<<1, kThreads, 0, h->stream>>>(h->red_partials, kRedBlocks, inv, out_dev);
+  const long long rows = (long long)G.n[1] * G.n[2], blocks = (rows + kThreads / 32 - 1) / (kThreads / 32);
+  k_fold<<<dim3((unsigned)(blocks < kRedBlocks ? blocks : kRedBlocks), nf), kThreads, 0, h->stream>>>(
+      G, fs, scale, h->red_partials, h->red_tickets, out);
   PSTEP_LAUNCHED(h);
   return PSTEP_OK;
 }
 
-// The momentum balance of the last int deposit: the interior sums of RHS_RU x/y/z,
-// each in the fixed order of k_sum_partial / k_sum_final (zeros without TWC).
-int momentum_sums(pstep_ctx *h) {
-  const Geom &G = h->geom;
-  if (!h->cfg.twc) {
-    PSTEP_CUDA(cudaMemsetAsync(h->mom_dev, 0, 3 * sizeof(double), h->stream));
-    return PSTEP_OK;
-  }
-  FieldSet fs;
-  fs.nf = 3;
-  for (int d = 0; d < 3; ++d) fs.f[d] = h->dep[PSTEP_FIELD_RU_X + d];
-  double *part = h->red_partials + kRedBlocks;
-  k_sum_partial<<<dim3(kRedBlocks, 3), kThreads, 0, h->stream>>>(G, fs, part);
-  PSTEP_LAUNCHED(h);
-  k_sum_final<<<3, kThreads, 0, h->stream>>>(part, kRedBlocks, 1.0, h->mom_dev);
-  PSTEP_LAUNCHED(h);
+// C and, with TWC, the momentum fields and their balance (the interior sums); without, RHS_RU = 0
+// (grid.cpp:671)
+int fold_int(pstep_ctx *h) {
+  // (the reference does not refresh C's ghosts)
+  double *all[4] = {h->dep[PSTEP_FIELD_C], h->dep[PSTEP_FIELD_RU_X], h->dep[PSTEP_FIELD_RU_Y], h->dep[PSTEP_FIELD_RU_Z]};
+  const int rc = fold_fields(h, all, h->cfg.twc ? 4 : 1, 1, 1.0, h->mom_dev);
+  if (rc || h->cfg.twc) return rc;
+  for (int q = 1; q < 4; ++q) PSTEP_CUDA(cudaMemsetAsync(all[q], 0, sizeof(double) * h->geom.gsize, h->stream));
+  PSTEP_CUDA(cudaMemsetAsync(h->mom_dev, 0, 3 * sizeof(double), h->stream));
   return PSTEP_OK;
 }
 
@@ -862,41 +845,16 @@ int deposit_temperature(pstep_ctx *h, const Csr &csr, double *const frac[3], con
     if (rc) return rc;
   }
   double *fl[1] = {out};
-  int rc = fold_fields(h, fl, 1, 1);
-  if (rc) return rc;
-  return interior_mean(h, out, h->emean_dev);
+  return fold_fields(h, fl, 1, 0, 1.0 / (double)((long long)G.n[0] * G.n[1] * G.n[2]), h->emean_dev);
 }
 
 // part2gas_concentration + part2gas_velocity at x_int (records of the previous CSR)
 int f64_deposit_int(pstep_ctx *h) {
-  const Geom &G = h->geom;
   DepIn d = make_in(h, h->csr_prev, h->s.frac_prev, h->s.key_prev, h->s.rhs_u[0], h->s.rhs_u[1], h->s.rhs_u[2]);
-  if (!reference_sums(h)) {
-    int rc = brick_launch(h, d, 0, h->dep[PSTEP_FIELD_C], h->dep[PSTEP_FIELD_RU_X], h->dep[PSTEP_FIELD_RU_Y],
-                          h->dep[PSTEP_FIELD_RU_Z]);
-    if (rc) return rc;
-    // (the reference does not refresh C's ghosts)
-    double *all[4] = {h->dep[PSTEP_FIELD_C], h->dep[PSTEP_FIELD_RU_X], h->dep[PSTEP_FIELD_RU_Y],
-                      h->dep[PSTEP_FIELD_RU_Z]};
-    rc = fold_fields(h, all, h->cfg.twc ? 4 : 1, h->cfg.twc ? 3 : 0);
-    if (rc) return rc;
-    if (!h->cfg.twc) {
-      for (int q = PSTEP_FIELD_RU_X; q <= PSTEP_FIELD_RU_Z; ++q)
-        PSTEP_CUDA(cudaMemsetAsync(h->dep[q], 0, sizeof(double) * G.gsize, h->stream));
-    }
-    return momentum_sums(h);
-  }
-  // (the reference does not refresh C's ghosts)
-  double *all[4] = {h->dep[PSTEP_FIELD_C], h->dep[PSTEP_FIELD_RU_X], h->dep[PSTEP_FIELD_RU_Y], h->dep[PSTEP_FIELD_RU_Z]};
-  int rc = ordered_launch(h, d, h->cfg.twc, 0, all[0], all[1], all[2], all[3]);
-  if (rc) return rc;
-  rc = fold_fields(h, all, h->cfg.twc ? 4 : 1, h->cfg.twc ? 3 : 0);
-  if (rc) return rc;
-  if (!h->cfg.twc) {
-    for (int q = PSTEP_FIELD_RU_X; q <= PSTEP_FIELD_RU_Z; ++q)
-      PSTEP_CUDA(cudaMemsetAsync(h->dep[q], 0, sizeof(double) * G.gsize, h->stream));  // RHS_RU = 0 (grid.cpp:671)
-  }
-  return momentum_sums(h);
+  double *c = h->dep[PSTEP_FIELD_C], *x = h->dep[PSTEP_FIELD_RU_X], *y = h->dep[PSTEP_FIELD_RU_Y],
+         *z = h->dep[PSTEP_FIELD_RU_Z];
+  const int rc = reference_sums(h) ? ordered_launch(h, d, h->cfg.twc, 0, c, x, y, z) : brick_launch(h, d, 0, c, x, y, z);
+  return rc ? rc : fold_int(h);
 }
 
 }  // namespace pstep

@@ -135,7 +135,7 @@ void release(pstep_ctx *h) {
   for (int d = 0; d < 3; ++d) dfree(h->own_u[d]);
   dfree(h->own_t);
   for (int f = 0; f < PSTEP_NUM_FIELDS; ++f) dfree(h->dep[f]);
-  dfree(h->emean_dev); dfree(h->mom_dev); dfree(h->red_partials);
+  dfree(h->emean_dev); dfree(h->mom_dev); dfree(h->red_partials); dfree(h->red_tickets);
   dfree(h->pmax64);
   dfree(h->ref_of_phys); dfree(h->phys_of_ref); dfree(h->leave_code); dfree(h->ord_scratch); dfree(h->ord_count);
   dfree(h->err_word);
@@ -199,6 +199,8 @@ int alloc_all(pstep_ctx *h) {
   TRY(dalloc(h, h->mom_dev, 3));
   PSTEP_CUDA(cudaMemsetAsync(h->mom_dev, 0, 3 * sizeof(double), h->stream));
   TRY(dalloc(h, h->red_partials, 4 * 1024));
+  TRY(dalloc(h, h->red_tickets, 4));
+  PSTEP_CUDA(cudaMemsetAsync(h->red_tickets, 0, 4 * sizeof(unsigned), h->stream));
   TRY(dalloc(h, h->err_word, 1));
   PSTEP_CUDA(cudaMemsetAsync(h->err_word, 0, sizeof(int32_t), h->stream));
   PSTEP_CUDA(cudaMemsetAsync(h->emean_dev, 0, sizeof(double), h->stream));

@@ -111,6 +111,7 @@ struct pstep_ctx {
   double *emean_dev;       // device scalar
   double *mom_dev;         // device: interior sums of the three deposited momentum fields (last stage)
   double *red_partials;    // reduction scratch (4 x 1024)
+  unsigned *red_tickets;   // blocks done, per field (4); 0 between launches
   double emean_host;
   double mom_host[3];
 
@@ -183,10 +184,6 @@ int csr_sort(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, const
 int csr_count(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, int32_t *cell_start);
 template <typename T>
 __global__ void k_gather(const T *__restrict__ src, const int32_t *__restrict__ idx, int64_t n, T *__restrict__ dst);
-int fold_cum(pstep_ctx *h, double *f);
-int refresh_ghosts(pstep_ctx *h, double *f);
-int interior_mean(pstep_ctx *h, const double *f, double *out_dev);
-int momentum_sums(pstep_ctx *h);
 int f32_download(pstep_ctx *h, double *const dst[7], int32_t *flag, int on_device);
 int f32_field_stats(pstep_ctx *h, int field, double r[3]);
 int f32_fused_max(pstep_ctx *h, int id, double *out);

@@ -37,7 +37,6 @@
 #include "tc05.cuh"
 
 namespace pstep {
-int interior_mean(pstep_ctx *h, const double *f, double *out_dev);
 int exclusive_scan(pstep_ctx *h, const int32_t *in, int64_t n, int32_t *out, int32_t *out2);
 }  // namespace pstep
 
