@@ -117,6 +117,26 @@ __global__ void k_gather_ref_i(const int32_t *__restrict__ src, const int32_t *_
   if (i < n) dst[i] = src[phys_of_ref ? phys_of_ref[i] : i];
 }
 
+// the seven base arrays and the ids in the reference's order, a thread a particle
+struct BaseSet {
+  const double *src[7];
+  double *dst[7];
+};
+__global__ void __launch_bounds__(kThreads) k_gather_base(BaseSet b, const int32_t *__restrict__ flag,
+                                                          const int32_t *__restrict__ phys_of_ref, int64_t n,
+                                                          int32_t *__restrict__ flag_to) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int32_t j = phys_of_ref[i];
+  double v[7];
+#pragma unroll
+  for (int q = 0; q < 7; ++q) v[q] = b.src[q][j];
+  const int32_t f = flag[j];
+#pragma unroll
+  for (int q = 0; q < 7; ++q) __stcs(b.dst[q] + i, v[q]);
+  flag_to[i] = f;
+}
+
 int blocks_for(int64_t n) { return (int)((n + kThreads - 1) / kThreads); }
 
 bool is_f32(const pstep_ctx *h) { return h->cfg.precision == PSTEP_FP32; }
@@ -137,7 +157,7 @@ void release(pstep_ctx *h) {
   for (int f = 0; f < PSTEP_NUM_FIELDS; ++f) dfree(h->dep[f]);
   dfree(h->emean_dev); dfree(h->mom_dev); dfree(h->red_partials); dfree(h->red_tickets);
   dfree(h->pmax64);
-  dfree(h->ref_of_phys); dfree(h->phys_of_ref); dfree(h->leave_code); dfree(h->ord_scratch); dfree(h->ord_count);
+  dfree(h->ref_of_phys); dfree(h->phys_of_ref); dfree(h->ref_spare); dfree(h->leave_code); dfree(h->ord_scratch); dfree(h->ord_count);
   dfree(h->err_word);
   if (is_f32(h)) f32_destroy(h);
 }
@@ -166,7 +186,7 @@ int alloc_all(pstep_ctx *h) {
     TRY(dalloc(h, h->csr_prev.sidx, cap)); TRY(dalloc(h, h->csr_new.sidx, cap));
     TRY(dalloc(h, h->pmax64, 2 * 1024));
     if (h->cfg.flags & PSTEP_TRACK_ORDER) {
-      TRY(dalloc(h, h->ref_of_phys, cap)); TRY(dalloc(h, h->phys_of_ref, cap));
+      TRY(dalloc(h, h->ref_of_phys, cap)); TRY(dalloc(h, h->phys_of_ref, cap)); TRY(dalloc(h, h->ref_spare, cap));
       TRY(dalloc(h, h->leave_code, cap));
       if (h->cfg.flags & PSTEP_REFERENCE_SUMS) {
         TRY(dalloc(h, h->csr_prev.okey, cap)); TRY(dalloc(h, h->csr_new.okey, cap));
@@ -383,8 +403,32 @@ int pstep_download_particles(pstep_handle h, double *x, double *y, double *z, do
   if (h->np > 0 && (!x || !y || !z || !u || !v || !w || !t || !flag)) return fail(h, PSTEP_ERR_ARG, "null array");
   double *dst[7] = {x, y, z, u, v, w, t};
   if (is_f32(h)) return pstep::f32_download(h, dst, flag, on_device);
-  for (int q = 0; q < 7; ++q) TRY(pstep_get_particle_array(h, PSTEP_X + q, dst[q], on_device));
-  return pstep_get_particle_array(h, PSTEP_FLAG, flag, on_device);
+  const int64_t n = h->np;
+  if (n == 0) return PSTEP_OK;
+  const double *src[7];
+  const int32_t *ids = h->s.flag;
+  for (int q = 0; q < 7; ++q) src[q] = h->s.base[q];
+  if (h->cfg.flags & PSTEP_TRACK_ORDER) {
+    if (h->phase != 0 || !h->np1_is_base) {  // no free arrays within a step: one at a time through one scratch
+      for (int q = 0; q < 7; ++q) TRY(pstep_get_particle_array(h, PSTEP_X + q, dst[q], on_device));
+      return pstep_get_particle_array(h, PSTEP_FLAG, flag, on_device);
+    }
+    // between steps *_np1 and the new sort hold nothing. (2^24 particles: eight gathers 0.64 ms,
+    // together 0.32)
+    BaseSet b;
+    for (int q = 0; q < 7; ++q) {
+      b.src[q] = h->s.base[q];
+      src[q] = b.dst[q] = h->s.np1[q];
+    }
+    ids = h->csr_new.sidx;
+    k_gather_base<<<blocks_for(n), kThreads, 0, h->stream>>>(b, h->s.flag, h->phys_of_ref, n, h->csr_new.sidx);
+    PSTEP_LAUNCHED(h);
+  }
+  for (int q = 0; q < 7; ++q)
+    PSTEP_CUDA(cudaMemcpyAsync(dst[q], src[q], sizeof(double) * n, kind_out(on_device), h->stream));
+  PSTEP_CUDA(cudaMemcpyAsync(flag, ids, sizeof(int32_t) * n, kind_out(on_device), h->stream));
+  if (!on_device) PSTEP_CUDA(cudaStreamSynchronize(h->stream));
+  return PSTEP_OK;
 }
 
 int pstep_set_tau_p(pstep_handle h, const double *tau, int on_device) {

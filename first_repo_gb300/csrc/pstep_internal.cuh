@@ -117,6 +117,7 @@ struct pstep_ctx {
 
   // reference-order bookkeeping
   int32_t *ref_of_phys, *phys_of_ref;
+  int32_t *ref_spare;       // takes ref_of_phys's place in the per-step reorder
   uint8_t *leave_code;      // per particle: bit 2d = high side, bit 2d+1 = low side, dimension d
   unsigned long long *pmax64;  // FP64 form: 1024 x 2 order keys of the last stage's max u and max ug
   int pmax64_state;            // 0: none; 1: filled by this step's last stage; 2: valid for the base state
@@ -182,8 +183,6 @@ int sort_by_node(pstep_ctx *h, const uint32_t *keys, Csr &out);
 int csr_sort(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, const int32_t *order, int32_t *cell_start,
              int32_t *sidx, int32_t *okey, int order_within);
 int csr_count(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, int32_t *cell_start);
-template <typename T>
-__global__ void k_gather(const T *__restrict__ src, const int32_t *__restrict__ idx, int64_t n, T *__restrict__ dst);
 int f32_download(pstep_ctx *h, double *const dst[7], int32_t *flag, int on_device);
 int f32_field_stats(pstep_ctx *h, int field, double r[3]);
 int f32_fused_max(pstep_ctx *h, int id, double *out);
@@ -191,5 +190,4 @@ int f64_fused_max(pstep_ctx *h, int id, double *out);
 int order_passes(pstep_ctx *h);
 int order_init(pstep_ctx *h);
 int order_clear(pstep_ctx *h);
-int order_permute(pstep_ctx *h, const int32_t *sidx);
 }  // namespace pstep

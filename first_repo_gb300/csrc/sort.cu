@@ -212,20 +212,41 @@ __global__ void k_segsort_big(const int32_t *__restrict__ cell_start, const unsi
 
 }  // namespace
 
-template <typename T>
-__global__ void k_gather(const T *__restrict__ src, const int32_t *__restrict__ idx, int64_t n, T *__restrict__ dst) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = src[idx[i]];
-}
-template __global__ void k_gather<float>(const float *, const int32_t *, int64_t, float *);
-template __global__ void k_gather<uint32_t>(const uint32_t *, const int32_t *, int64_t, uint32_t *);
-template __global__ void k_gather<int32_t>(const int32_t *, const int32_t *, int64_t, int32_t *);
-
 namespace {
 
-__global__ void k_invert(const int32_t *__restrict__ ref_of_phys, int64_t n, int32_t *__restrict__ phys_of_ref) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) phys_of_ref[ref_of_phys[i]] = (int32_t)i;
+// The per-step reorder: a thread a particle, all its values at once, so that the index is read once
+// and the gathers (short runs: a particle moves a fraction of a cell a step) are in flight together.
+// Bound by memory: 12 values, three words and the index each way. As a launch per array, the words
+// through one scratch array and back: 2^24 particles 1.20 ms, 131,072 85 us in 19 launches; this way
+// 0.52 ms and 4 us.
+constexpr int kReorderArrays = 12;
+struct Reorder {
+  const double *src[kReorderArrays];
+  double *dst[kReorderArrays];
+  const int32_t *flag, *ref;
+  const uint32_t *key;
+  int32_t *flag_to, *ref_to, *phys_of_ref;
+  uint32_t *key_to;
+};
+__global__ void __launch_bounds__(kThreads) k_reorder(Reorder r, int arrays, const int32_t *__restrict__ idx, int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int32_t j = __ldcs(idx + i);
+  double v[kReorderArrays];
+#pragma unroll
+  for (int a = 0; a < kReorderArrays; ++a)
+    if (a < arrays) v[a] = r.src[a][j];
+  const int32_t flag = r.flag[j], ref = r.ref ? r.ref[j] : 0;
+  const uint32_t key = r.key[j];
+#pragma unroll
+  for (int a = 0; a < kReorderArrays; ++a)
+    if (a < arrays) __stcs(r.dst[a] + i, v[a]);
+  __stcs(r.flag_to + i, flag);
+  __stcs(r.key_to + i, key);
+  if (r.ref) {
+    __stcs(r.ref_to + i, ref);
+    r.phys_of_ref[ref] = (int32_t)i;
+  }
 }
 
 inline int blocks_for(int64_t n, int per = kThreads) { return (int)((n + per - 1) / per); }
@@ -303,44 +324,42 @@ int sort_by_node(pstep_ctx *h, const uint32_t *keys, Csr &out) {
 }
 
 // Reorder particle storage by csr_prev.sidx (the sort of the positions the next
-// stage starts from): every per-particle array is gathered through the
-// permutation into scratch and the pointers swapped.
+// stage starts from): every per-particle array is gathered through the permutation into one that
+// holds nothing between steps (*_np1 and *_new are the base then, the new records and the
+// new sort not yet made), and the pointers are swapped.
 int f64_reorder(pstep_ctx *h) {
   const int64_t n = h->np;
   if (n == 0) return PSTEP_OK;
-  const int32_t *idx = h->csr_prev.sidx;
-  const int bl = blocks_for(n);
-  double *tmp = (double *)h->perm_tmp;
-  // each array is gathered into the free buffer, which then takes the array's place
-  auto gd = [&](double *&arr) {
-    k_gather<double><<<bl, kThreads, 0, h->stream>>>(arr, idx, n, tmp);
-    h->launches++;
-    double *old = arr;
-    arr = tmp;
-    tmp = old;
+  Reorder r{};
+  int arrays = 0;
+  auto move = [&](double *&arr, double *&free_one) {
+    r.src[arrays] = arr;
+    r.dst[arrays++] = free_one;
+    double *t = arr;
+    arr = free_one;
+    free_one = t;
   };
-  for (int q = 0; q < 7; ++q) gd(h->s.base[q]);
-  gd(h->s.rhs_t);
-  if (h->s.itp) gd(h->s.itp);
-  for (int d = 0; d < 3; ++d) gd(h->s.frac_prev[d]);
-  h->perm_tmp = tmp;
-  PSTEP_LAUNCHED(h);
-  h->launches--;
-  int32_t *itmp = (int32_t *)h->perm_tmp;
-  // int arrays through the same scratch (as int32), copied back
-  k_gather<int32_t><<<bl, kThreads, 0, h->stream>>>(h->s.flag, idx, n, itmp);
-  PSTEP_LAUNCHED(h);
-  PSTEP_CUDA(cudaMemcpyAsync(h->s.flag, itmp, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
-  k_gather<uint32_t><<<bl, kThreads, 0, h->stream>>>(h->s.key_prev, idx, n, (uint32_t *)itmp);
-  PSTEP_LAUNCHED(h);
-  PSTEP_CUDA(cudaMemcpyAsync(h->s.key_prev, itmp, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
+  for (int q = 0; q < 7; ++q) move(h->s.base[q], h->s.np1[q]);
+  move(h->s.rhs_t, h->s.snew[0]);
+  if (h->s.itp) move(h->s.itp, h->s.snew[1]);
+  for (int d = 0; d < 3; ++d) move(h->s.frac_prev[d], h->s.frac_new[d]);
+  r.flag = h->s.flag;
+  r.flag_to = h->csr_new.sidx;
+  h->csr_new.sidx = h->s.flag;
+  h->s.flag = r.flag_to;
+  r.key = h->s.key_prev;
+  r.key_to = h->s.key_new;
+  h->s.key_new = h->s.key_prev;
+  h->s.key_prev = r.key_to;
   if (h->cfg.flags & PSTEP_TRACK_ORDER) {
-    k_gather<int32_t><<<bl, kThreads, 0, h->stream>>>(h->ref_of_phys, idx, n, itmp);
-    PSTEP_LAUNCHED(h);
-    PSTEP_CUDA(cudaMemcpyAsync(h->ref_of_phys, itmp, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, h->stream));
-    k_invert<<<bl, kThreads, 0, h->stream>>>(h->ref_of_phys, n, h->phys_of_ref);
-    PSTEP_LAUNCHED(h);
+    r.ref = h->ref_of_phys;
+    r.ref_to = h->ref_spare;
+    r.phys_of_ref = h->phys_of_ref;
+    h->ref_of_phys = r.ref_to;
+    h->ref_spare = (int32_t *)r.ref;
   }
+  k_reorder<<<blocks_for(n), kThreads, 0, h->stream>>>(r, arrays, h->csr_prev.sidx, n);
+  PSTEP_LAUNCHED(h);
   h->csr_prev.identity = 1;
   return PSTEP_OK;
 }
