@@ -79,7 +79,6 @@ struct Work {
   uint32_t *mid;         // [brick row (z, y)][kRows][cells along x]
   uint32_t *side;        // [brick][kSideWords]: x = -1, x = 8 (kRows each), x = 9 (RHS_RU x's rows)
   long long *extra;      // [5][cells in brick order]: what does not fit a tile's 32-bit words, exact
-  int32_t *zero;         // a zero
   int nb;                // bricks
   int64_t ncell;
   int64_t slice_cap;     // most slices
@@ -811,6 +810,14 @@ __global__ void __launch_bounds__(kBoundSlots) k_dep_begin(F32Form f, int do_int
   if (t == 32) f.work.counts[2] = 0;
 }
 
+// q * 2^-se, exact: 2^52 + 2^31 + q from its digits, times 2^-se less the offset in one operation
+__device__ __forceinline__ double small_to_f64(int32_t q, int se) {
+  const int scale = (1023 - se) << 20;  // 2^-se's high word
+  const double x = __hiloint2double(0x43300000, (int)((uint32_t)q ^ 0x80000000u));
+  return fma(x, __hiloint2double(scale, 0),
+             __hiloint2double((int)((uint32_t)(scale + (52 << 20)) | 0x80000000u), (int)0x80000000u));
+}
+
 // exact conversion of a scaled 64-bit integer sum q * 2^-se to fp64 with integer operations
 __device__ inline double fixed_to_f64(long long q, int se) {
   if (q == 0) return 0.0;
@@ -1159,213 +1166,198 @@ __global__ void __launch_bounds__(kDepThreads, 4)
 // The deposit, second half: every cell's exact sums from the tiles that reach it -- its own brick's
 // and, on a brick's boundary layers, its neighbours' -- and the 64-bit extras where the brick
 // has any this launch, converted to fp64 and written to the cell and its periodic ghost images.
-// A warp takes 32 cells of a row: the own tiles' rows and those of the y and z neighbours (the
-// same branches for the warp) are read as 128-byte lines, the x neighbours' words by the end
-// lanes of each brick. The launch's exact field statistics are gathered on the way; the last
-// block to finish turns them into the balance sums (momentum components, interior mean of
-// RHS_Part_Temp, grid.cpp:541) and, with EXT, the fields' maxima and minima. Bound: loads (ten a
-// row, 1.9 times over for the neighbours' rows) and issue; 512^3: 4.2 ms, about 12 GB.
-template <int FIELDS, bool EXT>
-__global__ void __launch_bounds__(256, 4) k_dep_gather(Geom G, F32Form f, int32_t epoch, int zsplit,
-                                                                 double inv_cells,
-                                                                 double *__restrict__ outC, double *__restrict__ outX,
-                                                                 double *__restrict__ outY, double *__restrict__ outZ,
-                                                                 double *__restrict__ outE, double *__restrict__ mom,
-                                                                 double *__restrict__ emean) {
+// A block takes one field (blockIdx.y: RHS_Part_Temp, C, RHS_RU x, y, z; the ones from `sums` on are
+// zero, RHS_RU without TWC, grid.cpp:671); a warp takes 32 cells along x of a layer's eight rows in
+// a brick row: of every tile that reaches them ten rows (eleven of RHS_RU y) lie one behind the other, so
+// their words are in flight together, as 128-byte lines, and the x neighbours' words from the end lanes of
+// each brick. The launch's exact field statistics are gathered on the way; the last block to finish
+// turns them into the balance sums (momentum components, interior mean of RHS_Part_Temp,
+// grid.cpp:541) and, with EXT, the fields' maxima and minima. Bound: latency of the loads and memory
+// (12 GB at 512^3). A warp with one row of all fields at a time had ten words in flight and decided
+// about the neighbours row by row: 512^3 4.2 ms (6.1 with the extremes), 256^3 0.47 (0.70); this
+// way 3.0 and 0.33, with or without.
+template <bool EXT>
+__global__ void __launch_bounds__(256, 4) k_dep_gather(Geom G, F32Form f, int32_t epoch, int sums, double inv_cells,
+                                                       double *__restrict__ outC, double *__restrict__ outX,
+                                                       double *__restrict__ outY, double *__restrict__ outZ,
+                                                       double *__restrict__ outE, double *__restrict__ mom,
+                                                       double *__restrict__ emean) {
   const Work &w = f.work;
-  constexpr int NF = FIELDS ? 5 : 1;                              // fields written: E, C, RHS_RU x, y, z
-  constexpr int NS = FIELDS == 0 ? 1 : (FIELDS == 1 ? 2 : 5);     // and of those with sums
+  const int fq = blockIdx.y, fld = fq == 0 ? 4 : fq - 1;
+  double *__restrict__ out = fq == 0 ? outE : (fq == 1 ? outC : (fq == 2 ? outX : (fq == 3 ? outY : outZ)));
   const int nbx = G.n[0] / kBr, nby = G.n[1] / kBr, nbz = G.n[2] / kBr;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nx = (G.n[0] + 31) / 32, n0 = G.n[0], per = kBr / zsplit, tasks = nx * nby * nbz * zsplit;
-  const int64_t ncell = w.ncell;
-  int se[NS];
-#pragma unroll
-  for (int q = 0; q < NS; ++q) se[q] = f.se[q == 0 ? 4 : q - 1];
-  // Running sums, maxima and minima. The extremes of sums inside (-2^31, 2^31 - 1), nearly all, are
-  // kept in 32 bits (INT_MIN, INT_MAX: none yet), the others' in shared memory: ten 64-bit
-  // running values a thread halved the loads in flight (9.7 against 4.1 ms without extremes at
-  // 512^3; this way 6.1 ms).
-  __shared__ long long wide[NS][2];
-  long long tot[NS];
-  int32_t vmax[NS], vmin[NS];
-#pragma unroll
-  for (int q = 0; q < NS; ++q) {
-    tot[q] = 0;
-    vmax[q] = INT_MIN;
-    vmin[q] = INT_MAX;
-  }
+  const int n0 = G.n[0], nx = (n0 + 31) / 32;
+  // the running sum, maximum and minimum; the extremes in 32 bits (INT_MIN, INT_MAX: none yet) while
+  // a warp's sums are inside them, else in shared memory
+  __shared__ long long wide[2];
+  long long tot = 0;
+  int32_t vmax = INT_MIN, vmin = INT_MAX;
   if (EXT) {
-    if (threadIdx.x < NS) {
-      wide[threadIdx.x][0] = LLONG_MIN;
-      wide[threadIdx.x][1] = LLONG_MAX;
+    if (threadIdx.x == 0) {
+      wide[0] = LLONG_MIN;
+      wide[1] = LLONG_MAX;
     }
     __syncthreads();
   }
-  const int32_t *__restrict__ mid = reinterpret_cast<const int32_t *>(w.mid);
-  const int32_t *__restrict__ side = reinterpret_cast<const int32_t *>(w.side);
-  for (int task = blockIdx.x; task < tasks; task += gridDim.x) {
-    const int xb = task % nx, by = (task / nx) % nby, zs = task / (nx * nby), bz = zs / zsplit;
-    const int lz0 = (zs % zsplit) * per;
-    const int i = xb * 32 + lane;
-    if (i >= n0) continue;
-    const int bx = i / kBr, lx = i % kBr;
-    // Besides the cell's own brick, in each dimension, the neighbour whose tile reaches it: cell 0
-    // takes the lower brick's coordinate 8, cell 1 its 9 (the faces along that dimension alone),
-    // cell 7 the upper brick's -1. Along x: words of the side array, or a zero
-    const bool ex = lx == 0 || lx == kBr - 1, fx = ex || lx == 1;
-    const int ox = lx <= 1 ? (bx == 0 ? nbx - 1 : bx - 1) : (bx == nbx - 1 ? 0 : bx + 1);
-    const int at = lx == 0 ? kRows : (lx == 1 ? 2 * kRows - kRowX : 0);
-    const int yl = by == 0 ? nby - 1 : by - 1, yh = by == nby - 1 ? 0 : by + 1;
-    const int zl = bz == 0 ? nbz - 1 : bz - 1, zh = bz == nbz - 1 ? 0 : bz + 1;
-    const int own = (bz * nby + by) * nbx + bx;
-    const bool extras = w.extra_epoch[own] == epoch;
-    const int i2 = i == 0 ? n0 + 1 : (i == n0 - 1 ? 0 : -1);
-#pragma unroll 1
-    for (int lz = lz0; lz < lz0 + per; ++lz) {
-    // (the rows turn over the warps: those on the brick's boundary layers take longer)
-    const int ly = (wid + lz) % kBr, j = by * kBr + ly, k = bz * kBr + lz;
-    const bool hy = ly <= 1 || ly == kBr - 1, hz = lz <= 1 || lz == kBr - 1, ay = ly == 1, az = lz == 1;
-    const int oy = ly <= 1 ? yl : yh, oz = lz <= 1 ? zl : zh;
-    const int dy = ly <= 1 ? kBr + 1 + ly : 0, dz = lz <= 1 ? kBr + 1 + lz : 0;
-    long long v[NF];
+  if (fq >= sums) {
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < G.gsize; t += (int64_t)gridDim.x * blockDim.x)
+      out[t] = 0.0;
+  } else {
+    const int se = f.se[fld];
+    const int first = fq < 2 ? fq * kRowC : (fq == 2 ? kRowX : (fq == 3 ? kRowY : kRowZ));
+    const int layer_rows = fq == 3 ? kTE + 1 : kTE;
+    const int32_t *__restrict__ mid = reinterpret_cast<const int32_t *>(w.mid);
+    const int32_t *__restrict__ side = reinterpret_cast<const int32_t *>(w.side);
+    const int tasks = nx * nby * nbz;
+    for (int task = blockIdx.x; task < tasks; task += gridDim.x) {
+      const int xb = task % nx, row = task / nx, by = row % nby, bz = row / nby;
+      const int lz = (wid + task) % kBr;  // (the layers turn over the warps: the outer ones take longer)
+      const bool live = xb * 32 + lane < n0;
+      const int i = live ? xb * 32 + lane : n0 - 1;
+      const int bx = i / kBr, lx = i % kBr;
+      // Besides the cell's own brick, in each dimension, the neighbour whose tile reaches it: cell 0
+      // takes the lower brick's coordinate 8, cell 1 its 9 (the faces along that dimension alone),
+      // cell 7 the upper brick's -1. Along x: words of the side array
+      const bool end = lx == 0 || lx == kBr - 1 || (lx == 1 && fq == 2);
+      const int ox = lx <= 1 ? (bx == 0 ? nbx - 1 : bx - 1) : (bx == nbx - 1 ? 0 : bx + 1);
+      const int at = lx == 0 ? kRows : (lx == 1 ? 2 * kRows - kRowX : 0);
+      const int yl = by == 0 ? nby - 1 : by - 1, yh = by == nby - 1 ? 0 : by + 1;
+      long long v[kBr];
 #pragma unroll
-    for (int q = 0; q < NF; ++q) v[q] = 0;
-    // row (cy, cz) of the tiles of brick row (ty, tz); it may be reached by the faces along y (ny)
-    // or z (nz) alone
-    auto row = [&](int ty, int tz, int cy, int cz, bool ny, bool nz) {
-      const int brow = tz * nby + ty;
-      const int32_t *m = mid + (int64_t)brow * (kRows * n0) + i;
-      const int32_t *sd = side + ((int64_t)brow * nbx + ox) * kSideWords + at;
-      const int32_t *se_ = ex ? sd : w.zero, *sf_ = fx ? sd : w.zero;
-      const int te = ex ? 1 : 0, tf = fx ? 1 : 0;
-      const int re = cz * kTE + cy, rv = kRowY + cz * (kTE + 1) + cy;
-      int32_t p[NS], q[NS];
+      for (int r = 0; r < kBr; ++r) v[r] = 0;
+      // adds layer cz (z + 1) of the tiles of brick row (., tz) and its y neighbours
+      auto layer = [&](int tz, int cz) {
+        const int at_row = first + cz * layer_rows;
+        auto words = [&](int ty, int cy, const int32_t *&m, const int32_t *&sd) {
+          const int64_t brow = (int64_t)tz * nby + ty;
+          m = mid + (brow * kRows + at_row + cy) * n0 + i;
+          sd = side + (brow * nbx + ox) * kSideWords + at + at_row + cy;
+        };
+        const int32_t *m, *sd, *ml, *sl, *mh, *sh;
+        words(by, 1, m, sd);
+        words(yl, kBr + 1, ml, sl);
+        words(yh, 0, mh, sh);
+        // of each row a word, and the end lanes' side word: the eight rows, y = 8 and 9 of the lower
+        // brick's tile, y = -1 of the upper's
+        constexpr int R = kBr + 3;
+        int32_t p[R], q[R];
 #pragma unroll
-      for (int u = 0; u < NS; ++u) p[u] = q[u] = 0;
-      if (!ny && !nz) {
-        p[0] = m[re * n0];
-        q[0] = se_[re * te];
-        if (FIELDS) {
-          p[1] = m[(kRowC + re) * n0];
-          q[1] = se_[(kRowC + re) * te];
+        for (int r = 0; r < kBr; ++r) p[r] = m[(int64_t)r * n0];
+        p[kBr] = ml[0];
+        p[kBr + 1] = fq == 3 ? ml[n0] : 0;
+        p[kBr + 2] = mh[0];
+#pragma unroll
+        for (int r = 0; r < R; ++r) q[r] = 0;
+        if (end) {
+#pragma unroll
+          for (int r = 0; r < kBr; ++r) q[r] = sd[r];
+          q[kBr] = sl[0];
+          if (fq == 3) q[kBr + 1] = sl[1];
+          q[kBr + 2] = sh[0];
         }
-        if (FIELDS == 2) {
-          p[NS - 3] = m[(kRowX + re) * n0];
-          q[NS - 3] = sf_[(kRowX + re) * tf];
-        }
-      }
-      if (FIELDS == 2 && !nz) {
-        p[NS - 2] = m[rv * n0];
-        q[NS - 2] = se_[rv * te];
-      }
-      if (FIELDS == 2 && !ny) {
-        p[NS - 1] = m[(kRowZ + re) * n0];
-        q[NS - 1] = se_[(kRowZ + re) * te];
-      }
 #pragma unroll
-      for (int u = 0; u < NS; ++u) v[u] += (long long)p[u] + (long long)q[u];
-    };
-    row(by, bz, ly + 1, lz + 1, false, false);
-    if (hy && (FIELDS == 2 || !ay)) row(oy, bz, dy, lz + 1, ay, false);
-    if (hz && (FIELDS == 2 || !az)) row(by, oz, ly + 1, dz, false, az);
-    if (hy && hz && !(ay && az) && (FIELDS == 2 || !(ay || az))) row(oy, oz, dy, dz, ay, az);
-    if (extras) {
-      long long *x = w.extra + (int64_t)own * kBrickCells + (lz * kBr + ly) * kBr + lx;
-      long long e[NS];
+        for (int r = 0; r < R; ++r)
+          v[r < kBr ? r : (r == kBr + 2 ? kBr - 1 : r - kBr)] += (long long)p[r] + (long long)q[r];
+      };
+      layer(bz, lz + 1);
+      if (lz == 0 || (lz == 1 && fq == 4)) layer(bz == 0 ? nbz - 1 : bz - 1, kBr + 1 + lz);
+      if (lz == kBr - 1) layer(bz == nbz - 1 ? 0 : bz + 1, 0);
+      const int own = (bz * nby + by) * nbx + bx;
+      if (live && w.extra_epoch[own] == epoch) {
+        long long *x = w.extra + fld * w.ncell + (int64_t)own * kBrickCells + lz * kBr * kBr + lx;
+        long long e[kBr];
 #pragma unroll
-      for (int q = 0; q < NS; ++q) e[q] = x[(q == 0 ? 4 : q - 1) * ncell];
+        for (int r = 0; r < kBr; ++r) e[r] = x[r * kBr];
 #pragma unroll
-      for (int q = 0; q < NS; ++q) {
-        v[q] += e[q];
-        if (e[q]) x[(q == 0 ? 4 : q - 1) * ncell] = 0;  // ready for the next launch
-      }
-    }
-    const long long g = glin3(G, i + 1, j + 1, k + 1);
-    const int j2 = j == 0 ? G.n[1] + 1 : (j == G.n[1] - 1 ? 0 : -1),
-              k2 = k == 0 ? G.n[2] + 1 : (k == G.n[2] - 1 ? 0 : -1);
-    double o[NF];
-#pragma unroll
-    for (int q = 0; q < NF; ++q) {
-      o[q] = q < NS ? fixed_to_f64(v[q], se[q < NS ? q : 0]) : 0.0;  // RHS_RU = 0 without TWC (grid.cpp:671)
-      double *out = q == 0 ? outE : (q == 1 ? outC : (q == 2 ? outX : (q == 3 ? outY : outZ)));
-      out[g] = o[q];
-    }
-    if (i2 >= 0 || j2 >= 0 || k2 >= 0) {
-#pragma unroll 1
-      for (int s = 1; s < 8; ++s) {
-        const int ii = (s & 1) ? i2 : i + 1, jj = (s & 2) ? j2 : j + 1, kk = (s & 4) ? k2 : k + 1;
-        if (ii < 0 || jj < 0 || kk < 0) continue;
-        const long long gi = glin3(G, ii, jj, kk);
-#pragma unroll
-        for (int q = 0; q < NF; ++q) {
-          double *out = q == 0 ? outE : (q == 1 ? outC : (q == 2 ? outX : (q == 3 ? outY : outZ)));
-          out[gi] = o[q];
+        for (int r = 0; r < kBr; ++r) {
+          v[r] += e[r];
+          if (e[r]) x[r * kBr] = 0;  // ready for the next launch
         }
       }
-    }
+      if (!live) continue;
+      // the cell and its periodic images: along x the end cells of a row have one, along y and z whole
+      // rows do
+      const int j = by * kBr, k = bz * kBr + lz;
+      double *to = out + glin3(G, i + 1, j + 1, k + 1);
+      const int img_x = i == 0 ? n0 : (i == n0 - 1 ? -n0 : 0);
+      const long long plane = (long long)G.g[0] * G.g[1],
+                      img_z = k == 0 ? G.n[2] * plane : (k == G.n[2] - 1 ? -G.n[2] * plane : 0);
+      auto put = [&](int r, double o) {
+        double *c = to + (long long)r * G.g[0];
+        auto along_x = [&](double *a) {
+          *a = o;
+          if (img_x) a[img_x] = o;
+        };
+        along_x(c);
+        if (img_z) along_x(c + img_z);
+        if (j + r == 0 || j + r == G.n[1] - 1) {
+          double *y = c + (j + r == 0 ? G.n[1] : -G.n[1]) * (long long)G.g[0];
+          along_x(y);
+          if (img_z) along_x(y + img_z);
+        }
+        tot += v[r];
+      };
+      bool small = true;
 #pragma unroll
-    for (int q = 0; q < NF; ++q) {
-      if (q < NS) {
-        tot[q] += v[q];
-        if (EXT) {
-          if (v[q] > (long long)INT_MIN && v[q] < (long long)INT_MAX) {
-            vmax[q] = max(vmax[q], (int32_t)v[q]);
-            vmin[q] = min(vmin[q], (int32_t)v[q]);
-          } else {
-            atomicMax(&wide[q][0], v[q]);
-            atomicMin(&wide[q][1], v[q]);
+      for (int r = 0; r < kBr; ++r) small &= v[r] == (long long)(int)v[r] && (!EXT || (v[r] != INT_MIN && v[r] != INT_MAX));
+      if (small) {
+#pragma unroll
+        for (int r = 0; r < kBr; ++r) {
+          put(r, small_to_f64((int)v[r], se));
+          if (EXT) {
+            vmax = max(vmax, (int)v[r]);
+            vmin = min(vmin, (int)v[r]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < kBr; ++r) {
+          put(r, fixed_to_f64(v[r], se));
+          if (EXT) {
+            atomicMax(&wide[0], v[r]);
+            atomicMin(&wide[1], v[r]);
           }
         }
       }
     }
-    }
   }
-  __shared__ long long red[8][NS][3];
+  __shared__ long long red[8][3];
   __shared__ int last;
-#pragma unroll
-  for (int q = 0; q < NS; ++q) {
-    const long long sm = warp_sum_i64(tot[q]);
-    if (lane == 0) red[wid][q][0] = sm;
-    if (EXT) {
-      const int32_t mx = __reduce_max_sync(0xffffffffu, vmax[q]), mn = __reduce_min_sync(0xffffffffu, vmin[q]);
-      if (lane == 0) {
-        red[wid][q][1] = mx;
-        red[wid][q][2] = mn;
-      }
-    }
+  const long long sm = warp_sum_i64(tot);
+  const int32_t mx = __reduce_max_sync(0xffffffffu, vmax), mn = __reduce_min_sync(0xffffffffu, vmin);
+  if (lane == 0) {
+    red[wid][0] = sm;
+    red[wid][1] = mx;
+    red[wid][2] = mn;
   }
   __syncthreads();
-  if (threadIdx.x < NF) {
-    const int q = threadIdx.x, fld = q == 0 ? 4 : q - 1;
-    long long sm = 0, mx = q < NS ? LLONG_MIN : 0, mn = q < NS ? LLONG_MAX : 0;
-    if (q < NS) {
-      for (int u = 0; u < 8; ++u) {
-        sm += red[u][q][0];
-        if (EXT) {
-          if (red[u][q][1] > (long long)INT_MIN) mx = max(mx, red[u][q][1]);
-          if (red[u][q][2] < (long long)INT_MAX) mn = min(mn, red[u][q][2]);
-        }
-      }
+  if (threadIdx.x == 0) {
+    long long all = 0, high = fq < sums ? LLONG_MIN : 0, low = fq < sums ? LLONG_MAX : 0;
+    for (int u = 0; u < 8; ++u) {
+      all += red[u][0];
       if (EXT) {
-        mx = max(mx, wide[q][0]);
-        mn = min(mn, wide[q][1]);
+        if (red[u][1] > (long long)INT_MIN) high = max(high, red[u][1]);
+        if (red[u][2] < (long long)INT_MAX) low = min(low, red[u][2]);
       }
     }
-    if (sm) atomicAdd(&f.totals[fld], (unsigned long long)sm);
+    if (all) atomicAdd(&f.totals[fld], (unsigned long long)all);
     if (EXT) {
-      atomicMax(reinterpret_cast<long long *>(&f.totals[5 + fld]), mx);
-      atomicMin(reinterpret_cast<long long *>(&f.totals[10 + fld]), mn);
+      if (fq < sums) {
+        high = max(high, wide[0]);
+        low = min(low, wide[1]);
+      }
+      atomicMax(reinterpret_cast<long long *>(&f.totals[5 + fld]), high);
+      atomicMin(reinterpret_cast<long long *>(&f.totals[10 + fld]), low);
     }
     __threadfence();
+    last = atomicAdd(f.done, 1) == (int)(gridDim.x * gridDim.y) - 1;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(f.done, 1) == (int)gridDim.x - 1;
   __syncthreads();
   if (!last) return;
   if (threadIdx.x == 0) *f.done = 0;
   __threadfence();
-  if (threadIdx.x < NF) {
+  if (threadIdx.x < gridDim.y) {
     const int fld = threadIdx.x == 0 ? 4 : threadIdx.x - 1, e = f.se[fld];
     const long long sm = (long long)__ldcg(&f.totals[fld]);
     if (EXT) {  // integer order is the fp64 order at one scale
@@ -1751,8 +1743,6 @@ int f32_create(pstep_ctx *h) {
     TRY32(dalloc32(h, w.mid, mid));
     TRY32(dalloc32(h, w.side, sides));
     TRY32(dalloc32(h, w.extra, 5 * ncell));
-    TRY32(dalloc32(h, w.zero, 1));
-    PSTEP_CUDA(cudaMemsetAsync(w.zero, 0, sizeof(int32_t), h->stream));
     PSTEP_CUDA(cudaMemsetAsync(w.counts, 0, 4 * sizeof(int32_t), h->stream));
     PSTEP_CUDA(cudaMemsetAsync(w.extra_epoch, 0, sizeof(int32_t) * w.nb, h->stream));
     PSTEP_CUDA(cudaMemsetAsync(w.dirty, 0, w.nb, h->stream));
@@ -1795,7 +1785,7 @@ int f32_destroy(pstep_ctx *h) {
   {
     Work &w = f->work;
     dfree32(w.items); dfree32(w.counts); dfree32(w.dirty); dfree32(w.extra_epoch);
-    dfree32(w.mid); dfree32(w.side); dfree32(w.extra); dfree32(w.zero);
+    dfree32(w.mid); dfree32(w.side); dfree32(w.extra);
   }
   if (f->stage[0]) {
     cudaStreamSynchronize(f->copy_stream);
@@ -2136,16 +2126,11 @@ int dep_launch(pstep_ctx *h, bool do_int, Set32 SI, Set32 SN, bool ext) {
   if (fields == 2) f.whole_since = 1;
   double *C = h->dep[PSTEP_FIELD_C], *X = h->dep[PSTEP_FIELD_RU_X], *Y = h->dep[PSTEP_FIELD_RU_Y],
          *Z = h->dep[PSTEP_FIELD_RU_Z], *E = h->dep[PSTEP_FIELD_PART_TEMP];
-  auto gather = fields == 2 ? (ext ? k_dep_gather<2, true> : k_dep_gather<2, false>)
-                            : (fields == 1 ? (ext ? k_dep_gather<1, true> : k_dep_gather<1, false>)
-                                           : (ext ? k_dep_gather<0, true> : k_dep_gather<0, false>));
-  // a task is a brick row's 32 cells; cut along z while there are fewer than the CTAs that fit
   const int64_t tasks = (int64_t)((G.n[0] + 31) / 32) * (G.n[1] / kBr) * (G.n[2] / kBr), fit = 4 * (int64_t)h->num_sms;
-  int zsplit = 1;
-  while (zsplit < kBr && tasks * zsplit < 2 * fit) zsplit *= 2;
-  const unsigned grid_g = (unsigned)(tasks * zsplit < fit ? tasks * zsplit : fit);
-  gather<<<grid_g, 256, 0, h->stream>>>(G, f, epoch, zsplit, 1.0 / ((double)G.n[0] * G.n[1] * G.n[2]), C, X, Y, Z, E,
-                                        h->mom_dev, h->emean_dev);
+  auto gather = ext ? k_dep_gather<true> : k_dep_gather<false>;
+  gather<<<dim3((unsigned)(tasks < fit ? tasks : fit), fields ? 5 : 1), 256, 0, h->stream>>>(
+      G, f, epoch, fields == 2 ? 5 : fields + 1, 1.0 / ((double)G.n[0] * G.n[1] * G.n[2]), C, X, Y, Z, E, h->mom_dev,
+      h->emean_dev);
   PSTEP_LAUNCHED(h);
   for (int q = 0; q < 5; ++q)
     if (do_int || q == 4) f.ext_ok[q] = ext ? 1 : 0;
