@@ -155,29 +155,20 @@ __device__ inline void renorm(int &i, float &o, int n) {
 
 __device__ inline long long glin3(const Geom &G, int i, int j, int k) { return glin(G, i, j, k); }
 
-__device__ inline void atomic_max_abs(uint32_t *w, float v) {
-  // non-negative floats order like their bit patterns
-  atomicMax(w, __float_as_uint(fabsf(v)));
+// the warp's maxima of 4 non-negative values, which order like their bit patterns (and are numbers: a
+// maximum with 0 has dropped what is not), into one of the kBoundSlots (whole warps call; a block's
+// maximum behind a barrier took 5% of the advance kernels)
+__device__ __forceinline__ uint32_t warp_slot() {
+  return (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) % kBoundSlots;
 }
-
-// block maximum of 4 non-negative values into slot blockIdx % kBoundSlots
-__device__ inline void block_max4(uint32_t *slots, float a0, float a1, float a2, float a3) {
-  __shared__ float red[4][32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a0 = fmaxf(a0, __shfl_xor_sync(0xffffffffu, a0, o));
-    a1 = fmaxf(a1, __shfl_xor_sync(0xffffffffu, a1, o));
-    a2 = fmaxf(a2, __shfl_xor_sync(0xffffffffu, a2, o));
-    a3 = fmaxf(a3, __shfl_xor_sync(0xffffffffu, a3, o));
-  }
-  const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  if ((threadIdx.x & 31) == 0) { red[0][w] = a0; red[1][w] = a1; red[2][w] = a2; red[3][w] = a3; }
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    float m = 0.f;
-    for (int q = 0; q < nw; ++q) m = fmaxf(m, red[threadIdx.x][q]);
-    atomic_max_abs(&slots[(blockIdx.x % kBoundSlots) * 4 + threadIdx.x], m);
-  }
+__device__ __forceinline__ void warp_max4(uint32_t *slots, float a0, float a1, float a2, float a3) {
+  const uint32_t m0 = __reduce_max_sync(0xffffffffu, __float_as_uint(a0)),
+                 m1 = __reduce_max_sync(0xffffffffu, __float_as_uint(a1)),
+                 m2 = __reduce_max_sync(0xffffffffu, __float_as_uint(a2)),
+                 m3 = __reduce_max_sync(0xffffffffu, __float_as_uint(a3));
+  const int lane = threadIdx.x & 31;
+  const uint32_t m = lane == 0 ? m0 : (lane == 1 ? m1 : (lane == 2 ? m2 : m3));
+  if (lane < 4 && m) atomicMax(&slots[warp_slot() * 4 + lane], m);
 }
 
 // order-preserving 32-bit key of a float (larger float, larger key; 0 is below every key)
@@ -186,23 +177,13 @@ __device__ __forceinline__ uint32_t order_key(float v) {
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
-// block maximum of 2 signed values into slot blockIdx % kBoundSlots as order keys (a block
-// with no particle leaves its slots alone)
-__device__ inline void block_max2_signed(uint32_t *slots, float a0, float a1) {
-  __shared__ float red2[2][32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a0 = fmaxf(a0, __shfl_xor_sync(0xffffffffu, a0, o));
-    a1 = fmaxf(a1, __shfl_xor_sync(0xffffffffu, a1, o));
-  }
-  const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  if ((threadIdx.x & 31) == 0) { red2[0][w] = a0; red2[1][w] = a1; }
-  __syncthreads();
-  if (threadIdx.x < 2) {
-    float m = -INFINITY;
-    for (int q = 0; q < nw; ++q) m = fmaxf(m, red2[threadIdx.x][q]);
-    if (m > -INFINITY) atomicMax(&slots[(blockIdx.x % kBoundSlots) * 2 + threadIdx.x], order_key(m));
-  }
+// the same of 2 signed values as order keys (-infinity, or not a number: none)
+__device__ __forceinline__ void warp_max2_signed(uint32_t *slots, float a0, float a1) {
+  const uint32_t m0 = __reduce_max_sync(0xffffffffu, a0 > -INFINITY ? order_key(a0) : 0u),
+                 m1 = __reduce_max_sync(0xffffffffu, a1 > -INFINITY ? order_key(a1) : 0u);
+  const int lane = threadIdx.x & 31;
+  const uint32_t m = lane == 0 ? m0 : m1;
+  if (lane < 2 && m) atomicMax(&slots[warp_slot() * 2 + lane], m);
 }
 
 struct C32 {
@@ -383,8 +364,14 @@ __device__ __forceinline__ float adv_finish_mlp(const Geom &G, const F32Form &f,
   return adv_finish_t<K>(G, f, c, twc, p, a, ty, td_prev, err, mu0, mu1, mu2, mt);
 }
 
+// Bound by memory latency: a particle's 180 bytes a stage and the field values behind its cell are two
+// trips, so what counts is the warps in flight. 256 threads a block at 78 and 105 registers (stages
+// 0, 3 and 1, 2) and a block's maxima behind a barrier: 495, 704, 704, 586 us at 256^3 x 2^24; blocks of
+// 128, nine on an SM (56 registers; stage 3, which reads less, six), maxima by warp:
+// 440, 625, 625, 526 us (eight an SM 453, 625, 623, 568; six 517, 677, 676, 535).
+constexpr int kAdvThreads = 128;
 template <int K>
-__global__ void __launch_bounds__(256) k_advance32(Geom G, F32Form f, C32 c, int twc, int64_t n,
+__global__ void __launch_bounds__(kAdvThreads, K == 3 ? 6 : 9) k_advance32(Geom G, F32Form f, C32 c, int twc, int64_t n,
                                                    int32_t *__restrict__ err) {
   int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   float mu0 = 0.f, mu1 = 0.f, mu2 = 0.f, mt = 0.f, umax = -INFINITY, gmax = -INFINITY;
@@ -396,9 +383,9 @@ __global__ void __launch_bounds__(256) k_advance32(Geom G, F32Form f, C32 c, int
     gmax = a.gas[0];
   }
   // bounds for the fixed-point scales (order-independent maxima)
-  block_max4(f.slots, mu0, mu1, mu2, mt);
+  warp_max4(f.slots, mu0, mu1, mu2, mt);
   // the last stage: max u of the step's result and max ug (grid.cpp:726-727)
-  if (K == 3) block_max2_signed(f.pslots, umax, gmax);
+  if (K == 3) warp_max2_signed(f.pslots, umax, gmax);
 }
 
 // ----------------------------------------------------------------------------
@@ -720,8 +707,9 @@ __global__ void __launch_bounds__(corr::kThreads, 4) k_corr_net(Geom G, F32Form 
 
 // every stage with the correction: the kept network output, applied with this stage's
 // drive slip and prior
+constexpr int kCorrThreads = 128;  // (256^3 x 2^24, a stage: 256 x 5 an SM 664 us, 128 x 8, 9, 10: 676, 616, 656)
 template <int K>
-__global__ void __launch_bounds__(256, 5) k_advance32_corr(Geom G, F32Form f, C32 c, int twc, int64_t n,
+__global__ void __launch_bounds__(kCorrThreads, 9) k_advance32_corr(Geom G, F32Form f, C32 c, int twc, int64_t n,
                                                         int32_t *__restrict__ err, CorrDev cd) {
   int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   float mu0 = 0.f, mu1 = 0.f, mu2 = 0.f, mt = 0.f, umax = -INFINITY, gmax = -INFINITY;
@@ -750,8 +738,8 @@ __global__ void __launch_bounds__(256, 5) k_advance32_corr(Geom G, F32Form f, C3
     umax = a.vac[0];
     gmax = a.gas[0];
   }
-  block_max4(f.slots, mu0, mu1, mu2, mt);
-  if (K == 3) block_max2_signed(f.pslots, umax, gmax);
+  warp_max4(f.slots, mu0, mu1, mu2, mt);
+  if (K == 3) warp_max2_signed(f.pslots, umax, gmax);
 }
 
 // the prime (grid.cpp:223-226) at the base positions: Tg, RHS_T
@@ -775,7 +763,7 @@ __global__ void k_prime32(Geom G, F32Form f, float itth, int64_t n) {
     mt = (tg - B.v[3][p]) * (f.pp[PP_ITTH] ? f.pp[PP_ITTH][p] : itth);
     f.rhs_t[p] = mt;
   }
-  block_max4(f.slots, 0.f, 0.f, 0.f, fabsf(mt));
+  warp_max4(f.slots, 0.f, 0.f, 0.f, fmaxf(0.f, fabsf(mt)));
 }
 
 // Before a deposit: the exponents of the fixed-point scales from the advance's spread maxima (which
@@ -2056,6 +2044,7 @@ int f32_stage(pstep_ctx *h, int k, double pre, double post) {
   F32Form &f = *h->f32;
   const C32 c = make_c32(h, k, pre, post);
   const int64_t n = h->np;
+  const int nb_adv = (int)((n + kAdvThreads - 1) / kAdvThreads), nb_corr = (int)((n + kCorrThreads - 1) / kCorrThreads);
   CorrDev cd = *reinterpret_cast<const CorrDev *>(h->corr_dev);
   cd.wait_limit = h->wait_limit;
   cd.idle_first = h->wait_idle ? 1u : 0u;
@@ -2081,18 +2070,18 @@ int f32_stage(pstep_ctx *h, int k, double pre, double post) {
   prof_begin(h, PSTEP_PHASE_ADVANCE);
   if (n > 0 && h->corr_on) {
     switch (k) {
-      case 0: k_advance32_corr<0><<<nb(n), 256, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word, cd); break;
-      case 1: k_advance32_corr<1><<<nb(n), 256, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word, cd); break;
-      case 2: k_advance32_corr<2><<<nb(n), 256, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word, cd); break;
-      default: k_advance32_corr<3><<<nb(n), 256, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word, cd); break;
+      case 0: k_advance32_corr<0><<<nb_corr, kCorrThreads, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word, cd); break;
+      case 1: k_advance32_corr<1><<<nb_corr, kCorrThreads, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word, cd); break;
+      case 2: k_advance32_corr<2><<<nb_corr, kCorrThreads, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word, cd); break;
+      default: k_advance32_corr<3><<<nb_corr, kCorrThreads, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word, cd); break;
     }
     PSTEP_LAUNCHED(h);
   } else if (n > 0) {
     switch (k) {
-      case 0: k_advance32<0><<<nb(n), 256, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word); break;
-      case 1: k_advance32<1><<<nb(n), 256, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word); break;
-      case 2: k_advance32<2><<<nb(n), 256, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word); break;
-      default: k_advance32<3><<<nb(n), 256, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word); break;
+      case 0: k_advance32<0><<<nb_adv, kAdvThreads, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word); break;
+      case 1: k_advance32<1><<<nb_adv, kAdvThreads, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word); break;
+      case 2: k_advance32<2><<<nb_adv, kAdvThreads, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word); break;
+      default: k_advance32<3><<<nb_adv, kAdvThreads, 0, h->stream>>>(h->geom, f, c, h->cfg.twc, n, h->err_word); break;
     }
     PSTEP_LAUNCHED(h);
   }
