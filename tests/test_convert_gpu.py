@@ -54,3 +54,27 @@ def test_round_trip_is_the_float32_value(built_cuda, count):
     for a, name in zip(all_out, ("x", "y", "z", "u", "v", "w", "T")):
         assert a.tobytes() == g.array(name).tobytes()
     g.close()
+
+
+@pytest.mark.parametrize("n, dx", [(16, 1.0), (256, 0.3), (104, 2.0 * np.pi / 104)])
+def test_downloaded_positions_are_rounded_once_each(built_cuda, n, dx):
+    """(cell + offset) dx with one rounding in the product, over the offsets' whole range: zero, below and at
+    2^-19 (where the sum needs no rounding), random ones and the largest below 1."""
+    rng = np.random.default_rng(n)
+    edge = np.array([0.0, 2.0 ** -30, 2.0 ** -19 * (1 - 2.0 ** -24), 2.0 ** -19, 2.0 ** -18, 0.5, 1 - 2.0 ** -24])
+    o = np.concatenate([edge, 2.0 ** rng.uniform(-21, 0, 500), rng.uniform(0, 1, 500)]).astype(np.float32)
+    o = np.minimum(np.tile(o, 3), np.float32(1 - 2.0 ** -24))
+    cell = np.repeat([0.0, 1.0, n - 1.0], len(o) // 3)
+    count = len(o)
+    length = dx * n
+    g = pstep.ParticleStep(dict(config.box_params(n, count).step_config(), l=length), count, pstep.FP32, 0)
+    x = (cell + o.astype(np.float64)) * dx
+    zero = np.zeros(count)
+    g.load(x, zero, zero, zero, zero, zero, zero + 1.0, np.arange(count, dtype=np.int32))
+    # the cell and fp32 offset the upload made of it, by the host
+    xi = x * (1.0 / (length / n))
+    c = np.floor(xi)
+    f = (xi - c).astype(np.float32)
+    c, f = np.where(f >= 1.0, c + 1, c) % n, np.where(f >= 1.0, np.float32(0), f)
+    assert g.array("x").tobytes() == ((c + f.astype(np.float64)) * (length / n)).tobytes()
+    g.close()
