@@ -13,16 +13,43 @@ namespace {
 constexpr int kScanItems = 16;                       // per thread
 constexpr int kScanTile = kThreads * kScanItems;     // per block
 
+// A run of neighbouring lanes with one key: its first lane, and its length and the lane's place in
+// it. The storage is nearly in key order, so runs collect almost all that a match over the
+// whole warp would; that takes a pass per distinct key, and shuffles over the groups it finds go one
+// group after the other (2^24 particles on 256^3 cells: count 83, scatter 166 us; by runs
+// 55 and 97).
+struct Run {
+  int first, len, place;
+};
+__device__ __forceinline__ Run run_of(uint32_t key) {
+  const int lane = (int)(threadIdx.x & 31);
+  const uint32_t before = __shfl_up_sync(0xffffffffu, key, 1);
+  const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || key != before);
+  Run r;
+  r.first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+  const uint32_t after = heads & ~(0xffffffffu >> (31 - lane));  // heads above the lane
+  r.len = (after ? __ffs(after) - 1 : 32) - r.first;
+  r.place = lane - r.first;
+  return r;
+}
+
 __global__ void k_count(const uint32_t *__restrict__ keys, int shift, int64_t n, int32_t *__restrict__ counts) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  bool valid = i < n;
-  uint32_t node = valid ? (keys[i] >> shift) : 0xffffffffu;
-  // warp-aggregated increments: lanes with the same node add once
-  unsigned active = __ballot_sync(0xffffffffu, valid);
-  if (!valid) return;
-  unsigned peers = __match_any_sync(active, node);
-  int leader = __ffs(peers) - 1;
-  if ((int)(threadIdx.x & 31) == leader) atomicAdd(&counts[node], __popc(peers));
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = i < n;
+  const uint32_t node = valid ? (keys[i] >> shift) : 0xffffffffu;
+  const Run run = run_of(node);
+  if (valid && run.place == 0) atomicAdd(&counts[node], run.len);
+}
+
+// the particle's place among those of its key, from the keys' running positions (n: none)
+__device__ __forceinline__ int32_t place_of(const uint32_t *__restrict__ keys, int shift, int64_t i, int64_t n,
+                                            int32_t *__restrict__ cursor) {
+  const bool valid = i < n;
+  const uint32_t node = valid ? (keys[i] >> shift) : 0xffffffffu;
+  const Run run = run_of(node);
+  int32_t base = 0;
+  if (valid && run.place == 0) base = atomicAdd(&cursor[node], run.len);
+  return __shfl_sync(0xffffffffu, base, run.first) + run.place;
 }
 
 // Exclusive scan in one pass (scan_take, scan_before). Writes out[0..n] (out[n] = total) and out2
@@ -89,19 +116,9 @@ __global__ void __launch_bounds__(kThreads) k_scan(const int32_t *__restrict__ i
 
 __global__ void k_scatter(const uint32_t *__restrict__ keys, int shift, int64_t n, int32_t *__restrict__ cursor,
                           int32_t *__restrict__ sidx) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  bool valid = i < n;
-  uint32_t node = valid ? (keys[i] >> shift) : 0xffffffffu;
-  unsigned active = __ballot_sync(0xffffffffu, valid);
-  if (!valid) return;
-  unsigned peers = __match_any_sync(active, node);
-  int lane = threadIdx.x & 31;
-  int leader = __ffs(peers) - 1;
-  int32_t basepos = 0;
-  if (lane == leader) basepos = atomicAdd(&cursor[node], __popc(peers));
-  basepos = __shfl_sync(peers, basepos, leader);
-  int32_t rank = __popc(peers & ((1u << lane) - 1u));
-  sidx[basepos + rank] = (int32_t)i;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int32_t to = place_of(keys, shift, i, n, cursor);
+  if (i < n) sidx[to] = (int32_t)i;
 }
 
 // The order within a node: 64-bit items (secondary key << 32 | particle), where the secondary
@@ -119,18 +136,8 @@ __global__ void k_scatter_items(const uint32_t *__restrict__ keys, int shift, in
                                 unsigned long long *__restrict__ items, int32_t *__restrict__ big_count) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *big_count = 0;  // k_segrank's list
-  bool valid = i < n;
-  uint32_t node = valid ? (keys[i] >> shift) : 0xffffffffu;
-  unsigned active = __ballot_sync(0xffffffffu, valid);
-  if (!valid) return;
-  unsigned peers = __match_any_sync(active, node);
-  int lane = threadIdx.x & 31;
-  int leader = __ffs(peers) - 1;
-  int32_t basepos = 0;
-  if (lane == leader) basepos = atomicAdd(&cursor[node], __popc(peers));
-  basepos = __shfl_sync(peers, basepos, leader);
-  int32_t rank = __popc(peers & ((1u << lane) - 1u));
-  items[basepos + rank] = seg_item(order, keys, (int32_t)i);
+  const int32_t to = place_of(keys, shift, i, n, cursor);
+  if (i < n) items[to] = seg_item(order, keys, (int32_t)i);
 }
 
 // Segments of up to kRankSeg items: one thread per item counts the smaller items of its segment
