@@ -766,38 +766,6 @@ __global__ void k_prime32(Geom G, F32Form f, float itth, int64_t n) {
   warp_max4(f.slots, 0.f, 0.f, 0.f, fmaxf(0.f, fabsf(mt)));
 }
 
-// Before a deposit: the exponents of the fixed-point scales from the advance's spread maxima (which
-// are cleared for the next stage), the item counter, and the field statistics of the fields
-// this launch writes (sums 0, maxima and minima at the ends of the int64 range). One block.
-__global__ void __launch_bounds__(kBoundSlots) k_dep_begin(F32Form f, int do_int) {
-  __shared__ uint32_t part[4][kBoundSlots / 32];
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  uint4 *slots = reinterpret_cast<uint4 *>(f.slots);
-  const uint4 s = slots[t];
-  slots[t] = make_uint4(0u, 0u, 0u, 0u);
-  const uint32_t m[4] = {__reduce_max_sync(0xffffffffu, s.x), __reduce_max_sync(0xffffffffu, s.y),
-                         __reduce_max_sync(0xffffffffu, s.z), __reduce_max_sync(0xffffffffu, s.w)};
-  if (lane == 0) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) part[q][wid] = m[q];
-  }
-  __syncthreads();
-  if (wid < 5) {
-    // largest contribution of each field: concentration weights <= 1, momentum |RHS_u|,
-    // energy |RHS_T| (weights <= 1); its magnitude maps to at most 2^24
-    const float b = wid == 0 ? 1.f : __uint_as_float(__reduce_max_sync(0xffffffffu, part[wid - 1][lane]));
-    if (lane == 0) {
-      int e = 0;
-      if (b > 0.f && isfinite(b)) frexpf(b, &e);  // b < 2^e
-      const int se = 24 - e;
-      f.se[wid] = se > 100 ? 100 : se;
-    }
-  }
-  if (t < 15 && (do_int || t % 5 == 4))
-    f.totals[t] = t < 5 ? 0ull : (t < 10 ? (unsigned long long)LLONG_MIN : (unsigned long long)LLONG_MAX);
-  if (t == 32) f.work.counts[2] = 0;
-}
-
 // q * 2^-se, exact: 2^52 + 2^31 + q from its digits, times 2^-se less the offset in one operation
 __device__ __forceinline__ double small_to_f64(int32_t q, int se) {
   const int scale = (1023 - se) << 20;  // 2^-se's high word
@@ -995,9 +963,47 @@ __global__ void __launch_bounds__(kDepThreads, 4)
   __shared__ int4 next_item;
   const Work &w = f.work;
   const int32_t n_slices = w.counts[0], n_items = n_slices + w.counts[1];
+  // Every CTA works out the fields' scales from the stage's partial maxima (16 KB of L2 reads a CTA; a
+  // launch of their own cost 5 us with its gap), the first one leaves them to the gather and
+  // readies the statistics. The gather clears the maxima and the item counter.
+  __shared__ uint32_t part[4][kDepThreads / 32];
+  __shared__ int exponent[5];
+  {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t m[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int q = 0; q < kBoundSlots / kDepThreads; ++q) {
+      const uint4 v = reinterpret_cast<const uint4 *>(f.slots)[q * kDepThreads + threadIdx.x];
+      m[0] = max(m[0], v.x);
+      m[1] = max(m[1], v.y);
+      m[2] = max(m[2], v.z);
+      m[3] = max(m[3], v.w);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) m[q] = __reduce_max_sync(0xffffffffu, m[q]);
+    if (lane < 4) part[lane][wid] = lane == 0 ? m[0] : (lane == 1 ? m[1] : (lane == 2 ? m[2] : m[3]));
+    __syncthreads();
+    if (threadIdx.x < 5) {
+      // largest contribution of each field: concentration weights <= 1, momentum |RHS_u|,
+      // energy |RHS_T| (weights <= 1); its magnitude maps to at most 2^24
+      uint32_t top = 0u;
+      if (threadIdx.x)
+        for (int q = 0; q < kDepThreads / 32; ++q) top = max(top, part[threadIdx.x - 1][q]);
+      const float b = threadIdx.x ? __uint_as_float(top) : 1.f;
+      int e = 0;
+      if (b > 0.f && isfinite(b)) frexpf(b, &e);  // b < 2^e
+      const int se = 24 - e > 100 ? 100 : 24 - e;
+      exponent[threadIdx.x] = se;
+      if (blockIdx.x == 0) f.se[threadIdx.x] = se;
+    }
+    if (blockIdx.x == 0 && threadIdx.x < 15 && (FIELDS || threadIdx.x % 5 == 4))
+      f.totals[threadIdx.x] =
+          threadIdx.x < 5 ? 0ull : (threadIdx.x < 10 ? (unsigned long long)LLONG_MIN : (unsigned long long)LLONG_MAX);
+    __syncthreads();
+  }
   float scale[5];
 #pragma unroll
-  for (int q = 0; q < 5; ++q) scale[q] = ldexpf(1.0f, f.se[q]);  // exact powers of two
+  for (int q = 0; q < 5; ++q) scale[q] = ldexpf(1.0f, exponent[q]);  // exact powers of two
   auto fetch = [&](int idx) {
     return idx >= n_items ? make_int4(-1, 0, 0, 0)
                           : (idx < n_slices ? w.items[idx] : w.items[w.slice_cap + idx - n_slices]);
@@ -1187,6 +1193,10 @@ __global__ void __launch_bounds__(256, 4) k_dep_gather(Geom G, F32Form f, int32_
       wide[1] = LLONG_MAX;
     }
     __syncthreads();
+  }
+  if (blockIdx.x == 0 && fq == 0) {  // ready for the next stage's maxima and the next launch's items
+    for (int q = threadIdx.x; q < kBoundSlots; q += blockDim.x) reinterpret_cast<uint4 *>(f.slots)[q] = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x == 0) w.counts[2] = 0;
   }
   if (fq >= sums) {
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < G.gsize; t += (int64_t)gridDim.x * blockDim.x)
@@ -2122,8 +2132,6 @@ int dep_launch(pstep_ctx *h, bool do_int, Set32 SI, Set32 SN, bool ext) {
   const Geom &G = h->geom;
   const int32_t epoch = ++f.epoch;
   const int twc = h->cfg.twc;
-  k_dep_begin<<<1, kBoundSlots, 0, h->stream>>>(f, do_int ? 1 : 0);
-  PSTEP_LAUNCHED(h);
   // fields with sums: RHS_Part_Temp, and C, and (with TWC) the momentum
   const int fields = do_int ? (twc ? 2 : 1) : 0;
   const int64_t most = (int64_t)f.work.nb + f.work.slice_cap;
