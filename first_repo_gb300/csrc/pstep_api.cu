@@ -48,7 +48,6 @@ StageConst make_stage_const(const pstep_config &cfg, int k, double pre, double p
 int f64_prime_kernel(pstep_ctx *h);
 int deposit_temperature(pstep_ctx *h, const Csr &csr, double *const frac[3], const uint32_t *key);
 int f64_temp_gather(pstep_ctx *h);
-int exclusive_scan(pstep_ctx *h, const int32_t *in, int64_t n, int32_t *out, int32_t *out2);
 int64_t scan_blocks_needed(int64_t n);
 int64_t order_scratch_words(int64_t cap);
 int f32_create(pstep_ctx *h);

@@ -181,8 +181,8 @@ int f64_stage_temp(pstep_ctx *h);
 int f64_reorder(pstep_ctx *h);
 int sort_by_node(pstep_ctx *h, const uint32_t *keys, Csr &out);
 int csr_sort(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, const int32_t *order, int32_t *cell_start,
-             int32_t *sidx, int32_t *okey, int order_within);
-int csr_count(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, int32_t *cell_start);
+             int32_t *sidx, int32_t *okey, int order_within, bool counted = false);
+int exclusive_scan(pstep_ctx *h, const int32_t *in, int64_t n, int32_t *out, int32_t *out2);
 int f32_download(pstep_ctx *h, double *const dst[7], int32_t *flag, int on_device);
 int f32_field_stats(pstep_ctx *h, int field, double r[3]);
 int f32_fused_max(pstep_ctx *h, int id, double *out);

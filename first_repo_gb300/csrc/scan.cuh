@@ -75,6 +75,31 @@ __device__ inline int32_t scan_before(const ScanState &scan, uint32_t epoch, int
   return before;
 }
 
+// The lanes that add to a key together: those with lane 7's key, those with lane 24's, and else
+// the run of neighbouring lanes with one key. The storage is nearly in key order, so these are
+// almost all that a match over the whole warp would find; that takes a pass per distinct key, and
+// shuffles over the groups it finds go one group after the other. Runs alone are broken by every particle
+// that has moved on, and in a crowded cell each piece's addition waits for the others'. Count and
+// scatter of 2^24 particles on 256^3 cells, and of 2^27 on 512^3 with 1000 in the fullest cells:
+// by match 83, 166 us and 0.70, 1.46 ms; by runs 55, 97 us and 1.33, 1.81 ms; this way 55, 93 us and
+// 0.86, 1.22 ms.
+struct Run {
+  int first, len, place;
+};
+__device__ __forceinline__ Run run_of(uint32_t key) {
+  const int lane = (int)(threadIdx.x & 31);
+  const uint32_t before = __shfl_up_sync(0xffffffffu, key, 1);
+  const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || key != before);
+  const uint32_t low = __ballot_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, 7));
+  const uint32_t high = __ballot_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, 24));
+  const uint32_t upto = 0xffffffffu >> (31 - lane);  // the lane and those below
+  const int head = 31 - __clz(heads & upto);
+  const uint32_t after = heads & ~upto;
+  const uint32_t run = (after ? (1u << (__ffs(after) - 1)) - 1u : 0xffffffffu) & ~((1u << head) - 1u);
+  const uint32_t mine = (low >> lane) & 1u ? low : ((high >> lane) & 1u ? high : run);
+  return Run{__ffs(mine) - 1, __popc(mine), __popc(mine & upto) - 1};
+}
+
 // Exclusive scan over the block's kThreads threads; smem: kThreads / 32 words.
 __device__ inline int32_t block_excl_scan(int32_t v, int32_t *smem, int32_t &total) {
   int lane = threadIdx.x & 31, w = threadIdx.x >> 5;

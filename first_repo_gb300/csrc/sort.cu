@@ -13,31 +13,6 @@ namespace {
 constexpr int kScanItems = 16;                       // per thread
 constexpr int kScanTile = kThreads * kScanItems;     // per block
 
-// The lanes that add to a key together: those with lane 7's key, those with lane 24's, and else
-// the run of neighbouring lanes with one key. The storage is nearly in key order, so these are
-// almost all that a match over the whole warp would find; that takes a pass per distinct key, and
-// shuffles over the groups it finds go one group after the other. Runs alone are broken by every particle
-// that has moved on, and in a crowded cell each piece's addition waits for the others'. Count and
-// scatter of 2^24 particles on 256^3 cells, and of 2^27 on 512^3 with 1000 in the fullest cells:
-// by match 83, 166 us and 0.70, 1.46 ms; by runs 55, 97 us and 1.33, 1.81 ms; this way 55, 93 us and
-// 0.86, 1.22 ms.
-struct Run {
-  int first, len, place;
-};
-__device__ __forceinline__ Run run_of(uint32_t key) {
-  const int lane = (int)(threadIdx.x & 31);
-  const uint32_t before = __shfl_up_sync(0xffffffffu, key, 1);
-  const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || key != before);
-  const uint32_t low = __ballot_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, 7));
-  const uint32_t high = __ballot_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, 24));
-  const uint32_t upto = 0xffffffffu >> (31 - lane);  // the lane and those below
-  const int head = 31 - __clz(heads & upto);
-  const uint32_t after = heads & ~upto;
-  const uint32_t run = (after ? (1u << (__ffs(after) - 1)) - 1u : 0xffffffffu) & ~((1u << head) - 1u);
-  const uint32_t mine = (low >> lane) & 1u ? low : ((high >> lane) & 1u ? high : run);
-  return Run{__ffs(mine) - 1, __popc(mine), __popc(mine & upto) - 1};
-}
-
 __global__ void k_count(const uint32_t *__restrict__ keys, int shift, int64_t n, int32_t *__restrict__ counts) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = i < n;
@@ -279,11 +254,12 @@ int exclusive_scan(pstep_ctx *h, const int32_t *in, int64_t n, int32_t *out, int
 int64_t scan_blocks_needed(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
 
 // Counting sort of the h->np particles by (keys[i] >> shift) into nkeys buckets:
-// cell_start[0..nkeys] and sidx, every bucket ordered by the secondary key.
+// cell_start[0..nkeys] and sidx, every bucket ordered by the secondary key. counted: h->counts already
+// holds the buckets' sizes.
 int csr_sort(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, const int32_t *order, int32_t *cell_start,
-             int32_t *sidx, int32_t *okey, int order_within) {
-  PSTEP_CUDA(cudaMemsetAsync(h->counts, 0, sizeof(int32_t) * nkeys, h->stream));
-  if (h->np > 0) {
+             int32_t *sidx, int32_t *okey, int order_within, bool counted) {
+  if (!counted) PSTEP_CUDA(cudaMemsetAsync(h->counts, 0, sizeof(int32_t) * nkeys, h->stream));
+  if (h->np > 0 && !counted) {
     k_count<<<blocks_for(h->np), kThreads, 0, h->stream>>>(keys, shift, h->np, h->counts);
     PSTEP_LAUNCHED(h);
   }
@@ -313,17 +289,6 @@ int csr_sort(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, const
     }
   }
   return PSTEP_OK;
-}
-
-// the cell-start table of keys already in non-decreasing order (no permutation needed):
-// the counts and their exclusive scan, as csr_sort makes them
-int csr_count(pstep_ctx *h, const uint32_t *keys, int shift, int64_t nkeys, int32_t *cell_start) {
-  PSTEP_CUDA(cudaMemsetAsync(h->counts, 0, sizeof(int32_t) * nkeys, h->stream));
-  if (h->np > 0) {
-    k_count<<<blocks_for(h->np), kThreads, 0, h->stream>>>(keys, shift, h->np, h->counts);
-    PSTEP_LAUNCHED(h);
-  }
-  return exclusive_scan(h, h->counts, nkeys, cell_start, nullptr);
 }
 
 int sort_by_node(pstep_ctx *h, const uint32_t *keys, Csr &out) {
