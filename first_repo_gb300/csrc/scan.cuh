@@ -59,6 +59,7 @@ __device__ inline int32_t scan_before(const ScanState &scan, uint32_t epoch, int
       while ((uint32_t)(w >> 34) != epoch || ((uint32_t)(w >> 32) & 3u) == 0) {
         if (++polls == kScanWait) {
           atomicOr(scan.err, kErrTimeout);
+          w = 0;  // not an earlier scan's value: the sum stays within this one's, and what it indexes too
           break;
         }
         w = st[q];
