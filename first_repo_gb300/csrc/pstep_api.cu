@@ -511,6 +511,9 @@ int pstep_prime(pstep_handle h) {
   h->np1_is_base = 1;
   h->primed = 1;
   h->phase = 0;
+  // a stage that a prime breaks off leaves nothing to be gathered
+  h->t_rebound = 0;
+  h->t_pending = 0;
   return PSTEP_OK;
 }
 
@@ -750,7 +753,7 @@ int pstep_get_particle_array(pstep_handle h, int id, void *dst, int on_device) {
       src = h->np1_is_base ? h->s.base[q] : h->s.np1[q];
     } else {
       // asked for before pstep_stage_temp: with the temperature bound now
-      if (h->t_pending) TRY(f64_temp_gather(h));
+      if (h->t_pending && h->phase != 0) TRY(f64_temp_gather(h));
       src = h->s.rhs_t;
     }
     double *tmp = (double *)h->perm_tmp;
