@@ -29,6 +29,8 @@ struct DepIn {
   const double *frac[3];
   const uint32_t *key;
   const double *val[3];       // RHS_u,v,w (int-deposit) or RHS_T in val[0] (temperature deposit)
+  const double *kept;         // the int-deposit: a field to be copied beside the targets, or nullptr
+  double *keep;
 };
 
 __device__ inline int32_t pidx(const DepIn &d, int32_t p) { return d.sidx ? d.sidx[p] : p; }
@@ -175,6 +177,10 @@ __global__ void __launch_bounds__(32 * kOrdWarps) k_dep_ordered(Geom G, DepIn d,
     if (ti < G.g[0] && tj < G.g[1] && tk < G.g[2]) out[glin(G, ti, tj, tk)] = v;
   };
   put(out_tri, 0, 0, acc);
+  if (d.keep && b0 + tx < G.g[0] && b1 + ty < G.g[1] && b2 + tz < G.g[2]) {
+    const long long t = glin(G, b0 + tx, b1 + ty, b2 + tz);
+    d.keep[t] = d.kept[t];
+  }
   if (FACES) {
     put(out_x, 0, 2, ax);
     put(out_y, 2, 0, ay);
@@ -548,6 +554,8 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_dep_brick(Geom G, DepIn d,
     const int lx = s % kB, ly = (s / kB) % kB, lz = s / (kB * kB);
     const int ti = bx + lx, tj = by + ly, tk = bz + lz;
     if (ti >= G.g[0] || tj >= G.g[1] || tk >= G.g[2]) continue;
+    const long long t = glin(G, ti, tj, tk);
+    const double kept = !MODE && d.keep ? __ldcs(d.kept + t) : 0.0;
     double acc = 0.0;
 #pragma unroll
     for (int o = 0; o < 8; ++o) {
@@ -555,7 +563,8 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_dep_brick(Geom G, DepIn d,
       const double v = sm.tri[o][((lz + oz) * kB1 + (ly + oy)) * kB1 + (lx + ox)];
       acc = o ? acc + v : v;
     }
-    out_tri[glin(G, ti, tj, tk)] = acc;
+    out_tri[t] = acc;
+    if (!MODE && d.keep) __stcs(d.keep + t, kept);
   }
   if (!faces) return;
   __syncthreads();
@@ -774,6 +783,8 @@ DepIn make_in(pstep_ctx *h, const Csr &csr, double *const frac[3], const uint32_
   d.val[0] = v0;
   d.val[1] = v1;
   d.val[2] = v2;
+  d.kept = nullptr;
+  d.keep = nullptr;
   return d;
 }
 
@@ -851,6 +862,10 @@ int deposit_temperature(pstep_ctx *h, const Csr &csr, double *const frac[3], con
 // part2gas_concentration + part2gas_velocity at x_int (records of the previous CSR)
 int f64_deposit_int(pstep_ctx *h) {
   DepIn d = make_in(h, h->csr_prev, h->s.frac_prev, h->s.key_prev, h->s.rhs_u[0], h->s.rhs_u[1], h->s.rhs_u[2]);
+  if (h->t_pending) {
+    d.kept = h->tf;
+    d.keep = h->t_kept;
+  }
   double *c = h->dep[PSTEP_FIELD_C], *x = h->dep[PSTEP_FIELD_RU_X], *y = h->dep[PSTEP_FIELD_RU_Y],
          *z = h->dep[PSTEP_FIELD_RU_Z];
   const int rc = reference_sums(h) ? ordered_launch(h, d, h->cfg.twc, 0, c, x, y, z) : brick_launch(h, d, 0, c, x, y, z);

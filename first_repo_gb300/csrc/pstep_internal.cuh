@@ -133,6 +133,8 @@ struct pstep_ctx {
   int fields_t_at_advance;  // temperature binding seen by the fused advance kernel
   int t_rebound;            // FP64 form: the last stage's temperature was bound after its advance
   int t_pending;            // FP64 form: this stage's advance left the temperature gather to stage_temp
+  double *t_kept;           // the temperature field as that advance saw it, for a caller that then binds no other
+  double t_kept_itth;       // and the heat-transfer coefficient
   int64_t stages_done;
   int timed;
   int phase;  // 0: idle, 1: after interp_advance_deposit, 2: after wrap, 3: after stage_temp

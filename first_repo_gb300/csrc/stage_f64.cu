@@ -357,11 +357,10 @@ int f64_fused_max(pstep_ctx *h, int id, double *out) {
   return PSTEP_OK;
 }
 
-int f64_temp_gather(pstep_ctx *h) {
+int f64_temp_gather(pstep_ctx *h, const double *T, double itth) {
   if (h->np == 0) return PSTEP_OK;
-  StageConst c = make_stage_const(h->cfg, 0, 0.5, 1. / 6.);
   const int blocks = (int)((h->np + kThreads - 1) / kThreads);
-  k_temp_gather<<<blocks, kThreads, 0, h->stream>>>(h->geom, h->s, h->tf, c.itth, h->np);
+  k_temp_gather<<<blocks, kThreads, 0, h->stream>>>(h->geom, h->s, T, itth, h->np);
   PSTEP_LAUNCHED(h);
   return PSTEP_OK;
 }

@@ -97,8 +97,7 @@ enum {
   PSTEP_X_INT, PSTEP_Y_INT, PSTEP_Z_INT, PSTEP_U_INT, PSTEP_V_INT, PSTEP_W_INT, PSTEP_T_INT,
   PSTEP_X_NEW, PSTEP_Y_NEW, PSTEP_Z_NEW, PSTEP_U_NEW, PSTEP_V_NEW, PSTEP_W_NEW, PSTEP_T_NEW,
   PSTEP_X_NP1, PSTEP_Y_NP1, PSTEP_Z_NP1, PSTEP_U_NP1, PSTEP_V_NP1, PSTEP_W_NP1, PSTEP_T_NP1,
-  PSTEP_RHS_T,               /* particle.h:116; FP64 form, asked for between interp_advance_deposit and
-                                stage_temp: with the temperature bound at that time */
+  PSTEP_RHS_T,               /* particle.h:116 */
   PSTEP_FLAG,                /* int32 particle id (particle.h:119) */
   PSTEP_UG, PSTEP_VG, PSTEP_WG, /* gas velocity at x_int used by the last stage (gas2part_velocity,
                                    particle.cpp:340-360); FP32 with PSTEP_KEEP_GAS */
