@@ -114,6 +114,13 @@ __global__ void __launch_bounds__(kThreads) k_list(const uint8_t *__restrict__ c
   }
 }
 
+__device__ __noinline__ int32_t word_tile_sum(const uint32_t *bitmap, int32_t tile) {
+  bitmap += (int64_t)tile * kWordTile;
+  int32_t sum = 0;
+  for (int w = threadIdx.x & 31; w < kWordTile; w += 32) sum += __popc(bitmap[w]);
+  return (int32_t)__reduce_add_sync(0xffffffffu, (unsigned)sum);
+}
+
 // The leavers' positions in ascending order, the set bits before every word, and l; clears the
 // bitmap that k_pass sets next.
 __global__ void __launch_bounds__(kThreads) k_leavers(const uint32_t *__restrict__ bitmap, uint32_t *__restrict__ clear,
@@ -135,7 +142,7 @@ __global__ void __launch_bounds__(kThreads) k_leavers(const uint32_t *__restrict
   int32_t total;
   int32_t e = block_excl_scan(s, sm, total);
   if (threadIdx.x < 32) {
-    const int32_t before = scan_before(scan, epoch, tile, total);
+    const int32_t before = scan_before<uint32_t, word_tile_sum>(scan, epoch, tile, total, bitmap);
     if (threadIdx.x == 0) s_before = before;
   }
   __syncthreads();

@@ -1,9 +1,10 @@
 // One-pass scans over tiles (decoupled look-back), for kernels whose blocks take a tile each: every
 // block takes the next tile by a ticket, publishes its tile's sum, then adds up its predecessors'
 // published values from the nearest one back until it meets an inclusive prefix. Tickets are handed
-// out in order, so a tile's predecessors are running or done; the wait is bounded all the same. A
-// tile's word is (epoch, state, value): words of an earlier scan are told by their epoch, so nothing
-// is cleared. The epoch is counted on the device beside the ticket, so that a launch that is
+// out in order, so a tile's predecessors are running or done; the wait is bounded all the same, and a
+// tile that is still missing then is summed by the waiting block itself, so that a scan's result
+// never depends on the waits. A tile's word is (epoch, state, value): words of an earlier scan are
+// told by their epoch, so nothing is cleared. The epoch is counted on the device beside the ticket, so that a launch that is
 // replayed has one of its own each time.
 #pragma once
 #include "pstep_internal.cuh"
@@ -13,14 +14,16 @@ namespace pstep {
 struct ScanState {
   unsigned long long *status;  // a word per tile
   unsigned long long *ticket;  // epoch << 32 | the next tile
-  int32_t *err;
+  uint32_t polls;              // looks at a predecessor's word before its tile is summed here
 };
-
-inline ScanState scan_state(pstep_ctx *h) { return ScanState{h->scan_status, h->scan_ticket, h->err_word}; }
 
 constexpr uint32_t kScanSum = 1, kScanPrefix = 2;
 constexpr uint32_t kScanEpochs = 0x3fffffffu;
-constexpr uint32_t kScanWait = 1u << 24;  // polls of one predecessor
+constexpr uint32_t kScanPolls = 1u << 16;
+
+inline ScanState scan_state(pstep_ctx *h) {
+  return ScanState{h->scan_status, h->scan_ticket, h->wait_idle ? 0u : (h->wait_limit ? h->wait_limit : kScanPolls)};
+}
 
 // The block's tile of this launch (all threads call).
 __device__ inline int32_t scan_take(const ScanState &scan, uint32_t &epoch) {
@@ -36,8 +39,10 @@ __device__ inline int32_t scan_take(const ScanState &scan, uint32_t &epoch) {
   return (int32_t)(uint32_t)taken;
 }
 
-// The sum of the tiles before `tile`, whose own sum is `total` (one whole warp calls).
-__device__ inline int32_t scan_before(const ScanState &scan, uint32_t epoch, int32_t tile, int32_t total) {
+// The sum of the tiles before `tile`, whose own sum is `total` (one whole warp calls). sum_of(in, q): tile
+// q's sum from the scan's input, by the whole warp, in every lane.
+template <typename T, int32_t (*sum_of)(const T *, int32_t)>
+__device__ inline int32_t scan_before(const ScanState &scan, uint32_t epoch, int32_t tile, int32_t total, const T *in) {
   const int lane = (int)(threadIdx.x & 31);
   volatile unsigned long long *st = scan.status;
   auto word = [&](uint32_t state, int32_t value) {
@@ -55,20 +60,21 @@ __device__ inline int32_t scan_before(const ScanState &scan, uint32_t epoch, int
     int32_t value = 0;
     if (q >= 0) {
       unsigned long long w = st[q];
-      uint32_t polls = 0;
-      while ((uint32_t)(w >> 34) != epoch || ((uint32_t)(w >> 32) & 3u) == 0) {
-        if (++polls == kScanWait) {
-          atomicOr(scan.err, kErrTimeout);
-          w = 0;  // not an earlier scan's value: the sum stays within this one's, and what it indexes too
-          break;
-        }
-        w = st[q];
-      }
+      uint32_t polls = 1;
+      while (((uint32_t)(w >> 34) != epoch || ((uint32_t)(w >> 32) & 3u) == 0) && ++polls <= scan.polls) w = st[q];
+      if (polls > scan.polls) w = 0;  // not there
       state = (uint32_t)(w >> 32) & 3u;
       value = (int32_t)(uint32_t)w;
     }
     const unsigned prefix = __ballot_sync(0xffffffffu, state == kScanPrefix);
     const int stop = prefix ? __ffs(prefix) - 1 : 31;
+    // (of the tiles up to the prefix; what is behind it does not matter)
+    for (unsigned missing = __ballot_sync(0xffffffffu, state == 0u) & (0xffffffffu >> (31 - stop)); missing;
+         missing &= missing - 1u) {
+      const int l = __ffs(missing) - 1;
+      const int32_t sum = sum_of(in, at - l);
+      if (lane == l) value = sum;
+    }
     before += (int32_t)__reduce_add_sync(0xffffffffu, (unsigned)(lane <= stop ? value : 0));
     if (prefix) break;
   }

@@ -32,6 +32,13 @@ __device__ __forceinline__ int32_t place_of(const uint32_t *__restrict__ keys, i
   return __shfl_sync(0xffffffffu, base, run.first) + run.place;
 }
 
+__device__ __noinline__ int32_t tile_sum(const int32_t *in, int32_t tile) {
+  in += (int64_t)tile * kScanTile;
+  int32_t sum = 0;
+  for (int i = threadIdx.x & 31; i < kScanTile; i += 32) sum += in[i];
+  return (int32_t)__reduce_add_sync(0xffffffffu, (unsigned)sum);
+}
+
 // Exclusive scan in one pass (scan_take, scan_before). Writes out[0..n] (out[n] = total) and out2
 // (optional). The three-launch form (tile sums, their scan by one block, apply) took 9.3 us at 64^3
 // keys and 26 us at 256^3, this 4.5 and 25 us.
@@ -63,7 +70,7 @@ __global__ void __launch_bounds__(kThreads) k_scan(const int32_t *__restrict__ i
   int32_t total;
   int32_t e = block_excl_scan(s, sm, total);
   if (threadIdx.x < 32) {
-    const int32_t before = scan_before(scan, epoch, tile, total);
+    const int32_t before = scan_before<int32_t, tile_sum>(scan, epoch, tile, total, in);
     if (threadIdx.x == 0) s_before = before;
   }
   __syncthreads();

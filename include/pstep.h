@@ -201,7 +201,10 @@ int pstep_set_correction(pstep_handle h, const pstep_correction *c);
  * (always with the default bound), frees its tensor memory and returns. With
  * idle_first != 0 each warpgroup's first wait polls a barrier that nothing signals, so
  * the timeout path runs as it would for a completion that never arrives (for testing
- * that path; the stage's results are then incomplete). No reference counterpart. */
+ * that path; the stage's results are then incomplete). The scans of the sort and of the
+ * order passes take the same limit (default 2^16) for one block's wait on another, after
+ * which a block sums for itself what it waited for, with idle_first at once: their
+ * results are the same whatever the limit. No reference counterpart. */
 int pstep_set_wait_limit(pstep_handle h, uint32_t polls, int idle_first);
 int64_t pstep_num_particles(pstep_handle h);
 
