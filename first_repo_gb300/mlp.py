@@ -15,7 +15,7 @@ from . import _lib
 N_IN, N_HID, N_OUT, NPARAM = 10, 64, 4, 6288
 
 EXPORTS = ["pmlp_create", "pmlp_destroy", "pmlp_set_stream", "pmlp_get_params", "pmlp_set_params", "pmlp_set_data",
-           "pmlp_train", "pmlp_gradient", "pmlp_forward", "pmlp_steps", "pmlp_launch_count", "pmlp_last_error"]
+           "pmlp_train", "pmlp_gradient", "pmlp_forward", "pmlp_set_wait_limit", "pmlp_steps", "pmlp_launch_count", "pmlp_last_error"]
 
 _VP = C.c_void_p
 _F = C.POINTER(C.c_float)
@@ -34,6 +34,7 @@ def lib():
     L.pmlp_train.argtypes = [_VP, C.c_int64, C.c_int, C.c_float, C.c_uint64, _F]
     L.pmlp_gradient.argtypes = [_VP, C.c_int, _F, _F]
     L.pmlp_forward.argtypes = [_VP, _VP, C.c_int64, _VP, C.c_int]
+    L.pmlp_set_wait_limit.argtypes = [_VP, C.c_uint32, C.c_int64]
     L.pmlp_steps.argtypes = [_VP]
     L.pmlp_steps.restype = C.c_int64
     L.pmlp_launch_count.argtypes = [_VP]
@@ -118,6 +119,11 @@ class Mlp:
         y = np.empty((x.shape[0], N_OUT), dtype=np.float32)
         self._check(self.L.pmlp_forward(self.h, x.ctypes.data, x.shape[0], y.ctypes.data, 0))
         return y
+
+    def set_wait_limit(self, polls: int = 0, idle_step: int = -1):
+        """bound of the training kernels' tensor-core completion waits (0: default); idle_step: the step whose
+        first wait polls a barrier that nothing signals (timeout test)"""
+        self._check(self.L.pmlp_set_wait_limit(self.h, int(polls), int(idle_step)))
 
     @property
     def steps(self) -> int:

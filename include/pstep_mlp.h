@@ -50,7 +50,10 @@ int pmlp_set_data(pmlp_handle h, const float *x, const float *y, int64_t n, int 
 
 /* `steps` Adam steps on batches of `batch` rows (a multiple of 128) drawn with
  * replacement from the training set by a hash of (seed, step, slot); loss, if
- * not NULL, receives the batch loss of every step (steps floats, host) */
+ * not NULL, receives the batch loss of every step (steps floats, host). A tensor-core
+ * completion wait that runs out (PSTEP_ERR_TIMEOUT) ends the training with the step
+ * before: that step and later ones change nothing, pmlp_steps counts those taken, and
+ * the error stands until pmlp_set_params */
 int pmlp_train(pmlp_handle h, int64_t steps, int batch, float lr, uint64_t seed, float *loss);
 
 /* gradient of the mean squared error over rows [0, batch) of the training set
@@ -61,6 +64,10 @@ int pmlp_gradient(pmlp_handle h, int batch, float *grad, float *loss);
 /* outputs for n feature rows: x [n][PMLP_IN] -> y [n][PMLP_OUT] */
 int pmlp_forward(pmlp_handle h, const float *x, int64_t n, float *y, int on_device);
 
+/* The training and gradient kernels' completion waits give up after `polls` polls (0: the
+ * default, 2^22). With idle_step >= 0 the step after that many Adam steps polls a barrier
+ * that nothing signals first, so that its wait runs out (for testing that path; -1: none). */
+int pmlp_set_wait_limit(pmlp_handle h, uint32_t polls, int64_t idle_step);
 /* Adam steps taken so far */
 int64_t pmlp_steps(pmlp_handle h);
 /* tensor-core kernel launches made by this handle so far */
