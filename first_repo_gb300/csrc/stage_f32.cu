@@ -107,7 +107,8 @@ struct F32Form {
   int ext_ok[5];               // per field: its last deposit gathered the extrema too
   Work work;
   int32_t epoch;      // deposit launches so far
-  int whole_since;    // a launch has written all fields' tiles since the work lists were made
+  int whole_since;    // a launch has written C's and RHS_Part_Temp's tiles since the work lists were made
+  int mom_stale;      // a launch has written those alone: momentum rows of other bricks may hold sums
   int32_t *done;      // blocks of the running k_dep_gather that have finished
   void *corr_mem;     // learned correction: packed weight image + biases (device), or nullptr
   int sorted;
@@ -804,7 +805,8 @@ __device__ inline double fixed_to_f64(long long q, int se) {
 // more than kItemMax particles, which come first (no brick holds up the end). A brick whose
 // tile in memory holds an earlier population's words is an item with no particles: it then
 // writes a tile of zeros, so that the gather reads every tile without asking. keep: no launch has
-// written all fields' tiles since the last lists were made; what they were to clear is listed again.
+// written the tiles of C and RHS_Part_Temp since the last lists were made; what they were to clear is
+// listed again. (A run without TWC leaves the momentum rows as they are: dep_launch.)
 __global__ void __launch_bounds__(256) k_work(const int32_t *__restrict__ cs, Work w, int keep) {
   __shared__ int32_t warp_n[8], base;
   const int b = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -2152,10 +2154,17 @@ int dep_launch(pstep_ctx *h, bool do_int, Set32 SI, Set32 SN, bool ext) {
   const int fields = do_int ? (twc ? 2 : 1) : 0;
   const int64_t most = (int64_t)f.work.nb + f.work.slice_cap;
   const unsigned grid_t = (unsigned)(most < 4 * (int64_t)h->num_sms ? most : 4 * (int64_t)h->num_sms);
+  if (fields == 2 && f.mom_stale) {  // TWC switched on again: this launch writes the listed bricks' tiles, the rest are zeros
+    PSTEP_CUDA(cudaMemsetAsync(f.work.mid, 0, sizeof(uint32_t) * f.work.nb * kRows * kBr, h->stream));
+    PSTEP_CUDA(cudaMemsetAsync(f.work.side, 0, sizeof(uint32_t) * f.work.nb * kSideWords, h->stream));
+  }
   auto tile = fields == 2 ? k_dep_tile<2> : (fields == 1 ? k_dep_tile<1> : k_dep_tile<0>);
   tile<<<grid_t, kDepThreads, 0, h->stream>>>(G, f, SI, SN, epoch);
   PSTEP_LAUNCHED(h);
-  if (fields == 2) f.whole_since = 1;
+  if (fields) {
+    f.whole_since = 1;
+    f.mom_stale = fields == 1;
+  }
   double *C = h->dep[PSTEP_FIELD_C], *X = h->dep[PSTEP_FIELD_RU_X], *Y = h->dep[PSTEP_FIELD_RU_Y],
          *Z = h->dep[PSTEP_FIELD_RU_Z], *E = h->dep[PSTEP_FIELD_PART_TEMP];
   const int64_t tasks = (int64_t)((G.n[0] + 31) / 32) * (G.n[1] / kBr) * (G.n[2] / kBr), fit = 4 * (int64_t)h->num_sms;
