@@ -55,6 +55,13 @@ struct Set32 {
 // The deposit's work (see k_dep_tile): the sort's 8^3 bricks, or slices of those with more than
 // kItemMax particles.
 constexpr int kItemMax = 8192;
+// Thin populations have no tiles: the tiles' way through memory, 41 B a cell each way, is then most of
+// the deposit. A step at 512^3 with 4, 8, 16, 64, 512 cells a particle, tiles: 27.0, 23.3, 21.4, 19.5, 16.2 ms, a word
+// a cell: 31.0, 21.7, 16.7, 12.3, 8.5; at 256^3 3.33, 2.89, 2.66, 2.44, 2.01 and 3.95, 2.83, 2.22, 1.64, 1.20. At 64^3,
+// where all of it stays in L2, tiles are faster throughout (0.157 against 0.168 ms).
+inline bool thin_population(int64_t particles, int64_t cells) {
+  return cells >= (1 << 21) && particles * (cells >= (1 << 26) ? 6 : 8) <= cells;
+}
 constexpr int kBrickCells = kBr * kBr * kBr;
 // A brick's tile: the int32 sums of its particles' contributions to the cells and faces they
 // reach, one cell around the brick (momentum faces two above it along their own axis), as rows
@@ -75,7 +82,8 @@ struct Work {
   int32_t *counts;       // [0] slices, [1] whole bricks, [2] the running launch's next item
   uint8_t *dirty;        // per brick: 2 its tile in memory holds sums, 1 it is listed to be cleared, 0 zeros
   int32_t *extra_epoch;  // per brick: the last deposit launch that added to its cells in `extra`
-  uint32_t *mid;         // [brick row (z, y)][kRows][cells along x]
+  int32_t *word_epoch;   // thin populations, per brick: the last launch that added to its cells' words
+  uint32_t *mid;         // [brick row (z, y)][kRows][cells along x]; thin: [5][cells in brick order]
   uint32_t *side;        // [brick][kSideWords]: x = -1, x = 8 (kRows each), x = 9 (RHS_RU x's rows)
   long long *extra;      // [5][cells in brick order]: what does not fit a tile's 32-bit words, exact
   int nb;                // bricks
@@ -108,6 +116,7 @@ struct F32Form {
   Work work;
   int32_t epoch;      // deposit launches so far
   int whole_since;    // a launch has written C's and RHS_Part_Temp's tiles since the work lists were made
+  int thin;           // this step's deposits have no tiles (add_words)
   int mom_stale;      // a launch has written those alone: momentum rows of other bricks may hold sums
   int32_t *done;      // blocks of the running k_dep_gather that have finished
   void *corr_mem;     // learned correction: packed weight image + biases (device), or nullptr
@@ -807,7 +816,8 @@ __device__ inline double fixed_to_f64(long long q, int se) {
 // writes a tile of zeros, so that the gather reads every tile without asking. keep: no launch has
 // written the tiles of C and RHS_Part_Temp since the last lists were made; what they were to clear is
 // listed again. (A run without TWC leaves the momentum rows as they are: dep_launch.)
-__global__ void __launch_bounds__(256) k_work(const int32_t *__restrict__ cs, Work w, int keep) {
+// thin: there are no tiles, so nothing is listed but the slices.
+__global__ void __launch_bounds__(256) k_work(const int32_t *__restrict__ cs, Work w, int keep, int thin) {
   __shared__ int32_t warp_n[8], base;
   const int b = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int32_t p0 = 0, p1 = 0;
@@ -816,10 +826,10 @@ __global__ void __launch_bounds__(256) k_work(const int32_t *__restrict__ cs, Wo
     p0 = cs[(int64_t)b * kBrickCells];
     p1 = cs[((int64_t)b + 1) * kBrickCells];
     const int st = w.dirty[b];
-    was = st == 2 || (st == 1 && keep);
+    was = !thin && (st == 2 || (st == 1 && keep));
   }
   const int cnt = p1 - p0;
-  const bool sums = cnt > 0 && cnt <= kItemMax, whole = sums || was;
+  const bool sums = !thin && cnt > 0 && cnt <= kItemMax, whole = sums || was;
   if (b < w.nb) w.dirty[b] = sums ? 2 : (was ? 1 : 0);
   const unsigned votes = __ballot_sync(0xffffffffu, whole);
   if (lane == 0) warp_n[wid] = __popc(votes);
@@ -936,6 +946,82 @@ __device__ __forceinline__ long long warp_sum_i64(long long v) {
   return (long long)shi * (1ll << 42) + (long long)smid * (1ll << 21) + (long long)slo;
 }
 
+// Thin populations have no tiles: a particle's contributions go straight to a word per cell and field
+// (Work::mid as [5][cells in brick order]), with the tiles' own handling of overflows. A cell's place
+// is a sum over the dimensions. at[d][.], brick[d][.]: that of the particle's cell less one, its cell and
+// its cell plus one (periodic), and of their bricks.
+struct Places {
+  uint32_t at[3][3], brick[3][3];
+};
+__device__ __forceinline__ Places places_of(const Geom &G, uint32_t cell) {
+  const int c[3] = {ci_(cell), cj_(cell), ck_(cell)};
+  const uint32_t across[3] = {1u, (uint32_t)(G.n[0] / kBr), (uint32_t)(G.n[0] / kBr) * (uint32_t)(G.n[1] / kBr)};
+  Places r;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      const int q = s == 0 ? (c[d] == 0 ? G.n[d] - 1 : c[d] - 1) : (s == 1 ? c[d] : (c[d] == G.n[d] - 1 ? 0 : c[d] + 1));
+      r.brick[d][s] = (uint32_t)(q / kBr) * across[d];
+      r.at[d][s] = r.brick[d][s] * kBrickCells + ((uint32_t)(q % kBr) << (3 * d));
+    }
+  return r;
+}
+__device__ __forceinline__ void mark_bricks(const Work &w, int32_t epoch, const Places &r) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int x = q & 1 ? 2 : 0, y = q & 2 ? 2 : 0, z = q & 4 ? 2 : 0;
+    if ((!x || r.brick[0][2] != r.brick[0][0]) && (!y || r.brick[1][2] != r.brick[1][0]) &&
+        (!z || r.brick[2][2] != r.brick[2][0]))
+      w.word_epoch[r.brick[0][x] + r.brick[1][y] + r.brick[2][z]] = epoch;
+  }
+}
+__device__ __noinline__ void word_overflow(const Work &w, int32_t epoch, int64_t at, uint32_t brick, int32_t v) {
+  atomicAdd((unsigned long long *)&w.extra[at], v > 0 ? 1ull << 32 : (unsigned long long)-(1ll << 32));
+  w.extra_epoch[brick] = epoch;
+}
+// contributions v[0 .. N) of field fld at the cells id[.]
+template <int N>
+__device__ __forceinline__ void add_words(const Work &w, int32_t epoch, int fld, const uint32_t (&id)[N], const int32_t (&v)[N]) {
+  uint32_t *words = w.mid + fld * w.ncell, over[N], any = 0u;
+#pragma unroll
+  for (int q = 0; q < N; ++q) over[q] = v[q] ? add_word(words + id[q], v[q]) : 0u;
+#pragma unroll
+  for (int q = 0; q < N; ++q) any |= over[q];
+  if ((int32_t)any < 0) {
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+      if ((int32_t)over[q] < 0) word_overflow(w, epoch, fld * w.ncell + id[q], id[q] / kBrickCells, v[q]);
+  }
+}
+__device__ __forceinline__ void add_trilinear(const Work &w, int32_t epoch, int fld, const Places &r, const float o3[3],
+                                              float val) {
+  float wt[3][2];
+  bool h[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    h[d] = o3[d] >= 0.5f;
+    const float xl = o3[d] - (o3[d] >= 0.5f ? 1.f : 0.f) + 0.5f;
+    wt[d][0] = 1.f - xl;
+    wt[d][1] = xl;
+  }
+  uint32_t id[8];
+  int32_t v[8];
+#pragma unroll
+  for (int oz = 0; oz < 2; ++oz)
+#pragma unroll
+    for (int oy = 0; oy < 2; ++oy) {
+      const float wyz = wt[2][oz] * wt[1][oy] * val;
+      const uint32_t yz = (h[1] ? r.at[1][oy + 1] : r.at[1][oy]) + (h[2] ? r.at[2][oz + 1] : r.at[2][oz]);
+#pragma unroll
+      for (int ox = 0; ox < 2; ++ox) {
+        id[(oz * 2 + oy) * 2 + ox] = yz + (h[0] ? r.at[0][ox + 1] : r.at[0][ox]);
+        v[(oz * 2 + oy) * 2 + ox] = __float2int_rn(wt[0][ox] * wyz);
+      }
+    }
+  add_words(w, epoch, fld, id, v);
+}
+
 constexpr int kDepThreads = 256;
 
 // The deposit, first half. One CTA per item (a brick, or a slice of a crowded one): the item's
@@ -947,6 +1033,9 @@ constexpr int kDepThreads = 256;
 // the tile reaches one cell past it: a position more than half a cell outside the brick goes into
 // the 64-bit sums instead (as does everything of a slice, word by word).
 //
+// THIN: the particles of all bricks but the sliced ones by themselves, a thread each, into a word per
+// cell and field (add_words).
+//
 // Every particle is visited once. (Before, a CTA owned 16^3 cells and visited the particles of all
 // cells that could reach them, two cells around: 1.95 visits a particle, each with a test per
 // target, and two 32-bit adds per contribution so that sums of any size fitted: 840 warp
@@ -955,9 +1044,9 @@ constexpr int kDepThreads = 256;
 // an L1 (with blocks of 32 x 8 x 8 cells, 71 KB, it ran half as fast). 512^3 cells x 2^27 particles,
 // half of them in 64 blobs: 3.8 ms, and 4.2 ms for the gather, against 10.4 ms; 256^3 x 2^24: 0.51 +
 // 0.46 against 1.57 ms.
-template <int FIELDS>
+template <int FIELDS, bool THIN>
 __global__ void __launch_bounds__(kDepThreads, 4)
-    k_dep_tile(Geom G, F32Form f, Set32 SI, Set32 SN, int32_t epoch) {
+    k_dep_tile(Geom G, F32Form f, Set32 SI, Set32 SN, int32_t epoch, int64_t n) {
   constexpr int ROWS = FIELDS == 0 ? kRowsTri : (FIELDS == 1 ? 2 * kRowsTri : kRows);
   constexpr int WORDS = ROWS * kRowWords + 4;
   __shared__ __align__(16) uint32_t acc[WORDS];
@@ -1005,6 +1094,41 @@ __global__ void __launch_bounds__(kDepThreads, 4)
   float scale[5];
 #pragma unroll
   for (int q = 0; q < 5; ++q) scale[q] = ldexpf(1.0f, exponent[q]);  // exact powers of two
+  if (THIN) {
+    for (int64_t p = (int64_t)blockIdx.x * kDepThreads + threadIdx.x; p < n; p += (int64_t)gridDim.x * kDepThreads) {
+      const uint32_t cb = f.set[SBASE].cell[p], cn = SN.cell[p];
+      uint32_t ci = 0;
+      float oi[3] = {0.f, 0.f, 0.f}, on[3], ru[3] = {0.f, 0.f, 0.f};
+      if (FIELDS) ci = SI.cell[p];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        on[d] = SN.o[d][p];
+        if (FIELDS) oi[d] = SI.o[d][p];
+        if (FIELDS == 2) ru[d] = f.rhs_u[d][p];
+      }
+      const float rt = f.rhs_t[p];
+      const int32_t *first = f.cell_start + (brick_id(G, ci_(cb), cj_(cb), ck_(cb)) & ~(uint32_t)(kBrickCells - 1));
+      if (first[kBrickCells] - first[0] > kItemMax) continue;  // in a slice
+      if (FIELDS) {
+        const Places r = places_of(G, ci);
+        mark_bricks(w, epoch, r);
+        add_trilinear(w, epoch, 0, r, oi, scale[0]);
+        if (FIELDS == 2) {
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const float u = ru[d] * scale[1 + d];
+            const uint32_t across = d == 0 ? r.at[1][1] + r.at[2][1] : (d == 1 ? r.at[0][1] + r.at[2][1] : r.at[0][1] + r.at[1][1]);
+            const uint32_t id[2] = {across + r.at[d][1], across + r.at[d][2]};
+            const int32_t v[2] = {__float2int_rn((1.f - oi[d]) * u), __float2int_rn(oi[d] * u)};
+            add_words(w, epoch, 1 + d, id, v);
+          }
+        }
+      }
+      const Places r = places_of(G, cn);
+      mark_bricks(w, epoch, r);
+      add_trilinear(w, epoch, 4, r, on, rt * scale[4]);
+    }
+  }
   auto fetch = [&](int idx) {
     return idx >= n_items ? make_int4(-1, 0, 0, 0)
                           : (idx < n_slices ? w.items[idx] : w.items[w.slice_cap + idx - n_slices]);
@@ -1161,6 +1285,7 @@ __global__ void __launch_bounds__(kDepThreads, 4)
 // The deposit, second half: every cell's exact sums from the tiles that reach it -- its own brick's
 // and, on a brick's boundary layers, its neighbours' -- and the 64-bit extras where the brick
 // has any this launch, converted to fp64 and written to the cell and its periodic ghost images.
+// THIN: the cell's own word instead of the tiles.
 // A block takes one field (blockIdx.y: RHS_Part_Temp, C, RHS_RU x, y, z; the ones from `sums` on are
 // zero, RHS_RU without TWC, grid.cpp:671); a warp takes 32 cells along x of a layer's eight rows in
 // a brick row: of every tile that reaches them ten rows (eleven of RHS_RU y) lie one behind the other, so
@@ -1171,7 +1296,7 @@ __global__ void __launch_bounds__(kDepThreads, 4)
 // (12 GB at 512^3). A warp with one row of all fields at a time had ten words in flight and decided
 // about the neighbours row by row: 512^3 4.2 ms (6.1 with the extremes), 256^3 0.47 (0.70); this
 // way 3.0 and 0.33, with or without.
-template <bool EXT>
+template <bool EXT, bool THIN>
 __global__ void __launch_bounds__(256, 4) k_dep_gather(Geom G, F32Form f, int32_t epoch, int sums, double inv_cells,
                                                        double *__restrict__ outC, double *__restrict__ outX,
                                                        double *__restrict__ outY, double *__restrict__ outZ,
@@ -1259,10 +1384,22 @@ __global__ void __launch_bounds__(256, 4) k_dep_gather(Geom G, F32Form f, int32_
         for (int r = 0; r < R; ++r)
           v[r < kBr ? r : (r == kBr + 2 ? kBr - 1 : r - kBr)] += (long long)p[r] + (long long)q[r];
       };
-      layer(bz, lz + 1);
-      if (lz == 0 || (lz == 1 && fq == 4)) layer(bz == 0 ? nbz - 1 : bz - 1, kBr + 1 + lz);
-      if (lz == kBr - 1) layer(bz == nbz - 1 ? 0 : bz + 1, 0);
       const int own = (bz * nby + by) * nbx + bx;
+      if (!THIN) {
+        layer(bz, lz + 1);
+        if (lz == 0 || (lz == 1 && fq == 4)) layer(bz == 0 ? nbz - 1 : bz - 1, kBr + 1 + lz);
+        if (lz == kBr - 1) layer(bz == nbz - 1 ? 0 : bz + 1, 0);
+      } else if (live && w.word_epoch[own] == epoch) {
+        uint32_t *x = w.mid + fld * w.ncell + (int64_t)own * kBrickCells + lz * kBr * kBr + lx;
+        int32_t e[kBr];
+#pragma unroll
+        for (int r = 0; r < kBr; ++r) e[r] = (int32_t)x[r * kBr];
+#pragma unroll
+        for (int r = 0; r < kBr; ++r) {
+          v[r] = e[r];
+          if (e[r]) x[r * kBr] = 0u;  // ready for the next launch
+        }
+      }
       if (live && w.extra_epoch[own] == epoch) {
         long long *x = w.extra + fld * w.ncell + (int64_t)own * kBrickCells + lz * kBr * kBr + lx;
         long long e[kBr];
@@ -1714,7 +1851,14 @@ int sort_step(pstep_ctx *h, bool check_sorted = false) {
   }
   // deposit work lists for this step's particle distribution
   PSTEP_CUDA(cudaMemsetAsync(f.work.counts, 0, 2 * sizeof(int32_t), h->stream));
-  k_work<<<nb(f.work.nb), 256, 0, h->stream>>>(f.cell_start, f.work, f.whole_since ? 0 : 1);
+  const int thin = thin_population(n, ncell);
+  if (thin && !f.thin) {  // no tiles from here on: every word 0, as the gather leaves them
+    PSTEP_CUDA(cudaMemsetAsync(f.work.mid, 0, sizeof(uint32_t) * f.work.nb * kRows * kBr, h->stream));
+    PSTEP_CUDA(cudaMemsetAsync(f.work.side, 0, sizeof(uint32_t) * f.work.nb * kSideWords, h->stream));
+    f.mom_stale = 0;
+  }
+  f.thin = thin;
+  k_work<<<nb(f.work.nb), 256, 0, h->stream>>>(f.cell_start, f.work, f.whole_since ? 0 : 1, thin);
   PSTEP_LAUNCHED(h);
   f.whole_since = 0;
   f.sorted = 1;
@@ -1774,6 +1918,8 @@ int f32_create(pstep_ctx *h) {
     TRY32(dalloc32(h, w.counts, 4));
     TRY32(dalloc32(h, w.dirty, (size_t)w.nb));
     TRY32(dalloc32(h, w.extra_epoch, (size_t)w.nb));
+    TRY32(dalloc32(h, w.word_epoch, (size_t)w.nb));
+    PSTEP_CUDA(cudaMemsetAsync(w.word_epoch, 0, sizeof(int32_t) * w.nb, h->stream));
     const size_t mid = (size_t)w.nb * kRows * kBr, sides = (size_t)w.nb * kSideWords;
     TRY32(dalloc32(h, w.mid, mid));
     TRY32(dalloc32(h, w.side, sides));
@@ -1819,7 +1965,7 @@ int f32_destroy(pstep_ctx *h) {
   dfree32(f->done); dfree32(f->se); dfree32(f->slots); dfree32(f->pslots); dfree32(f->unsorted); dfree32(f->totals); dfree32(f->fstat);
   {
     Work &w = f->work;
-    dfree32(w.items); dfree32(w.counts); dfree32(w.dirty); dfree32(w.extra_epoch);
+    dfree32(w.items); dfree32(w.counts); dfree32(w.dirty); dfree32(w.extra_epoch); dfree32(w.word_epoch);
     dfree32(w.mid); dfree32(w.side); dfree32(w.extra);
   }
   if (f->stage[0]) {
@@ -2154,21 +2300,23 @@ int dep_launch(pstep_ctx *h, bool do_int, Set32 SI, Set32 SN, bool ext) {
   const int fields = do_int ? (twc ? 2 : 1) : 0;
   const int64_t most = (int64_t)f.work.nb + f.work.slice_cap;
   const unsigned grid_t = (unsigned)(most < 4 * (int64_t)h->num_sms ? most : 4 * (int64_t)h->num_sms);
-  if (fields == 2 && f.mom_stale) {  // TWC switched on again: this launch writes the listed bricks' tiles, the rest are zeros
+  if (fields == 2 && f.mom_stale && !f.thin) {  // TWC switched on again: this launch writes the listed bricks' tiles, the rest are zeros
     PSTEP_CUDA(cudaMemsetAsync(f.work.mid, 0, sizeof(uint32_t) * f.work.nb * kRows * kBr, h->stream));
     PSTEP_CUDA(cudaMemsetAsync(f.work.side, 0, sizeof(uint32_t) * f.work.nb * kSideWords, h->stream));
   }
-  auto tile = fields == 2 ? k_dep_tile<2> : (fields == 1 ? k_dep_tile<1> : k_dep_tile<0>);
-  tile<<<grid_t, kDepThreads, 0, h->stream>>>(G, f, SI, SN, epoch);
+  auto tile = f.thin ? (fields == 2 ? k_dep_tile<2, true> : (fields == 1 ? k_dep_tile<1, true> : k_dep_tile<0, true>))
+                     : (fields == 2 ? k_dep_tile<2, false> : (fields == 1 ? k_dep_tile<1, false> : k_dep_tile<0, false>));
+  tile<<<grid_t, kDepThreads, 0, h->stream>>>(G, f, SI, SN, epoch, h->np);
   PSTEP_LAUNCHED(h);
-  if (fields) {
+  if (fields && !f.thin) {
     f.whole_since = 1;
     f.mom_stale = fields == 1;
   }
   double *C = h->dep[PSTEP_FIELD_C], *X = h->dep[PSTEP_FIELD_RU_X], *Y = h->dep[PSTEP_FIELD_RU_Y],
          *Z = h->dep[PSTEP_FIELD_RU_Z], *E = h->dep[PSTEP_FIELD_PART_TEMP];
   const int64_t tasks = (int64_t)((G.n[0] + 31) / 32) * (G.n[1] / kBr) * (G.n[2] / kBr), fit = 4 * (int64_t)h->num_sms;
-  auto gather = ext ? k_dep_gather<true> : k_dep_gather<false>;
+  auto gather = f.thin ? (ext ? k_dep_gather<true, true> : k_dep_gather<false, true>)
+                       : (ext ? k_dep_gather<true, false> : k_dep_gather<false, false>);
   gather<<<dim3((unsigned)(tasks < fit ? tasks : fit), fields ? 5 : 1), 256, 0, h->stream>>>(
       G, f, epoch, fields == 2 ? 5 : fields + 1, 1.0 / ((double)G.n[0] * G.n[1] * G.n[2]), C, X, Y, Z, E, h->mom_dev,
       h->emean_dev);
