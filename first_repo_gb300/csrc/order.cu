@@ -298,6 +298,9 @@ __global__ void k_iota(int32_t *__restrict__ a, int32_t *__restrict__ b, int64_t
 
 int64_t order_scratch_words(int64_t cap) { return 4 * word_len(cap) + 5 * pos_len(cap); }
 
+// capacity words that hold nothing outside a pass
+int32_t *order_free_words(pstep_ctx *h) { return bufs(h).bsphys; }
+
 // The state between stages, restored by every pass after use: no bits, empty slots, an empty list.
 int order_clear(pstep_ctx *h) {
   OrdBuf b = bufs(h);

@@ -50,6 +50,7 @@ int deposit_temperature(pstep_ctx *h, const Csr &csr, double *const frac[3], con
 int f64_temp_gather(pstep_ctx *h, const double *T, double itth);
 int64_t scan_blocks_needed(int64_t n);
 int64_t order_scratch_words(int64_t cap);
+int32_t *order_free_words(pstep_ctx *h);
 int f32_create(pstep_ctx *h);
 int f32_destroy(pstep_ctx *h);
 int f32_upload(pstep_ctx *h, const double *x, const double *y, const double *z, const double *u, const double *v,
@@ -170,7 +171,6 @@ void release(pstep_ctx *h) {
   for (int d = 0; d < 3; ++d) { dfree(h->s.frac_prev[d]); dfree(h->s.frac_new[d]); dfree(h->s.rhs_u[d]); }
   dfree(h->s.key_prev); dfree(h->s.key_new);
   dfree(h->csr_prev.cell_start); dfree(h->csr_prev.sidx); dfree(h->csr_new.cell_start); dfree(h->csr_new.sidx);
-  dfree(h->csr_prev.okey); dfree(h->csr_new.okey);
   dfree(h->counts); dfree(h->cursor); dfree(h->scan_status); dfree(h->scan_ticket); dfree(h->big_list); dfree(h->big_count);
   void *pt = h->perm_tmp; if (pt) cudaFree(pt); h->perm_tmp = nullptr;
   for (int d = 0; d < 3; ++d) dfree(h->own_u[d]);
@@ -210,22 +210,21 @@ int alloc_all(pstep_ctx *h) {
     if (h->cfg.flags & PSTEP_TRACK_ORDER) {
       TRY(dalloc(h, h->ref_of_phys, cap)); TRY(dalloc(h, h->phys_of_ref, cap)); TRY(dalloc(h, h->ref_spare, cap));
       TRY(dalloc(h, h->leave_code, cap));
-      if (h->cfg.flags & PSTEP_REFERENCE_SUMS) {
-        TRY(dalloc(h, h->csr_prev.okey, cap)); TRY(dalloc(h, h->csr_new.okey, cap));
-      }
       TRY(dalloc(h, h->ord_scratch, (size_t)order_scratch_words((int64_t)cap)));
+      // made by a stage's sort and read until the next stage's order passes, which have no use for it before
+      if (h->cfg.flags & PSTEP_REFERENCE_SUMS) h->csr_prev.okey = h->csr_new.okey = order_free_words(h);
       TRY(dalloc(h, h->ord_count, 8));
       TRY(order_clear(h));
     }
   }
-  {  // permutation / download scratch, both forms
+  if (!is_f32(h)) {  // sort items and download scratch, the sorts by node
     double *pt = nullptr;
     TRY(dalloc(h, pt, cap));
     h->perm_tmp = pt;
+    TRY(dalloc(h, h->csr_prev.cell_start, gs + 1)); TRY(dalloc(h, h->csr_new.cell_start, gs + 1));
+    TRY(dalloc(h, h->big_list, gs)); TRY(dalloc(h, h->big_count, 1));
   }
-  TRY(dalloc(h, h->csr_prev.cell_start, gs + 1)); TRY(dalloc(h, h->csr_new.cell_start, gs + 1));
   TRY(dalloc(h, h->counts, gs)); TRY(dalloc(h, h->cursor, gs));
-  TRY(dalloc(h, h->big_list, gs)); TRY(dalloc(h, h->big_count, 1));
   int64_t scan_n = (int64_t)gs + 1;
   if ((int64_t)cap > scan_n) scan_n = (int64_t)cap;
   h->scan_nblocks = scan_blocks_needed(scan_n) + 1;
@@ -764,7 +763,9 @@ int pstep_get_particle_array(pstep_handle h, int id, void *dst, int on_device) {
   if (is_f32(h) && id != PSTEP_FLAG) return f32_get_array(h, id, dst, on_device);
   if (id >= PSTEP_UG) return fail(h, PSTEP_ERR_CONFIG, "gas values per particle are kept by the FP32 form");
   const int32_t *perm = (h->cfg.flags & PSTEP_TRACK_ORDER) ? h->phys_of_ref : nullptr;
-  if (id == PSTEP_FLAG) {
+  if (id == PSTEP_FLAG && is_f32(h)) {
+    PSTEP_CUDA(cudaMemcpyAsync(dst, h->s.flag, sizeof(int32_t) * n, kind_out(on_device), h->stream));
+  } else if (id == PSTEP_FLAG) {
     int32_t *tmp = (int32_t *)h->perm_tmp;
     k_gather_ref_i<<<blocks_for(n), kThreads, 0, h->stream>>>(h->s.flag, perm, n, tmp);
     PSTEP_LAUNCHED(h);

@@ -65,7 +65,7 @@ struct F32Form;
 struct Csr {
   int32_t *cell_start;  // gsize + 1
   int32_t *sidx;        // sorted physical indices
-  int32_t *okey;        // REFERENCE_SUMS: the sorted particles' reference positions (order within a node)
+  int32_t *okey;        // REFERENCE_SUMS: the sorted particles' reference positions (order within a node); one for both
   int identity;         // sidx[i] == i (after the per-step reorder)
 };
 
@@ -100,7 +100,7 @@ struct pstep_ctx {
   int32_t *big_list;    // nodes with long segments (gsize)
   int32_t *big_count;   // device counter
   int64_t scan_nblocks;
-  // permutation scratch (per-step reorder)
+  // FP64 form: sort items, downloads
   void *perm_tmp;
   size_t perm_tmp_bytes;
 

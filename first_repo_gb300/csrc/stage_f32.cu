@@ -102,9 +102,7 @@ struct F32Form {
   uint2 *corr_y;   // learned correction: the network output of the step's stage 0 (bf16 x 4)
   float *rhs_u[3];
   float *uf[3], *tf;  // fp32 ghosted copies of the bound fields
-  uint32_t *key;      // brick-major cell id of the base position
   int32_t *cell_start;  // n^3 + 1, brick-major order (per step)
-  int32_t *sidx;
   uint32_t *slots;    // kBoundSlots x 4 partial maxima (spread so blocks do not contend on one word)
   uint32_t *pslots;   // kBoundSlots x 2: the last stage's max u and max ug (order-preserving keys)
   int pmax_state;     // 0: none; 1: filled by this step's last stage; 2: valid for the base state
@@ -1762,15 +1760,18 @@ int sort_step(pstep_ctx *h, bool check_sorted = false) {
   const Geom &G = h->geom;
   const int64_t n = h->np;
   const int64_t ncell = (int64_t)G.n[0] * G.n[1] * G.n[2];
+  // the brick-major cells and the permutation: RHS_u holds nothing between stages
+  uint32_t *key = reinterpret_cast<uint32_t *>(f.rhs_u[0]);
+  int32_t *sidx = reinterpret_cast<int32_t *>(f.rhs_u[1]);
   PSTEP_CUDA(cudaMemsetAsync(h->counts, 0, sizeof(int32_t) * ncell, h->stream));
   if (n > 0) {
-    k_keys32<<<nb(n), kThreads, 0, h->stream>>>(G, f.set[SBASE], n, f.key, h->counts);
+    k_keys32<<<nb(n), kThreads, 0, h->stream>>>(G, f.set[SBASE], n, key, h->counts);
     PSTEP_LAUNCHED(h);
   }
   bool in_order = false;
   if (check_sorted && n > 1) {
     PSTEP_CUDA(cudaMemsetAsync(f.unsorted, 0, sizeof(int32_t), h->stream));
-    k_keys_unsorted<<<h->num_sms * 8, kThreads, 0, h->stream>>>(f.key, n, f.unsorted);
+    k_keys_unsorted<<<h->num_sms * 8, kThreads, 0, h->stream>>>(key, n, f.unsorted);
     PSTEP_LAUNCHED(h);
     int32_t u = 1;
     PSTEP_CUDA(cudaMemcpyAsync(&u, f.unsorted, sizeof u, cudaMemcpyDeviceToHost, h->stream));
@@ -1782,7 +1783,7 @@ int sort_step(pstep_ctx *h, bool check_sorted = false) {
   if (in_order)
     TRY32(exclusive_scan(h, h->counts, ncell, f.cell_start, nullptr));
   else
-    TRY32(csr_sort(h, f.key, 0, ncell, h->s.flag, f.cell_start, f.sidx, nullptr, 0, true));
+    TRY32(csr_sort(h, key, 0, ncell, h->s.flag, f.cell_start, sidx, nullptr, 0, true));
   if (n > 0 && !in_order) {
     Set32 &B = f.set[SBASE];
     // every 4-byte per-particle array that lives across steps; the addresses of their
@@ -1816,18 +1817,18 @@ int sort_step(pstep_ctx *h, bool check_sorted = false) {
         pb.dst[a] = (uint32_t *)get(scr[a]);
       }
       switch (k) {
-        case 1: k_perm_batch<uint32_t, 1><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 2: k_perm_batch<uint32_t, 2><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 3: k_perm_batch<uint32_t, 3><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 4: k_perm_batch<uint32_t, 4><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 5: k_perm_batch<uint32_t, 5><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 6: k_perm_batch<uint32_t, 6><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 7: k_perm_batch<uint32_t, 7><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 8: k_perm_batch<uint32_t, 8><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 9: k_perm_batch<uint32_t, 9><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 10: k_perm_batch<uint32_t, 10><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        case 11: k_perm_batch<uint32_t, 11><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
-        default: k_perm_batch<uint32_t, 12><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n); break;
+        case 1: k_perm_batch<uint32_t, 1><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 2: k_perm_batch<uint32_t, 2><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 3: k_perm_batch<uint32_t, 3><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 4: k_perm_batch<uint32_t, 4><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 5: k_perm_batch<uint32_t, 5><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 6: k_perm_batch<uint32_t, 6><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 7: k_perm_batch<uint32_t, 7><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 8: k_perm_batch<uint32_t, 8><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 9: k_perm_batch<uint32_t, 9><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 10: k_perm_batch<uint32_t, 10><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        case 11: k_perm_batch<uint32_t, 11><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
+        default: k_perm_batch<uint32_t, 12><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n); break;
       }
       PSTEP_LAUNCHED(h);
       for (int a = 0; a < k; ++a) {  // the gathered copy takes the array's place; the old one is scratch
@@ -1842,7 +1843,7 @@ int sort_step(pstep_ctx *h, bool check_sorted = false) {
       PermBatch<uint2> pb{};
       pb.src[0] = f.drive;
       pb.dst[0] = f.corr_y;
-      k_perm_batch<uint2, 1><<<pgrid, 256, 0, h->stream>>>(pb, f.sidx, n);
+      k_perm_batch<uint2, 1><<<pgrid, 256, 0, h->stream>>>(pb, sidx, n);
       PSTEP_LAUNCHED(h);
       uint2 *t = f.drive;
       f.drive = f.corr_y;
@@ -1904,10 +1905,8 @@ int f32_create(pstep_ctx *h) {
   const size_t gs = (size_t)G.gsize;
   for (int d = 0; d < 3; ++d) TRY32(dalloc32(h, f->uf[d], gs));
   TRY32(dalloc32(h, f->tf, gs));
-  TRY32(dalloc32(h, f->key, cap));
   const size_t ncell = (size_t)G.n[0] * G.n[1] * G.n[2];
   TRY32(dalloc32(h, f->cell_start, ncell + 1));
-  TRY32(dalloc32(h, f->sidx, cap));
   {  // deposit work lists, tiles and 64-bit sums
     Work &w = f->work;
     w.nb = (G.n[0] / kBr) * (G.n[1] / kBr) * (G.n[2] / kBr);
@@ -1961,7 +1960,7 @@ int f32_destroy(pstep_ctx *h) {
   dfree32(f->drive);
   dfree32(f->corr_y);
   for (int d = 0; d < 3; ++d) { dfree32(f->rhs_u[d]); dfree32(f->uf[d]); }
-  dfree32(f->tf); dfree32(f->key); dfree32(f->cell_start); dfree32(f->sidx);
+  dfree32(f->tf); dfree32(f->cell_start);
   dfree32(f->done); dfree32(f->se); dfree32(f->slots); dfree32(f->pslots); dfree32(f->unsorted); dfree32(f->totals); dfree32(f->fstat);
   {
     Work &w = f->work;
