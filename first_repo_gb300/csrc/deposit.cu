@@ -3,11 +3,12 @@
 //
 // Fast path (k_dep_brick): one CTA per brick of B^3 target cells of the ghosted
 // grid. Its threads walk the CSR segments (particles sorted by node, then h,
-// then storage index) of the brick's nodes plus a one-node halo, form per-node
-// partial sums in shared memory -- the 8 trilinear offsets of a node, and the
-// face-normal partials of each trunc cell, added in 8 conflict-free phases (one
-// per h class) -- then every target cell sums its partials in a fixed order.
-// Halo nodes are walked by both neighbouring bricks; no cross-brick reduction.
+// then storage index) of the brick's nodes plus a one-node halo and form partial
+// sums in shared memory -- the 8 trilinear offsets of every node, and the
+// face-normal partials of every trunc cell from the h classes' runs that fall into
+// it, lists of like length side by side -- then every target cell sums its partials
+// in a fixed order. Halo nodes are walked by both neighbouring bricks; no cross-brick
+// reduction.
 //
 // Reference-order path (PSTEP_REFERENCE_SUMS, k_dep_ordered): a warp merges the node lists
 // around its targets by the particles' positions in the reference's vectors, so every cell

@@ -25,8 +25,8 @@
 // 8^3 cells is one work item: its particles (sorted by cell once per step, moving
 // less than a cell per stage) are added into 32-bit sums in shared memory over the
 // brick and the cells around it, and a second kernel sums the tiles that reach a
-// cell. What a 32-bit sum cannot hold goes into 64-bit sums in memory. No per-stage
-// sort.
+// cell. What a 32-bit sum cannot hold goes into 64-bit sums in memory. (Thin populations
+// on large grids add to one 32-bit sum per cell in memory instead.) No per-stage sort.
 //
 // FP64 on GB300 runs at a small fraction of the fp32 rate, so this form keeps
 // fp64 out of every per-particle operation: the only fp64 arithmetic left is
@@ -284,8 +284,8 @@ __device__ __forceinline__ float adv_finish_t(const Geom &G, const F32Form &f, c
       in_[d] = ia[d];
     }
   }
-  // x_new within one cell of the step-start cell on every axis: the deposit's source
-  // windows (two cells around a brick) hold a particle's x_int and x_new cells only then
+  // x_new more than one cell from the step-start cell along some axis is reported: the step is meant for
+  // moves of at most one cell (the deposit takes any: what leaves a brick's tile goes into the 64-bit sums)
   {
     bool far = false;
 #pragma unroll
@@ -1040,8 +1040,8 @@ constexpr int kDepThreads = 256;
 // instructions a visit.) Bound: the shared-memory adds (22 a particle) and instruction issue;
 // four CTAs per SM let one's flush overlap the others' particles, and the 25 KB tile leaves them
 // an L1 (with blocks of 32 x 8 x 8 cells, 71 KB, it ran half as fast). 512^3 cells x 2^27 particles,
-// half of them in 64 blobs: 3.8 ms, and 4.2 ms for the gather, against 10.4 ms; 256^3 x 2^24: 0.51 +
-// 0.46 against 1.57 ms.
+// half of them in 64 blobs: 3.8 ms, and 3.0 ms for the gather, against 10.4 ms; 256^3 x 2^24: 0.51 +
+// 0.33 against 1.57 ms.
 template <int FIELDS, bool THIN>
 __global__ void __launch_bounds__(kDepThreads, 4)
     k_dep_tile(Geom G, F32Form f, Set32 SI, Set32 SN, int32_t epoch, int64_t n) {
@@ -1595,8 +1595,7 @@ __global__ void k_from_f64(Geom G, F32Form f, const double *__restrict__ x, cons
   B.v[3][p] = narrow(V[3] - tref);
 }
 
-// the cell sizes l/n of the position conversions (a double division each, made on the host)
-// a dimension's cell size and -1024 times it
+// the position conversions' cell sizes l/n (a double division each, made on the host) and -1024 times them
 struct Dx {
   double d[3], off[3];
 };
