@@ -201,9 +201,10 @@ constexpr int kBrickThreads = 384;
 // hold up its whole brick.
 // The line: a warp pays ceil(n / 32) rounds and a reduction, 32 threads with lists alike n rounds
 // for 32 lists; beside each other at 2^24 particles in 64 blobs: node lists up to 24, 32, 64, 128
-// by threads 2.06, 2.05, 1.86, 1.83 ms (temperature deposit), but cell lists, which gather from
-// eight runs, 4.28, 4.13, 4.50, 4.77 ms (with the trilinear part).
-constexpr int kDenseNode = 64, kDenseCell = 32;
+// by threads 2.06, 2.05, 1.86, 1.83 ms (temperature deposit), cell lists, which gather from
+// eight runs, 4.28, 4.13, 4.50, 4.77 ms (with the trilinear part). Nodes stop at 32 all the same: a chain of
+// 64 additions rounds more than lane sums and a tree (error of RHS_Part_Temp 6.95e-16 -> 7.25e-16).
+constexpr int kDenseNode = 32, kDenseCell = 32;
 constexpr int kBins = kDenseNode + 2;  // list lengths 0 .. 64, and longer
 
 // The warp's sums of m[0..7] in a fixed order; each round a lane hands over the half of its values
@@ -234,7 +235,7 @@ __device__ __forceinline__ double warp_sums8(const double (&m)[8], int lane) {
 // t = (x_l, y_l, z_l) of each particle and value v (1 for the concentration),
 // M[s] = sum v * prod_{d in s} t_d for the 8 subsets s of {x (4), y (2), z (1)}.
 // The corner with (1 - t_d) in the dimensions of bit set o and t_d in the others is
-// sum_{A subset of o} (-1)^|A| M[A | ~o], formed once per node, a dimension at a time.
+// sum_{A subset of o} (-1)^|A| M[A | ~o], formed once per node.
 // GB300's FP64 pipe (two lanes per SM and clock) is the bound of this kernel, and per particle
 // this takes 3 + 4 + 8 FP64 operations instead of 6 + 3 + 24 (+ 8). x_l = frac + 0.5 - h is formed as
 // frac + (h ? -0.5 : 0.5), the same value (frac - 1 and frac - 0.5 are exact for
@@ -280,20 +281,25 @@ __device__ __forceinline__ void moments_add(double (&m)[8], const TriRec<MODE> &
   }
 }
 
-// moments -> corner partials in place (index bit 2: x takes 1 - x_l, bit 1: y, bit 0: z)
+// moments -> corner partials in place (index bit 2: x takes 1 - x_l, bit 1: y, bit 0: z), the terms of the sum
+// above one after the other (a dimension at a time takes 12 additions instead of 19 and rounds more: the
+// error of C in a box of 64^3 cells and 2^15 particles 1.425e-16 -> 1.445e-16)
 __device__ __forceinline__ void corners_of(double (&m)[8]) {
+  double c[8];
 #pragma unroll
-  for (int bit = 1; bit < 8; bit <<= 1)
+  for (int o = 0; o < 8; ++o) {
+    const int rest = ~o & 7;
+    c[o] = m[rest];
 #pragma unroll
-    for (int s = 0; s < 8; ++s)
-      if (!(s & bit)) {
-        const double without = m[s], with = m[s | bit];
-        m[s] = with;
-        m[s | bit] = without - with;
-      }
+    for (int a = 1; a < 8; ++a)
+      if ((a & o) == a) c[o] = (__popc(a) & 1) ? c[o] - m[a | rest] : c[o] + m[a | rest];
+  }
+#pragma unroll
+  for (int o = 0; o < 8; ++o) m[o] = c[o];
 }
 
-// face sums of one particle: (sum r, sum t r) per dimension, r = RHS_u component
+// face sums: (sum (1 - t) r, sum t r) per dimension, t the in-cell fraction and r the RHS_u component; the first
+// one's terms are rounded once each (as sum r - sum t r a cell of two particles lost a bit)
 struct FaceRec {
   double f[3], r[3];
 };
@@ -309,7 +315,7 @@ __device__ __forceinline__ FaceRec face_load(const DepIn &d, int32_t p) {
 __device__ __forceinline__ void face_add(double (&f)[6], const FaceRec &q) {
 #pragma unroll
   for (int D = 0; D < 3; ++D) {
-    f[2 * D] += q.r[D];
+    f[2 * D] += fma(-q.f[D], q.r[D], q.r[D]);
     f[2 * D + 1] = fma(q.f[D], q.r[D], f[2 * D + 1]);
   }
 }
@@ -419,11 +425,11 @@ __device__ __forceinline__ void take_items(BrickSmem<MODE> &sm, Dense dense, Lig
 // one item per trunc cell of [b-1, b+B-1]; its particles are, for each h class, that class's
 // run in node c + h's segment (the runs in class order, the empty ones skipped by a mask), so
 // all of a cell's particles are summed by one thread. Bound: the FP64 pipe; per particle 14 (15
-// in mode 1) operations for the trilinear sums and 6 for the faces, 12 + 7 a node and target,
-// 3 + 3 a cell and target. The pipe answers through a queue (short scoreboard), so a brick's
+// in mode 1) operations for the trilinear sums and 9 for the faces, 19 + 7 a node and target,
+// 6 + 3 a cell and target. The pipe answers through a queue (short scoreboard), so a brick's
 // phases stay latency-bound between barriers (three CTAs per SM). 256^3 cells x 2^24 particles in
-// 64 blobs: 4.4 and 1.7 ms, of the first 1.9 the trilinear part, 0.8 the class table and order
-// of the cells, 1.7 the face sums (a thread per node in storage order, the faces in eight
+// 64 blobs: 4.2 and 2.0 ms (node lists to 64, corners a dimension at a time, faces as sum r - sum x_l r: 4.4 and
+// 1.7; of the first 1.9 the trilinear part, 0.8 the class table and order of the cells, 1.7 the face sums; a thread per node in storage order, the faces in eight
 // h-class phases over all nodes: 15 and 5 ms).
 template <int MODE>
 __global__ void __launch_bounds__(kBrickThreads, 3) k_dep_brick(Geom G, DepIn d, int twc,
@@ -573,14 +579,6 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_dep_brick(Geom G, DepIn d,
   // ---- faces
   for (int s = threadIdx.x; s < 6 * kNodes; s += blockDim.x) sm.face[0][s] = 0.0;
   order_by_length<kDenseCell>(sm);
-  auto put = [&](int s, const double (&fs)[6]) {
-    // (1 - x_l) r summed as sum r - sum x_l r; x_l r as is
-#pragma unroll
-    for (int D = 0; D < 3; ++D) {
-      sm.face[2 * D][s] = fs[2 * D] - fs[2 * D + 1];
-      sm.face[2 * D + 1][s] = fs[2 * D + 1];
-    }
-  };
   take_items(
       sm,
       [&](int s) {
@@ -594,12 +592,7 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_dep_brick(Geom G, DepIn d,
         }
         const double m[8] = {fs[0], fs[1], fs[2], fs[3], fs[4], fs[5], 0.0, 0.0};
         const double v = warp_sums8(m, lane);  // lanes 0, 4, .. 20: fs[0..5]
-        const double w = __shfl_down_sync(0xffffffffu, v, 4);
-        // (1 - x_l) r summed as sum r - sum x_l r; x_l r as is
-        if (!(lane & 7) && lane < 24) {
-          sm.face[lane >> 2][s] = v - w;
-          sm.face[(lane >> 2) + 1][s] = w;
-        }
+        if (!(lane & 3) && lane < 24) sm.face[lane >> 2][s] = v;
       },
       [&](int s) {
         const int base = ((s / (kB1 * kB1)) * kB2 + (s / kB1) % kB1) * kB2 + s % kB1;
@@ -616,17 +609,25 @@ __global__ void __launch_bounds__(kBrickThreads, 3) k_dep_brick(Geom G, DepIn d,
           }
           return pidx(d, q++);
         };
+        double fb[6] = {0, 0, 0, 0, 0, 0};  // every other particle's
         int32_t ahead = next();
         FaceRec rec = face_load(d, ahead);
         ahead = next();
         while (ahead >= 0) {
-          const FaceRec following = face_load(d, ahead);
+          const FaceRec other = face_load(d, ahead);
           ahead = next();
           face_add(fs, rec);
-          rec = following;
+          if (ahead < 0) {
+            rec = other;
+            break;
+          }
+          rec = face_load(d, ahead);
+          ahead = next();
+          face_add(fb, other);
         }
-        face_add(fs, rec);
-        put(s, fs);
+        face_add(fb, rec);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) sm.face[q][s] = fs[q] + fb[q];
       });
   __syncthreads();
   for (int s = threadIdx.x; s < kB * kB * kB; s += blockDim.x) {

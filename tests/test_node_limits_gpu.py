@@ -1,5 +1,5 @@
-"""The FP64 form's lists a node at the lengths that its present lines make special: 63 to 66 particles a node (64
-are one thread's, 65 a warp's in the brick deposit) and 16383 to 16385 (16384 is the longest list sorted on
+"""The FP64 form's lists a node around the lengths where their handling changes or has changed: 31 to 34 and 63 to
+66 particles a node (one thread's, or a warp's in the brick deposit) and 16383 to 16385 (16384 is the longest list sorted on
 chip; one more is reported as PSTEP_ERR_CAPACITY, in bounds, and the handle goes on). Fields by bricks
 against the reference's sums within the form's 1e-12 of max|field| (tests/test_deposit_lists_gpu.py);
 the reference's sums and order against the oracle, bit for bit."""
@@ -35,7 +35,7 @@ def start(g, arrs, fields):
     return g
 
 
-@pytest.mark.parametrize("per_node", [63, 64, 65, 66])
+@pytest.mark.parametrize("per_node", [31, 32, 33, 34, 63, 64, 65, 66])
 def test_brick_lists_at_their_line(built_cuda, per_node):
     n = 13
     bp, arrs = crowd(n, per_node, 40, per_node)
