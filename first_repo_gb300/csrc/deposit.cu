@@ -428,9 +428,9 @@ __device__ __forceinline__ void take_items(BrickSmem<MODE> &sm, Dense dense, Lig
 // in mode 1) operations for the trilinear sums and 9 for the faces, 19 + 7 a node and target,
 // 6 + 3 a cell and target. The pipe answers through a queue (short scoreboard), so a brick's
 // phases stay latency-bound between barriers (three CTAs per SM). 256^3 cells x 2^24 particles in
-// 64 blobs: 4.2 and 2.0 ms (node lists to 64, corners a dimension at a time, faces as sum r - sum x_l r: 4.4 and
-// 1.7; of the first 1.9 the trilinear part, 0.8 the class table and order of the cells, 1.7 the face sums; a thread per node in storage order, the faces in eight
-// h-class phases over all nodes: 15 and 5 ms).
+// 64 blobs: 4.2 and 2.0 ms. (Node lists to 64, corners a dimension at a time, faces as sum r - sum x_l r:
+// 4.4 and 1.7, of the first 1.9 the trilinear part, 0.8 the class table and order of the cells, 1.7 the face
+// sums. A thread per node in storage order, the faces in eight h-class phases over all nodes: 15 and 5 ms.)
 template <int MODE>
 __global__ void __launch_bounds__(kBrickThreads, 3) k_dep_brick(Geom G, DepIn d, int twc,
                                                              double *__restrict__ out_tri,
